@@ -40,6 +40,23 @@ def test_attention_forward(dtype, d, lens):
 
 
 @pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("lens", [[1], [257], [129, 1, 1, 640], [900]])
+def test_attention_forward_extreme_scores(d, lens):
+    """Rows whose scores span hundreds (the running maximum advances block by block), rows with a single key, and tiles
+    in which some rows have no key in a block.  P is rounded to 16 bits (half an ulp, 2^-9) and so is the result."""
+    T, nh, nkv = sum(lens), 5, 1
+    qkv, ds, de = _make(T, nh, nkv, d, lens, torch.bfloat16, seed=3)
+    q = qkv[:, : nh * d].view(T, nh, d) * 4
+    k = qkv[:, nh * d: (nh + nkv) * d].view(T, nkv, d) * (1 + torch.arange(T, device=DEV)[:, None, None] % 7).to(qkv.dtype)
+    v = qkv[:, (nh + nkv) * d:].view(T, nkv, d)
+    o = AT.varlen_attention(q, k, v, ds, de)
+    NV.check_status()
+    ref = AT.attention_ref(q, k, v, ds)
+    assert torch.isfinite(o.float()).all()
+    assert _rel(o, ref) < 2 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("d", [128, 64])
 @pytest.mark.parametrize("lens", [[256], [100, 156, 7, 249], [640, 129, 255]])
 def test_attention_backward(d, lens):
     T = sum(lens)
