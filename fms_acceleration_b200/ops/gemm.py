@@ -260,9 +260,6 @@ def gemm_q4_fused(x: torch.Tensor, qs, xa: torch.Tensor | None = None, bl: torch
         shard_ptrs = (_ct.c_void_p * 1)(qs.packed.data_ptr())
     else:
         world = len(shard_ptrs)
-    if bn is None:
-        # enough CTAs to put every SM to work on a thin problem
-        bn = 128 if (Nn // 128) * ((M + 127) // 128) >= 148 else (64 if (Nn // 64) * ((M + 127) // 128) >= 148 else 32)
     code_host = _code16_host(qs.quant_type)  # host constants: no device read on the launch path
     r2 = 0
     if xa is not None:
@@ -274,7 +271,7 @@ def gemm_q4_fused(x: torch.Tensor, qs, xa: torch.Tensor | None = None, bl: torch
         x.data_ptr(), x.stride(0), shard_ptrs, int(shard_bytes), world, N.ptr(qs.absmax), N.ptr(qs.absmax_q),
         N.ptr(qs.code2), N.ptr(qs.absmax2), float(qs.offset), code_host, N.ptr(xa), xa.stride(0) if xa is not None else 0,
         N.ptr(bl), bl.stride(0) if bl is not None else 0, r2, out.data_ptr(), out.stride(0), float(alpha), M, Nn, K,
-        N.dtype_code(x.dtype), bn, st.data_ptr(), N.stream_ptr())
+        N.dtype_code(x.dtype), bn or 0, st.data_ptr(), N.stream_ptr())  # 0: the library chooses kernel and tile
     N.check(rc, "fmsb_gemm_q4_fused")
     return out
 

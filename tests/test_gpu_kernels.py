@@ -360,6 +360,29 @@ def test_fused_q4_gemm_matches_dequant_then_gemm(M, Nn, K, bn, double_quant, lor
         assert torch.equal(y2, y)
 
 
+@pytest.mark.parametrize("M,Nn,K,dtype,double_quant", [
+    (1, 8, 64, torch.bfloat16, True), (4, 4104, 64, torch.float16, False), (3, 4096, 4096, torch.bfloat16, True),
+    (1, 1032, 14336, torch.float16, True), (3, 4096, 14336, torch.bfloat16, True), (4, 256, 14336, torch.bfloat16, True),
+    (5, 264, 192, torch.bfloat16, True), (77, 14336, 512, torch.bfloat16, True), (129, 4104, 256, torch.float16, False)])
+def test_fused_q4_gemm_chosen_kernel_matches_fp64(M, Nn, K, dtype, double_quant):
+    """The kernel the library chooses (few rows on the CUDA cores, else a tile width by size) against 64 bits.  The
+    result is rounded to the 16-bit type once (half an ulp); the tensor-core form also rounds every weight (half an
+    ulp each, independent), so 2 ulp of the largest |x| |w| row sum / sqrt(K) is generous: 4 ulp of the result's scale."""
+    from fms_acceleration_b200.ops.gemm import gemm_q4_fused
+
+    torch.manual_seed(M + Nn + K)
+    qs = Q.quantize_4bit((torch.randn(Nn, K, device=DEV) * 0.05).to(dtype), "nf4", 64, double_quant)
+    wd = Q.dequantize_4bit_ref(qs, torch.float64).view(Nn, K)
+    base = (torch.randn(M, K + 8, device=DEV) * 0.5).to(dtype)
+    x = base[:, :K]  # rows that are not adjacent
+    y = gemm_q4_fused(x, qs)
+    NV.check_status()
+    ref = x.double() @ wd.t()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert y.shape == (M, Nn) and y.dtype == dtype
+    assert (y.double() - ref).abs().max() <= 4 * ulp * ref.abs().max()
+
+
 @pytest.mark.parametrize("M,Nn,K,gs,bn,dtype,zoff,lora", [(64, 512, 256, 128, 128, torch.float16, 0, False),
                                                          (128, 384, 512, 64, 64, torch.bfloat16, 1, True),
                                                          (200, 264, 1024, 1024, 32, torch.bfloat16, 0, True),
