@@ -1,0 +1,1052 @@
+// Chunked state-space-duality scan with its decay matrices kept on the chip (chunk 256, head dimension 64, state 128;
+// other shapes take the batched products of gemm_tcgen05.cu and the passes of mamba_scan.cu).
+//
+// Per chunk c and head h, with L the within-chunk cumulative sum of dt*A and CB = C B^T (shared by the heads of a group):
+//
+//   G[t, s]  = CB[t, s] exp(L_t - L_s) dt_s          (s <= t, else 0)
+//   y        = G x + exp(L_t) (C Hprev^T) + D x       Hprev: state entering the chunk
+//   S        = (x w)^T B,   w = exp(L_last - L) dt     what the chunk adds to the state
+//   dx       = G^T dy + w (B dS^T) + D dy              dS: gradient of the state leaving the chunk
+//   dHprev   = (exp(L) dy)^T C,   dC = (exp(L) dy) Hprev + dCB B,   dB = (x w) dS + dCB^T C
+//   dCB      = sum over heads of (dy x^T) o exp(L_t - L_s) dt_s
+//
+// Written as separate products these cost a [chunks, heads, 256, 256] 16-bit matrix (2.7 GB per layer at 65536 tokens)
+// through memory several times and fp32 copies of every [T, heads, 64] product.  Here G is built in registers
+// from CB (held as 16-bit pairs, 64 registers a thread) and written to tensor memory as the A operand of G x, like the
+// probabilities of an attention kernel; scaled copies of x and dy exist only in shared memory; the epilogues add the
+// terms and take the row dot products.  What is left is bound by reading x / dy and writing y / dx once.
+//
+// Roles of every kernel here (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute (lane quarter
+// warp % 4, column half (warp - 2) / 4).  Every wait is bounded.
+#include "common.cuh"
+
+namespace fmsb {
+namespace ssdf {
+
+constexpr int CQ = 256;  // chunk
+constexpr int CP = 64;   // head dimension
+constexpr int CN = 128;  // state
+constexpr int kTile = 128 * 128;      // bytes of a [128 x 64] 16-bit tile
+constexpr float kSplitLimit = 60.f;   // |exponent| across eight columns below which the decay factorises safely
+
+struct ScanParams {
+  int nc, nh, G, hp;   // hp: heads per CTA
+  const float* Lt;     // [nc, nh, 256]
+  const float* dtt;    // [nc, nh, 256]
+  const float* D;      // [nh]
+  float* red;          // MODE 1: [nc, nh, 256]; MODE 2: three of them (dy.x, w x.(B dS^T), x.(G^T dy))
+  float* S;            // state kernel: [nc, nh, 64, 128]
+  float* part;         // partial sums over head splits
+  int wmode;           // state kernel: 0 rows scaled by exp(L_last - L) dt, 1 by exp(L)
+  int T;
+  int* status;
+};
+
+__device__ __forceinline__ void compute_sync(int id) { asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory"); }
+
+template <int FMT>
+__device__ __forceinline__ void unpack2(uint32_t w, float& a, float& b) {
+  if (FMT == 1) {
+    a = __uint_as_float(w << 16);
+    b = __uint_as_float(w & 0xffff0000u);
+  } else {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    a = f.x;
+    b = f.y;
+  }
+}
+template <int FMT>
+__device__ __forceinline__ uint32_t pack2f(float a, float b) {
+  return FMT == 1 ? pack_bf16x2(a, b) : pack_f16x2(a, b);
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint32_t swz(int r, int c16) { return static_cast<uint32_t>(r * 128 + ((c16 ^ (r & 7)) << 4)); }
+
+// Per-head scalars of a chunk in shared memory, three sets (a set is rewritten only after every compute warp has passed
+// the barrier that follows its last use).  The decay of eight neighbouring columns is factorised around their first
+// one: exp(L_t - L_s) = exp(L_t - L_ref) exp(L_ref - L_s), one exponential per row and eight columns; `ok` says whether
+// the exponents are moderate enough for that, otherwise every element takes its own exponential.
+struct HeadScalars {
+  float L[CQ];
+  float d[CQ];
+  float cf[CQ];  // rows t: exp(L_ref - L_s) dt_s; rows s (MODE 2): exp(L_t - L_ref)
+  int ok[CQ / 8];
+};
+
+template <int MODE>
+__device__ __forceinline__ void publish(HeadScalars& hs, int i, float L, float d) {
+  const int lane = i & 31;
+  const float ref = __shfl_sync(0xffffffffu, L, lane & ~7), last = __shfl_sync(0xffffffffu, L, lane | 7);
+  hs.L[i] = L;
+  hs.d[i] = d;
+  hs.cf[i] = MODE == 2 ? __expf(L - ref) : __expf(ref - L) * d;
+  if ((lane & 7) == 0) hs.ok[i >> 3] = fabsf(ref - last) < kSplitLimit ? 1 : 0;
+}
+
+// ----------------------------------------------------------------------------------------
+// Scan kernel.  grid (nc * 2, G * splits): one 128-row tile of a chunk, hp heads in turn.
+//   MODE 0: rows t; R = C, columns B; V = x, H = Hprev; out = y
+//   MODE 1: the same products, out = dy . (G x + exp(L) C Hprev^T) per row (E = dy)
+//   MODE 2: rows s; R = B, columns C; V = dy, H = dS; out = dx and three row dot products (E = x)
+// Tensor memory: two G buffers of 128 columns (256 contraction indices as 16-bit pairs), two accumulators of 64 + 64.
+// While the tensor core works on head i, the compute warps build G of head i + 1, then drain head i.
+// ----------------------------------------------------------------------------------------
+constexpr int kScanStage = 2 * kTile + kTile + kTile;  // V (256 rows), H (64 x 128), E
+constexpr int kScanSmem = 2 * kTile + 2 * kScanStage + 2 * kTile + 3 * (int)sizeof(HeadScalars) + 2 * 3 * 2 * 128 * 4 + 1024 + 256;
+
+template <int MODE, int FMT>
+__global__ void __launch_bounds__(320, 1)
+ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmCol,
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmH,
+                const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmOut, const ScanParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t sR = base;
+  auto sV = [&](int s) { return base + 2 * kTile + s * kScanStage; };
+  auto sH = [&](int s) { return sV(s) + 2 * kTile; };
+  auto sE = [&](int s) { return sV(s) + 3 * kTile; };
+  const uint32_t sCol = sV(0);  // prologue only: 2 x [128 x 128] = stage 0
+  const uint32_t sOut = base + 2 * kTile + 2 * kScanStage;
+  const uint32_t scal = sOut + 2 * kTile;
+  const uint32_t dots = scal + 3 * (uint32_t)sizeof(HeadScalars);
+  const uint32_t bars = dots + 2 * 3 * 2 * 128 * 4;
+  const uint32_t bar_r = bars, bar_cb = bars + 8u;
+  auto full = [&](int s) { return bars + 16u + 8u * s; };
+  auto empty = [&](int s) { return bars + 32u + 8u * s; };
+  auto g_full = [&](int b) { return bars + 48u + 8u * b; };
+  auto acc_full = [&](int b) { return bars + 64u + 8u * b; };
+  const uint32_t holder = bars + 80u;
+  HeadScalars* hs = reinterpret_cast<HeadScalars*>(smem_raw + (scal - smem_u32(smem_raw)));
+  float* sdot = reinterpret_cast<float*>(smem_raw + (dots - smem_u32(smem_raw)));  // [2][3][2][128]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x >> 1, tile = blockIdx.x & 1;
+  const int hpg = p.nh / p.G, spg = gridDim.y / p.G;
+  const int g = blockIdx.y / spg;
+  const int h_begin = g * hpg + (blockIdx.y % spg) * p.hp;
+  const int n_heads = min(p.hp, (g + 1) * hpg - h_begin);
+  const int kt0 = MODE == 2 ? tile : 0;               // first 128-wide contraction tile
+  const int nks = MODE == 2 ? 2 - tile : tile + 1;    // number of them
+  const int own = MODE == 2 ? 0 : tile;               // which of V's tiles holds this CTA's own rows
+
+  if (warp == 1 && lane == 0) {
+    mbar_init(bar_r, 1);
+    mbar_init(bar_cb, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 8);
+      mbar_init(g_full(s), 8);
+      mbar_init(acc_full(s), 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(holder, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
+  auto tG = [&](int b) { return tmem + 128u * b; };
+  auto tAcc = [&](int b) { return tmem + 256u + 128u * b; };  // [G V: 64 | R H^T: 64]
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_expect_tx(bar_r, 2 * kTile * (1 + nks));
+      for (int k = 0; k < 2; ++k) {
+        tma_load_2d(sR + k * kTile, &tmR, bar_r, g * CN + 64 * k, c * CQ + tile * 128);
+        for (int i = 0; i < nks; ++i)
+          tma_load_2d(sCol + (2 * i + k) * kTile, &tmCol, bar_r, g * CN + 64 * k, c * CQ + (kt0 + i) * 128);
+      }
+      bool ok = mbar_wait(bar_cb, 0, p.status, kTimeoutProducer);  // stage 0 is free once C B^T is done
+      for (int it = 0; it < n_heads && ok; ++it) {
+        const int s = it & 1, h = h_begin + it;
+        if (!mbar_wait(empty(s), ((it >> 1) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(full(s), kTile * (nks + 1 + (MODE != 0 ? 1 : 0)));
+        for (int i = 0; i < nks; ++i) tma_load_2d(sV(s) + i * kTile, &tmV, full(s), h * CP, c * CQ + (kt0 + i) * 128);
+        for (int k = 0; k < 2; ++k)
+          tma_load_2d(sH(s) + k * (kTile / 2), &tmH, full(s), 64 * k, (c * p.nh + h) * CP);
+        if (MODE != 0) tma_load_2d(sE(s), &tmE, full(s), h * CP, c * CQ + tile * 128);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool ok = mbar_wait(bar_r, 0, p.status, kTimeoutMma);
+      if (ok) {
+        tc_fence_after();
+        const uint32_t idesc = make_idesc_f16(128, 128, FMT, 0, 0);
+        const SmemDescBase a = make_smem_desc_base(sR, 16, 1024);
+        for (int i = 0; i < nks; ++i) {
+          const SmemDescBase b = make_smem_desc_base(sCol + 2 * i * kTile, 16, 1024);
+#pragma unroll
+          for (int ks = 0; ks < CN / 16; ++ks) {
+            const uint32_t off = (ks / 4) * kTile + (ks % 4) * 32;
+            tc_mma_f16(tmem + 128u * i, smem_desc_at(a, off), smem_desc_at(b, off), idesc, ks != 0);
+          }
+        }
+        tc_commit(bar_cb);
+      }
+      const uint32_t idesc_v = make_idesc_f16(128, CP, FMT, 0, 1), idesc_h = make_idesc_f16(128, CP, FMT, 0, 0);
+      const SmemDescBase r = make_smem_desc_base(sR, 16, 1024);
+      for (int it = 0; it < n_heads && ok; ++it) {
+        const int s = it & 1;
+        if (!mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutMma)) break;
+        if (!mbar_wait(g_full(s), (it >> 1) & 1, p.status, kTimeoutMma)) break;
+        tc_fence_after();
+        const SmemDescBase v = make_smem_desc_base(sV(s), 8192, 1024), hd = make_smem_desc_base(sH(s), 16, 1024);
+        for (int ks = 0; ks < nks * 8; ++ks)
+          tc_mma_f16_ts(tAcc(s), tG(s) + ks * 8, smem_desc_at(v, ks * 2048), idesc_v, ks != 0);
+#pragma unroll
+        for (int ks = 0; ks < CN / 16; ++ks)
+          tc_mma_f16(tAcc(s) + 64u, smem_desc_at(r, (ks / 4) * kTile + (ks % 4) * 32),
+                     smem_desc_at(hd, (ks / 4) * (kTile / 2) + (ks % 4) * 32), idesc_h, ks != 0);
+        tc_commit(acc_full(s));
+      }
+    }
+  } else {
+    const int quarter = warp & 3, chalf = (warp - 2) >> 2;
+    const int ctid = threadIdx.x - 64;
+    const int row = quarter * 32 + lane;
+    const int pos = tile * 128 + row;              // position in the chunk
+    const int rbase = tile * 128 + quarter * 32;   // first position of this warp's rows
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const float* Lg = p.Lt + ((long long)c * p.nh + h_begin) * CQ + ctid;
+    const float* dg = p.dtt + ((long long)c * p.nh + h_begin) * CQ + ctid;
+    float nL = Lg[0], nd = dg[0];
+    // C B^T of this row, blocks of 32 columns taken in turn by the two column halves (their causal work is then equal)
+    uint32_t cb[4][16];
+    bool ok = mbar_wait(bar_cb, 0, p.status, kTimeoutEpilogue);
+    if (ok) {
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < 2 * nks) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem + lane_addr + (2 * i + chalf) * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) cb[i][j] = pack2f<FMT>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        }
+      }
+      tc_fence_before();
+    }
+    auto build = [&](int it) {
+      const HeadScalars& q = hs[it % 3];
+      const float Lrow = q.L[pos], drow = MODE == 2 ? q.d[pos] : 1.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= 2 * nks) break;
+        const int b = 2 * i + chalf, col0 = kt0 * 128 + b * 32;
+        uint32_t pk[16];
+        if (MODE == 2 ? col0 < rbase : col0 > rbase) {  // wholly above the diagonal
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = 0u;
+        } else {
+#pragma unroll
+          for (int gq = 0; gq < 4; ++gq) {
+            const int cg = col0 + gq * 8;
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) unpack2<FMT>(cb[i][gq * 4 + j], f[2 * j], f[2 * j + 1]);
+            if (q.ok[cg >> 3]) {
+              const float Lref = q.L[cg];
+              const float e = MODE == 2 ? __expf(Lref - Lrow) * drow : __expf(Lrow - Lref);
+              const uint64_t e2 = pack_f32x2(e, e);
+              const float4 c0 = *reinterpret_cast<const float4*>(&q.cf[cg]), c1 = *reinterpret_cast<const float4*>(&q.cf[cg + 4]);
+              unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[0], f[1]), e2), pack_f32x2(c0.x, c0.y)), f[0], f[1]);
+              unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[2], f[3]), e2), pack_f32x2(c0.z, c0.w)), f[2], f[3]);
+              unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[4], f[5]), e2), pack_f32x2(c1.x, c1.y)), f[4], f[5]);
+              unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[6], f[7]), e2), pack_f32x2(c1.z, c1.w)), f[6], f[7]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                f[j] *= MODE == 2 ? __expf(q.L[cg + j] - Lrow) * drow : __expf(Lrow - q.L[cg + j]) * q.d[cg + j];
+            }
+            if (col0 == rbase) {  // the diagonal block
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (MODE == 2 ? gq * 8 + j < lane : gq * 8 + j > lane) f[j] = 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) pk[gq * 4 + j] = pack2f<FMT>(f[2 * j], f[2 * j + 1]);
+          }
+        }
+        tmem_st_32x16(tG(it & 1) + lane_addr + b * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(g_full(it & 1));
+    };
+    publish<MODE>(hs[0], ctid, nL, nd);
+    if (n_heads > 1) {
+      nL = Lg[CQ];
+      nd = dg[CQ];
+    }
+    compute_sync(1);  // scalars of the first head are there, and C B^T has been read everywhere: G may overwrite it
+    tc_fence_after();
+    if (ok) build(0);
+    for (int it = 0; it < n_heads; ++it) {
+      const int s = it & 1, h = h_begin + it;
+      const bool more = it + 1 < n_heads;
+      if (more) {
+        publish<MODE>(hs[(it + 1) % 3], ctid, nL, nd);
+        if (it + 2 < n_heads) {
+          nL = Lg[(it + 2) * CQ];
+          nd = dg[(it + 2) * CQ];
+        }
+      }
+      compute_sync(1);  // also orders the reuse of sOut and sdot
+      if (more && ok) build(it + 1);
+      if (ok) ok = mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+      if (ok) ok = mbar_wait(acc_full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+      const HeadScalars& q = hs[it % 3];
+      if (ok) {
+        tc_fence_after();
+        const float Lrow = q.L[pos];
+        // weight of the second product: exp(L_t) for rows t, w_s for rows s
+        const float e = MODE == 2 ? __expf(q.L[CQ - 1] - Lrow) * q.d[pos] : __expf(Lrow);
+        const float dh = MODE == 1 ? 0.f : p.D[h];
+        float d0 = 0.f, d1 = 0.f, d2 = 0.f;
+        uint32_t ra[16], ri[16];
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+          if ((ch & 1) == 0) {  // 16 columns of each product at a time: C B^T keeps 64 registers busy
+            tmem_ld_32x16(tAcc(s) + lane_addr + chalf * 32 + ch * 8, ra);
+            tmem_ld_32x16(tAcc(s) + lane_addr + 64 + chalf * 32 + ch * 8, ri);
+            tmem_ld_wait();
+          }
+          const uint32_t off = swz(row, chalf * 4 + ch);
+          const uint4 u = lds128(sV(s) + own * kTile + off);
+          const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
+          uint4 e4 = make_uint4(0u, 0u, 0u, 0u);
+          if (MODE != 0) e4 = lds128(sE(s) + off);
+          const uint32_t ew[4] = {e4.x, e4.y, e4.z, e4.w};
+          uint32_t ow[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float v0, v1, x0 = 0.f, x1 = 0.f;
+            unpack2<FMT>(uw[j], v0, v1);
+            if (MODE != 0) unpack2<FMT>(ew[j], x0, x1);
+            const int k = (ch & 1) * 8 + j * 2;
+            const float a0 = __uint_as_float(ra[k]), a1 = __uint_as_float(ra[k + 1]);
+            const float i0 = e * __uint_as_float(ri[k]), i1 = e * __uint_as_float(ri[k + 1]);
+            if (MODE == 1) {
+              d0 += x0 * (a0 + i0) + x1 * (a1 + i1);
+            } else {
+              ow[j] = pack2f<FMT>(a0 + i0 + dh * v0, a1 + i1 + dh * v1);
+              if (MODE == 2) {
+                d0 += v0 * x0 + v1 * x1;
+                d1 += i0 * x0 + i1 * x1;
+                d2 += a0 * x0 + a1 * x1;
+              }
+            }
+          }
+          if (MODE != 1) sts128(sOut + (it & 1) * kTile + off, ow[0], ow[1], ow[2], ow[3]);
+        }
+        if (MODE != 0) {
+          float* sd = sdot + (it & 1) * 768 + chalf * 128 + row;
+          sd[0] = d0;
+          if (MODE == 2) {
+            sd[256] = d1;
+            sd[512] = d2;
+          }
+        }
+        if (MODE != 1) fence_proxy_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty(s));
+      }
+      compute_sync(2);
+      if (ok && MODE != 1 && ctid == 0) {
+        tma_store_2d(&tmOut, sOut + (it & 1) * kTile, h * CP, c * CQ + tile * 128);
+        tma_store_commit();
+        tma_store_wait_read<1>();
+      }
+      if (ok && MODE != 0) {
+        const long long o = ((long long)c * p.nh + h) * CQ + tile * 128;
+        const float* sd = sdot + (it & 1) * 768;
+        const long long plane = (long long)p.nc * p.nh * CQ;
+        for (int i = ctid; i < (MODE == 2 ? 384 : 128); i += 256) {
+          const int k = i >> 7, r = i & 127;
+          p.red[k * plane + o + r] = sd[k * 256 + r] + sd[k * 256 + 128 + r];
+        }
+      }
+    }
+    if (MODE != 1 && ctid == 0) tma_store_wait<0>();
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// ----------------------------------------------------------------------------------------
+// State kernel.  grid (nc, G * splits), hp heads in turn.  V [256, 64] of a head (x or dy) is scaled by a factor per row
+// IN PLACE in shared memory (rounded to 16 bits as the separate pass did), then serves both products:
+//   STATE:  S^T [128 n, 64 p] = R^T V        R = B or C of the chunk, MN-major       -> S [nc, nh, 64, 128] fp32
+//   ACC:    acc [256 t, 128 n] += V H        H [64, 128] = entering state or dS, summed over the CTA's heads in
+//                                            tensor memory                            -> part [splits, T, G*128] fp32
+// ----------------------------------------------------------------------------------------
+constexpr int kStateStage = 3 * kTile;  // V, H
+template <bool STATE>
+constexpr int state_smem() {
+  return (STATE ? 4 * kTile : 0) + 2 * kStateStage + 1024 + 256;
+}
+
+template <int FMT, bool STATE, bool ACC>
+__global__ void __launch_bounds__(320, 1)
+ssd_state_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmV,
+                 const __grid_constant__ CUtensorMap tmH, const ScanParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t sR = base;  // two 64-column halves of 256 rows
+  const uint32_t st0 = base + (STATE ? 4 * kTile : 0);
+  auto sV = [&](int s) { return st0 + s * kStateStage; };
+  auto sH = [&](int s) { return st0 + s * kStateStage + 2 * kTile; };
+  const uint32_t bars = st0 + 2 * kStateStage;
+  const uint32_t bar_r = bars;
+  auto full = [&](int s) { return bars + 8u + 8u * s; };
+  auto ready = [&](int s) { return bars + 24u + 8u * s; };
+  auto done = [&](int s) { return bars + 40u + 8u * s; };
+  const uint32_t holder = bars + 56u;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x;
+  const int hpg = p.nh / p.G, spg = gridDim.y / p.G;
+  const int g = blockIdx.y / spg, sp = blockIdx.y % spg;
+  const int h_begin = g * hpg + sp * p.hp;
+  const int n_heads = min(p.hp, (g + 1) * hpg - h_begin);
+
+  if (warp == 1 && lane == 0) {
+    mbar_init(bar_r, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(ready(s), 8);
+      mbar_init(done(s), 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(holder, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
+
+  if (warp == 0) {
+    if (lane == 0) {
+      if (STATE) {
+        mbar_expect_tx(bar_r, 4 * kTile);
+        for (int k = 0; k < 2; ++k)
+          for (int i = 0; i < 2; ++i)
+            tma_load_2d(sR + (2 * k + i) * kTile, &tmR, bar_r, g * CN + 64 * k, c * CQ + 128 * i);
+      }
+      for (int it = 0; it < n_heads; ++it) {
+        const int s = it & 1, h = h_begin + it;
+        if (!mbar_wait(done(s), ((it >> 1) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(full(s), (2 + (ACC ? 1 : 0)) * kTile);
+        for (int i = 0; i < 2; ++i) tma_load_2d(sV(s) + i * kTile, &tmV, full(s), h * CP, c * CQ + 128 * i);
+        if (ACC)
+          for (int k = 0; k < 2; ++k) tma_load_2d(sH(s) + k * (kTile / 2), &tmH, full(s), 64 * k, (c * p.nh + h) * CP);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool ok = !STATE || mbar_wait(bar_r, 0, p.status, kTimeoutMma);
+      const uint32_t idesc_s = make_idesc_f16(128, CP, FMT, 1, 1), idesc_a = make_idesc_f16(128, CN, FMT, 0, 1);
+      for (int it = 0; it < n_heads && ok; ++it) {
+        const int s = it & 1;
+        if (!mbar_wait(ready(s), (it >> 1) & 1, p.status, kTimeoutMma)) break;
+        tc_fence_after();
+        if (STATE) {
+          const SmemDescBase a = make_smem_desc_base(sR, 2 * kTile, 1024), b = make_smem_desc_base(sV(s), 8192, 1024);
+#pragma unroll
+          for (int ks = 0; ks < CQ / 16; ++ks)
+            tc_mma_f16(tmem + 64u * s, smem_desc_at(a, ks * 2048), smem_desc_at(b, ks * 2048), idesc_s, ks != 0);
+        }
+        if (ACC) {
+          const SmemDescBase b = make_smem_desc_base(sH(s), kTile / 2, 1024);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const SmemDescBase a = make_smem_desc_base(sV(s) + i * kTile, 16, 1024);
+#pragma unroll
+            for (int ks = 0; ks < CP / 16; ++ks)
+              tc_mma_f16(tmem + 128u + 128u * i, smem_desc_at(a, ks * 32), smem_desc_at(b, ks * 2048), idesc_a, (it | ks) != 0);
+          }
+        }
+        tc_commit(done(s));
+      }
+    }
+  } else {
+    const int quarter = warp & 3, chalf = (warp - 2) >> 2;
+    const int ctid = threadIdx.x - 64;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const long long lb = ((long long)c * p.nh + h_begin) * CQ;
+    bool ok = true;
+    float nL = p.Lt[lb + ctid], nd = p.dtt[lb + ctid], nT = p.Lt[lb + CQ - 1];
+    auto scale = [&](int it) {
+      const int s = it & 1;
+      const float w = p.wmode == 0 ? __expf(nT - nL) * nd : __expf(nL);
+      if (it + 1 < n_heads) {
+        const long long o = lb + (long long)(it + 1) * CQ;
+        nL = p.Lt[o + ctid];
+        nd = p.dtt[o + ctid];
+        nT = p.Lt[o + CQ - 1];
+      }
+      if (ok) ok = mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+      if (!ok) return;
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        const uint32_t a = sV(s) + swz(ctid, ch);
+        uint4 u = lds128(a);
+        uint32_t uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float v0, v1;
+          unpack2<FMT>(uw[j], v0, v1);
+          uw[j] = pack2f<FMT>(v0 * w, v1 * w);
+        }
+        sts128(a, uw[0], uw[1], uw[2], uw[3]);
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ready(s));
+    };
+    scale(0);
+    for (int it = 0; it < n_heads && ok; ++it) {
+      const int s = it & 1, h = h_begin + it;
+      if (it + 1 < n_heads) scale(it + 1);
+      if (STATE) {
+        if (ok) ok = mbar_wait(done(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[32];
+        tmem_ld_32x32(tmem + lane_addr + 64u * s + chalf * 32, r);
+        tmem_ld_wait();
+        float* out = p.S + (((long long)c * p.nh + h) * CP + chalf * 32) * CN + quarter * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) out[i * CN] = __uint_as_float(r[i]);
+      }
+    }
+    if (ACC) {
+      const int last = n_heads - 1;
+      if (ok && mbar_wait(done(last & 1), (last >> 1) & 1, p.status, kTimeoutEpilogue)) {
+        tc_fence_after();
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+          const long long t = (long long)c * CQ + i * 128 + quarter * 32 + lane;
+          float* out = p.part + ((long long)sp * p.T + t) * (p.G * CN) + g * CN + chalf * 64;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem + lane_addr + 128u + 128u * i + chalf * 64 + k * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<uint4*>(out + k * 32 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// ----------------------------------------------------------------------------------------
+// dCB.  grid (nc * 3, G * splits): tile pair (t, s) in {(0,0), (1,0), (1,1)}, hp heads in turn.  dy x^T [128, 128] of a
+// head (fp32 in tensor memory, two buffers) is weighted by the decay and summed in 64 registers a thread.
+// part [splits, nc*G*3, 128, 128] fp32; elements above the diagonal are zeroed by the reduction that follows.
+// ----------------------------------------------------------------------------------------
+constexpr int kDcbStages = 4;
+constexpr int kDcbSmem = kDcbStages * 2 * kTile + 3 * (int)sizeof(HeadScalars) + 1024 + 256;
+
+template <int FMT>
+__global__ void __launch_bounds__(320, 1)
+ssd_dcb_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUtensorMap tmX, const ScanParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  auto sA = [&](int s) { return base + s * 2 * kTile; };
+  auto sB = [&](int s) { return base + s * 2 * kTile + kTile; };
+  const uint32_t scal = base + kDcbStages * 2 * kTile;
+  const uint32_t bars = scal + 3 * (uint32_t)sizeof(HeadScalars);
+  auto full = [&](int s) { return bars + 8u * s; };
+  auto empty = [&](int s) { return bars + 32u + 8u * s; };
+  auto dg_full = [&](int b) { return bars + 64u + 8u * b; };
+  auto dg_empty = [&](int b) { return bars + 80u + 8u * b; };
+  const uint32_t holder = bars + 96u;
+  HeadScalars* hs = reinterpret_cast<HeadScalars*>(smem_raw + (scal - smem_u32(smem_raw)));
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x / 3, pair = blockIdx.x % 3;
+  const int tt = pair > 0 ? 1 : 0, ts = pair == 2 ? 1 : 0;
+  const int hpg = p.nh / p.G, spg = gridDim.y / p.G;
+  const int g = blockIdx.y / spg, sp = blockIdx.y % spg;
+  const int h_begin = g * hpg + sp * p.hp;
+  const int n_heads = min(p.hp, (g + 1) * hpg - h_begin);
+
+  if (warp == 1 && lane == 0) {
+    for (int s = 0; s < kDcbStages; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(dg_full(b), 1);
+      mbar_init(dg_empty(b), 8);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(holder, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int it = 0; it < n_heads; ++it) {
+        const int s = it % kDcbStages, h = h_begin + it;
+        if (!mbar_wait(empty(s), ((it / kDcbStages) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(full(s), 2 * kTile);
+        tma_load_2d(sA(s), &tmDy, full(s), h * CP, c * CQ + tt * 128);
+        tma_load_2d(sB(s), &tmX, full(s), h * CP, c * CQ + ts * 128);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = make_idesc_f16(128, 128, FMT, 0, 0);
+      for (int it = 0; it < n_heads; ++it) {
+        const int s = it % kDcbStages, b = it & 1;
+        if (!mbar_wait(full(s), (it / kDcbStages) & 1, p.status, kTimeoutMma)) break;
+        if (!mbar_wait(dg_empty(b), ((it >> 1) & 1) ^ 1u, p.status, kTimeoutMma)) break;
+        tc_fence_after();
+        const SmemDescBase a = make_smem_desc_base(sA(s), 16, 1024), bb = make_smem_desc_base(sB(s), 16, 1024);
+#pragma unroll
+        for (int ks = 0; ks < CP / 16; ++ks)
+          tc_mma_f16(tmem + 128u * b, smem_desc_at(a, ks * 32), smem_desc_at(bb, ks * 32), idesc, ks != 0);
+        tc_commit(empty(s));
+        tc_commit(dg_full(b));
+      }
+    }
+  } else {
+    const int quarter = warp & 3, chalf = (warp - 2) >> 2;
+    const int ctid = threadIdx.x - 64;
+    const int row = quarter * 32 + lane;
+    const int pos = tt * 128 + row, col0 = ts * 128 + chalf * 64;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const float* Lg = p.Lt + ((long long)c * p.nh + h_begin) * CQ + ctid;
+    const float* dg = p.dtt + ((long long)c * p.nh + h_begin) * CQ + ctid;
+    float nL = Lg[0], nd = dg[0];
+    uint64_t acc[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc[j] = 0ull;
+    bool ok = true;
+    for (int it = 0; it < n_heads; ++it) {
+      const int b = it & 1;
+      HeadScalars& q = hs[it % 3];
+      publish<0>(q, ctid, nL, nd);
+      if (it + 1 < n_heads) {
+        nL = Lg[(it + 1) * CQ];
+        nd = dg[(it + 1) * CQ];
+      }
+      compute_sync(1);
+      if (ok) ok = mbar_wait(dg_full(b), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+      if (!ok) continue;
+      tc_fence_after();
+      const float Lrow = q.L[pos];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem + 128u * b + lane_addr + chalf * 64 + k * 32, r);
+        tmem_ld_wait();
+        if (k == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dg_empty(b));
+        }
+#pragma unroll
+        for (int gq = 0; gq < 4; ++gq) {
+          const int cg = col0 + k * 32 + gq * 8;
+          uint64_t* ac = acc + k * 16 + gq * 4;
+          if (q.ok[cg >> 3]) {
+            const float e = __expf(Lrow - q.L[cg]);
+            const uint64_t e2 = pack_f32x2(e, e);
+            const float4 c0 = *reinterpret_cast<const float4*>(&q.cf[cg]), c1 = *reinterpret_cast<const float4*>(&q.cf[cg + 4]);
+            const uint64_t cf[4] = {pack_f32x2(c0.x, c0.y), pack_f32x2(c0.z, c0.w), pack_f32x2(c1.x, c1.y), pack_f32x2(c1.z, c1.w)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              ac[j] = fma_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(r[gq * 8 + 2 * j]), __uint_as_float(r[gq * 8 + 2 * j + 1])), e2),
+                                cf[j], ac[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float w0 = __expf(Lrow - q.L[cg + 2 * j]) * q.d[cg + 2 * j];
+              const float w1 = __expf(Lrow - q.L[cg + 2 * j + 1]) * q.d[cg + 2 * j + 1];
+              ac[j] = fma_f32x2(pack_f32x2(__uint_as_float(r[gq * 8 + 2 * j]), __uint_as_float(r[gq * 8 + 2 * j + 1])),
+                                pack_f32x2(w0, w1), ac[j]);
+            }
+          }
+        }
+      }
+    }
+    if (ok) {
+      float* out = p.part + (((long long)sp * p.nc + c) * p.G + g) * (3 * 128 * 128) + (pair * 128 + row) * 128 + chalf * 64;
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        float4 v;
+        unpack_f32x2(acc[j], v.x, v.y);
+        unpack_f32x2(acc[j + 1], v.z, v.w);
+        *reinterpret_cast<float4*>(out + 2 * j) = v;
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
+}
+
+// dCB in 16 bits, [nc*G, 256, 256], zero above the diagonal: the sum of the head splits' partial tiles.
+// grid nc*G*32, block 256: eight rows per CTA, eight columns per thread.
+template <int FMT>
+__global__ void __launch_bounds__(256) ssd_dcb_reduce_kernel(const float* __restrict__ part, uint4* __restrict__ out, int splits,
+                                                             long long tiles) {
+  const int m = blockIdx.x >> 5;
+  const int t = (blockIdx.x & 31) * 8 + (threadIdx.x >> 5), s0 = (threadIdx.x & 31) * 8;
+  float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (s0 <= t) {
+    const int pair = t < 128 ? 0 : (s0 < 128 ? 1 : 2);
+    const float* src = part + (long long)m * 49152 + (pair * 128 + (t & 127)) * 128 + (s0 & 127);
+    for (int k = 0; k < splits; ++k) {
+      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+      f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+      f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+      src += tiles * 49152;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (s0 + j > t) f[j] = 0.f;
+  }
+  out[((long long)m * CQ + t) * 32 + (threadIdx.x & 31)] = make_uint4(pack2f<FMT>(f[0], f[1]), pack2f<FMT>(f[2], f[3]),
+                                                                      pack2f<FMT>(f[4], f[5]), pack2f<FMT>(f[6], f[7]));
+}
+
+// out (16-bit) = sum of `splits` fp32 partials of n elements + add (fp32); eight elements per thread.
+template <int FMT>
+__global__ void __launch_bounds__(256) ssd_sum_kernel(const float* __restrict__ part, const float* __restrict__ add,
+                                                      uint4* __restrict__ out, int splits, long long n) {
+  const long long i = (blockIdx.x * 256LL + threadIdx.x) * 8;
+  if (i >= n) return;
+  float4 a = *reinterpret_cast<const float4*>(add + i), b = *reinterpret_cast<const float4*>(add + i + 4);
+  for (int k = 0; k < splits; ++k) {
+    const float4 u = *reinterpret_cast<const float4*>(part + k * n + i), v = *reinterpret_cast<const float4*>(part + k * n + i + 4);
+    a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+    b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+  }
+  out[i >> 3] = make_uint4(pack2f<FMT>(a.x, a.y), pack2f<FMT>(a.z, a.w), pack2f<FMT>(b.x, b.y), pack2f<FMT>(b.z, b.w));
+}
+
+// ----------------------------------------------------------------------------------------
+// Decay bookkeeping: a warp per head, eight positions per lane.  grid (nc, ceil(nh / 8)), block 256.
+// ----------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) ssd_decay_kernel(const float* __restrict__ dt, const float* __restrict__ A,
+                                                        float* __restrict__ Lt, float* __restrict__ dtt,
+                                                        float* __restrict__ Ltot, int nh) {
+  __shared__ float sd[8][CQ + 4];
+  const int c = blockIdx.x, h0 = blockIdx.y * 8;
+  for (int i = threadIdx.x; i < CQ * 8; i += 256) {
+    const int t = i >> 3, h = i & 7;
+    sd[h][t] = h0 + h < nh ? dt[((long long)c * CQ + t) * nh + h0 + h] : 0.f;
+  }
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + w;
+  if (h >= nh) return;
+  const float a = A[h];
+  float d[8], s[8], run = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    d[j] = sd[w][lane * 8 + j];
+    run += d[j] * a;
+    s[j] = run;
+  }
+  float inc = run;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  float before = __shfl_up_sync(0xffffffffu, inc, 1);
+  if (lane == 0) before = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s[j] += before;
+  const long long o = ((long long)c * nh + h) * CQ + lane * 8;
+  *reinterpret_cast<float4*>(Lt + o) = make_float4(s[0], s[1], s[2], s[3]);
+  *reinterpret_cast<float4*>(Lt + o + 4) = make_float4(s[4], s[5], s[6], s[7]);
+  *reinterpret_cast<float4*>(dtt + o) = make_float4(d[0], d[1], d[2], d[3]);
+  *reinterpret_cast<float4*>(dtt + o + 4) = make_float4(d[4], d[5], d[6], d[7]);
+  if (lane == 31) Ltot[(long long)c * nh + h] = s[7];
+}
+
+// Gradients through the decay.  yd = dy . (y - D x), dww = w x.(B dS^T), col = x.(G^T dy), dyx = dy . x per (chunk, head,
+// position).  dL = yd - dww - col (+ dLtot and the sum of dww at the last position); through L = cumsum(dt A) that is a
+// reverse cumulative sum da; ddt = (dww + col) / dt + da A; partial dA = sum da dt and dD = sum dyx per (chunk, head).
+__global__ void __launch_bounds__(256) ssd_decay_bwd_kernel(const float* __restrict__ yd, const float* __restrict__ red,
+                                                            const float* __restrict__ dtt, const float* __restrict__ A,
+                                                            const float* __restrict__ dLtot, float* __restrict__ ddt,
+                                                            float* __restrict__ sums, int nc, int nh) {
+  __shared__ float sd[8][CQ + 4];
+  const int c = blockIdx.x, h0 = blockIdx.y * 8;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + w;
+  const long long plane = (long long)nc * nh * CQ;
+  if (h < nh) {
+    const long long o = ((long long)c * nh + h) * CQ + lane * 8;
+    auto ld = [](const float* q, float (&f)[8]) {
+      const float4 u = *reinterpret_cast<const float4*>(q), v = *reinterpret_cast<const float4*>(q + 4);
+      f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w;
+      f[4] = v.x; f[5] = v.y; f[6] = v.z; f[7] = v.w;
+    };
+    float y[8], k[8], ww[8], co[8], d[8];
+    ld(yd + o, y);
+    ld(red + o, k);
+    ld(red + plane + o, ww);
+    ld(red + 2 * plane + o, co);
+    ld(dtt + o, d);
+    float sw = 0.f, sk = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      sw += ww[j];
+      sk += k[j];
+    }
+    sw = warp_sum(sw);
+    sk = warp_sum(sk);
+    const float a = A[h];
+    float dl[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dl[j] = y[j] - ww[j] - co[j];
+    if (lane == 31) dl[7] += dLtot[(long long)c * nh + h] + sw;
+    float run = 0.f;
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      run += dl[j];
+      dl[j] = run;
+    }
+    float inc = run;
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1) {
+      const float v = __shfl_down_sync(0xffffffffu, inc, q);
+      if (lane + q < 32) inc += v;
+    }
+    float after = __shfl_down_sync(0xffffffffu, inc, 1);
+    if (lane == 31) after = 0.f;
+    float sa = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float da = dl[j] + after;
+      sa += da * d[j];
+      sd[w][lane * 8 + j] = (ww[j] + co[j]) / d[j] + da * a;
+    }
+    sa = warp_sum(sa);
+    if (lane == 0) {
+      sums[(long long)c * nh + h] = sa;
+      sums[(long long)nc * nh + (long long)c * nh + h] = sk;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < CQ * 8; i += 256) {
+    const int t = i >> 3, k = i & 7;
+    if (h0 + k < nh) ddt[((long long)c * CQ + t) * nh + h0 + k] = sd[k][t];
+  }
+}
+
+}  // namespace ssdf
+}  // namespace fmsb
+
+using namespace fmsb;
+using namespace fmsb::ssdf;
+
+// Heads per CTA: the split of a group's heads for which the machine (148 SMs, one CTA each) finishes first, a CTA
+// costing its heads plus about two heads' worth of prologue and drain.
+static int pick_heads(long long tiles, int hpg) {
+  long long best = -1;
+  int hp = hpg;
+  for (int spg = 1; spg <= hpg; ++spg) {
+    const int n = (hpg + spg - 1) / spg;
+    if ((hpg + n - 1) / n != spg) continue;
+    const long long cost = (tiles * spg + 147) / 148 * (n + 2);
+    if (best < 0 || cost < best) { best = cost; hp = n; }
+  }
+  return hp;
+}
+
+// kind 0: scan tiles (2 per chunk and group), 1: state kernel (1), 2: dCB (3).  Returns heads per CTA.
+extern "C" int fmsb_ssdf_heads(int kind, int nc, int nh, int G) {
+  if (nc <= 0 || G <= 0 || nh % G) return 1;
+  return pick_heads((long long)nc * G * (kind == 0 ? 2 : kind == 1 ? 1 : 3), nh / G);
+}
+
+static int map_rows(CUtensorMap* m, const void* p, long long rows, long long cols, long long ld, int box_rows) {
+  return fmsb_host::make_tmap_2d_16b(m, p, rows, cols, ld, box_rows, 64);
+}
+
+template <typename K>
+static int set_smem(K kern, int bytes) {
+  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+// mode 0: out = y (v = x, r = C, col = B, hst = entering states); mode 1: red = dy . y-terms (e = dy);
+// mode 2: out = dx and red (v = dy, r = B, col = C, hst = dS, e = x).  v, e, out [nc*256, nh*64] dense; r, col rows of
+// G*128 with leading dimensions ldr / ldc; hst [nc*nh*64, 128].
+extern "C" int fmsb_ssdf_scan(int mode, const void* r, long long ldr, const void* col, long long ldc, const void* v,
+                              const void* hst, const void* e, void* out, const float* Lt, const float* dtt, const float* D,
+                              float* red, int nc, int nh, int G, int hp, int fmt, int* status, cudaStream_t stream) {
+  if (nc <= 0) return 0;
+  if (nh % G || hp <= 0 || (ldr % 8) || (ldc % 8) || fmt < 0 || fmt > 1 || mode < 0 || mode > 2) return -2;
+  const long long T = (long long)nc * CQ;
+  CUtensorMap tr, tc, tv, th, te, to;
+  int rc;
+  if ((rc = map_rows(&tr, r, T, (long long)G * CN, ldr, 128))) return rc;
+  if ((rc = map_rows(&tc, col, T, (long long)G * CN, ldc, 128))) return rc;
+  if ((rc = map_rows(&tv, v, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  if ((rc = map_rows(&th, hst, (long long)nc * nh * CP, CN, CN, 64))) return rc;
+  te = tv;
+  to = tv;
+  if (mode != 0 && (rc = map_rows(&te, e, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  if (mode != 1 && (rc = map_rows(&to, out, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  ScanParams p{};
+  p.nc = nc; p.nh = nh; p.G = G; p.hp = hp; p.Lt = Lt; p.dtt = dtt; p.D = D; p.red = red; p.T = (int)T; p.status = status;
+  const int hpg = nh / G;
+  const dim3 grid(nc * 2, G * ((hpg + hp - 1) / hp));
+#define FMSB_SCAN(MM, FF)                                                                              \
+  do {                                                                                                 \
+    static bool cfg = false;                                                                           \
+    if (!cfg) {                                                                                        \
+      if ((rc = set_smem(ssd_scan_kernel<MM, FF>, kScanSmem))) return rc;                              \
+      cfg = true;                                                                                      \
+    }                                                                                                  \
+    ssd_scan_kernel<MM, FF><<<grid, 320, kScanSmem, stream>>>(tr, tc, tv, th, te, to, p);              \
+  } while (0)
+  if (fmt == 1) { if (mode == 0) FMSB_SCAN(0, 1); else if (mode == 1) FMSB_SCAN(1, 1); else FMSB_SCAN(2, 1); }
+  else { if (mode == 0) FMSB_SCAN(0, 0); else if (mode == 1) FMSB_SCAN(1, 0); else FMSB_SCAN(2, 0); }
+#undef FMSB_SCAN
+  return (int)cudaGetLastError();
+}
+
+// S (may be null) [nc, nh, 64, 128] = (v w)^T r; part (may be null) [splits, T, G*128] = sum over heads of (v w) hst.
+extern "C" int fmsb_ssdf_state(const void* r, long long ldr, const void* v, const void* hst, const float* Lt,
+                               const float* dtt, float* S, float* part, int wmode, int nc, int nh, int G, int hp, int fmt,
+                               int* status, cudaStream_t stream) {
+  if (nc <= 0) return 0;
+  if (nh % G || hp <= 0 || fmt < 0 || fmt > 1 || (S == nullptr && part == nullptr) || (S != nullptr && (ldr % 8))) return -2;
+  const long long T = (long long)nc * CQ;
+  CUtensorMap tr, tv, th;
+  int rc;
+  if ((rc = map_rows(&tv, v, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  tr = tv;
+  th = tv;
+  if (S != nullptr && (rc = map_rows(&tr, r, T, (long long)G * CN, ldr, 128))) return rc;
+  if (part != nullptr && (rc = map_rows(&th, hst, (long long)nc * nh * CP, CN, CN, 64))) return rc;
+  ScanParams p{};
+  p.nc = nc; p.nh = nh; p.G = G; p.hp = hp; p.Lt = Lt; p.dtt = dtt; p.S = S; p.part = part; p.wmode = wmode; p.T = (int)T;
+  p.status = status;
+  const int hpg = nh / G;
+  const dim3 grid(nc, G * ((hpg + hp - 1) / hp));
+#define FMSB_STATE(FF, SS, AA)                                                                   \
+  do {                                                                                           \
+    static bool cfg = false;                                                                     \
+    if (!cfg) {                                                                                  \
+      if ((rc = set_smem(ssd_state_kernel<FF, SS, AA>, state_smem<SS>()))) return rc;            \
+      cfg = true;                                                                                \
+    }                                                                                            \
+    ssd_state_kernel<FF, SS, AA><<<grid, 320, state_smem<SS>(), stream>>>(tr, tv, th, p);        \
+  } while (0)
+  if (fmt == 1) {
+    if (S && part) FMSB_STATE(1, true, true); else if (S) FMSB_STATE(1, true, false); else FMSB_STATE(1, false, true);
+  } else {
+    if (S && part) FMSB_STATE(0, true, true); else if (S) FMSB_STATE(0, true, false); else FMSB_STATE(0, false, true);
+  }
+#undef FMSB_STATE
+  return (int)cudaGetLastError();
+}
+
+// dcb [nc*G, 256, 256] 16-bit; part: scratch of splits * nc * G * 3 * 128 * 128 floats.
+extern "C" int fmsb_ssdf_dcb(const void* dy, const void* x, const float* Lt, const float* dtt, float* part, void* dcb, int nc,
+                             int nh, int G, int hp, int fmt, int* status, cudaStream_t stream) {
+  if (nc <= 0) return 0;
+  if (nh % G || hp <= 0 || fmt < 0 || fmt > 1) return -2;
+  const long long T = (long long)nc * CQ;
+  CUtensorMap td, tx;
+  int rc;
+  if ((rc = map_rows(&td, dy, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  if ((rc = map_rows(&tx, x, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  ScanParams p{};
+  p.nc = nc; p.nh = nh; p.G = G; p.hp = hp; p.Lt = Lt; p.dtt = dtt; p.part = part; p.T = (int)T; p.status = status;
+  const int spg = (nh / G + hp - 1) / hp;
+  const dim3 grid(nc * 3, G * spg);
+#define FMSB_DCB(FF)                                                                                              \
+  do {                                                                                                            \
+    static bool cfg = false;                                                                                      \
+    if (!cfg) {                                                                                                   \
+      if ((rc = set_smem(ssd_dcb_kernel<FF>, kDcbSmem))) return rc;                                               \
+      cfg = true;                                                                                                 \
+    }                                                                                                             \
+    ssd_dcb_kernel<FF><<<grid, 320, kDcbSmem, stream>>>(td, tx, p);                                               \
+    ssd_dcb_reduce_kernel<FF><<<nc * G * 32, 256, 0, stream>>>(part, (uint4*)dcb, spg, (long long)nc * G);        \
+  } while (0)
+  if (fmt == 1) FMSB_DCB(1);
+  else FMSB_DCB(0);
+#undef FMSB_DCB
+  return (int)cudaGetLastError();
+}
+
+extern "C" int fmsb_ssdf_sum(const float* part, const float* add, void* out, int splits, long long n, int fmt,
+                             cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (n % 8 || fmt < 0 || fmt > 1) return -2;
+  const unsigned blocks = (unsigned)((n / 8 + 255) / 256);
+  if (fmt == 1) ssd_sum_kernel<1><<<blocks, 256, 0, stream>>>(part, add, (uint4*)out, splits, n);
+  else ssd_sum_kernel<0><<<blocks, 256, 0, stream>>>(part, add, (uint4*)out, splits, n);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int fmsb_ssdf_decay(const float* dt, const float* A, float* Lt, float* dtt, float* Ltot, int nc, int nh,
+                               cudaStream_t stream) {
+  if (nc <= 0 || nh <= 0) return 0;
+  ssd_decay_kernel<<<dim3(nc, (nh + 7) / 8), 256, 0, stream>>>(dt, A, Lt, dtt, Ltot, nh);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int fmsb_ssdf_decay_bwd(const float* yd, const float* red, const float* dtt, const float* A, const float* dLtot,
+                                   float* ddt, float* sums, int nc, int nh, cudaStream_t stream) {
+  if (nc <= 0 || nh <= 0) return 0;
+  ssd_decay_bwd_kernel<<<dim3(nc, (nh + 7) / 8), 256, 0, stream>>>(yd, red, dtt, A, dLtot, ddt, sums, nc, nh);
+  return (int)cudaGetLastError();
+}

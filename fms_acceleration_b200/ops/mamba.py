@@ -31,6 +31,13 @@ NV.declare("fmsb_ssd_rowdot", [P_, P_, P_, P_, L_, I_, I_, P_])
 NV.declare("fmsb_ssd_bwd_combine", [P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_fwd", [P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_bwd", [P_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
+NV.declare("fmsb_ssdf_heads", [I_, I_, I_, I_])
+NV.declare("fmsb_ssdf_scan", [I_, P_, L_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, P_, P_])
+NV.declare("fmsb_ssdf_state", [P_, L_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, P_, P_])
+NV.declare("fmsb_ssdf_dcb", [P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, P_, P_])
+NV.declare("fmsb_ssdf_sum", [P_, P_, P_, I_, L_, I_, P_])
+NV.declare("fmsb_ssdf_decay", [P_, P_, P_, P_, P_, I_, I_, P_])
+NV.declare("fmsb_ssdf_decay_bwd", [P_, P_, P_, P_, P_, P_, P_, I_, I_, P_])
 
 
 # ------------------------------------------------------------------------------------------------ oracles
@@ -402,6 +409,186 @@ class _SSDScan(torch.autograd.Function):
                 dD.to(D.dtype), dh0, None, None, None)
 
 
+# ---- the same scan with its decay matrices kept on the chip (csrc/mamba_fused.cu)
+def _fused_ok(x, B, C, Q):
+    """Chunk 256, head dimension 64, state 128 (what the Mamba2 presets use): the tile sizes of the fused kernels.
+    Other shapes take the batched products of :class:`_SSDScan`.  Sizes are bounded by the launch grid."""
+    T, nh, P = x.shape
+    G, N = B.shape[1], B.shape[2]
+    return (Q == 256 and P == 64 and N == 128 and T > 0 and T % Q == 0 and nh > 0 and nh % G == 0 and nh <= 65535
+            and x.dtype in (torch.bfloat16, torch.float16) and B.dtype == x.dtype and C.dtype == x.dtype)
+
+
+class _Fused:
+    """Launches of the fused kernels for one call's geometry."""
+
+    def __init__(self, x2, dt, A, B2, C2, T, nh, G, Q):
+        self.nc, self.nh, self.G, self.T, self.dev, self.dtype = T // Q, nh, G, T, x2.device, x2.dtype
+        self.code, self.st = NV.dtype_code(x2.dtype), NV.status_word(x2.device)
+        self.x2, self.B2, self.C2, self.A = x2, B2, C2, A
+        bk = torch.empty(2, self.nc, nh, Q, dtype=torch.float32, device=self.dev)
+        self.Lt, self.dtt = bk[0], bk[1]
+        self.Ltot = torch.empty(self.nc, nh, dtype=torch.float32, device=self.dev)
+        rc = NV.lib().fmsb_ssdf_decay(dt.data_ptr(), A.data_ptr(), self.Lt.data_ptr(), self.dtt.data_ptr(),
+                                      self.Ltot.data_ptr(), self.nc, nh, NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_decay")
+
+    def heads(self, kind):
+        """(heads per CTA, number of head splits of a group) of a kernel."""
+        hp = NV.lib().fmsb_ssdf_heads(kind, self.nc, self.nh, self.G)
+        return hp, -(-(self.nh // self.G) // hp)
+
+    def scan(self, mode, r, col, v, h, e=None, out=None, D=None, red=None):
+        rc = NV.lib().fmsb_ssdf_scan(mode, r.data_ptr(), r.stride(0), col.data_ptr(), col.stride(0), v.data_ptr(),
+                                     h.data_ptr(), NV.ptr(e), NV.ptr(out), self.Lt.data_ptr(), self.dtt.data_ptr(),
+                                     NV.ptr(D), NV.ptr(red), self.nc, self.nh, self.G, self.heads(0)[0], self.code,
+                                     self.st.data_ptr(), NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_scan")
+
+    def state(self, r, v, wmode, h=None, want_s=True):
+        """``(S, part)``: chunk states ``(v w)^T r`` and, with ``h``, the partial sums over heads of ``(v w) h``."""
+        hp, splits = self.heads(1)
+        S = torch.empty(self.nc * self.nh * 64, 128, dtype=torch.float32, device=self.dev) if want_s else None
+        part = torch.empty(splits, self.T, self.G * 128, dtype=torch.float32, device=self.dev) if h is not None else None
+        rc = NV.lib().fmsb_ssdf_state(r.data_ptr(), r.stride(0), v.data_ptr(), NV.ptr(h), self.Lt.data_ptr(),
+                                      self.dtt.data_ptr(), NV.ptr(S), NV.ptr(part), wmode, self.nc, self.nh, self.G, hp,
+                                      self.code, self.st.data_ptr(), NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_state")
+        return S, part
+
+    def dcb(self, dy2):
+        hp, splits = self.heads(2)
+        part = torch.empty(splits * self.nc * self.G * 3 * 128 * 128, dtype=torch.float32, device=self.dev)
+        out = torch.empty(self.nc * self.G * 256, 256, dtype=self.dtype, device=self.dev)
+        rc = NV.lib().fmsb_ssdf_dcb(dy2.data_ptr(), self.x2.data_ptr(), self.Lt.data_ptr(), self.dtt.data_ptr(),
+                                    part.data_ptr(), out.data_ptr(), self.nc, self.nh, self.G, hp, self.code,
+                                    self.st.data_ptr(), NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_dcb")
+        return out
+
+    def total(self, part, add):
+        out = torch.empty(add.shape, dtype=self.dtype, device=self.dev)
+        rc = NV.lib().fmsb_ssdf_sum(part.data_ptr(), add.data_ptr(), out.data_ptr(), part.shape[0], add.numel(), self.code,
+                                    NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_sum")
+        return out
+
+    def states(self, h0, cp=None, want_zero_start=False):
+        """(hprev, hT, h_in, hprev0): what :func:`_chunk_states` computes, with the same context-parallel hand-off."""
+        S, _ = self.state(self.B2, self.x2, 0)
+        shape = (self.nc * self.nh * 64, 128)
+        hprev0 = None
+        if cp is not None:
+            hprev0 = torch.empty(shape, dtype=self.dtype, device=self.dev)
+            h0 = cp.forward(S, self.Ltot, hprev0, self.nc, self.nh, 64 * 128, self.dtype)
+        elif want_zero_start:
+            hprev0 = torch.empty(shape, dtype=self.dtype, device=self.dev)
+            self._recur(S, None, hprev0, torch.empty(self.nh, 64, 128, dtype=torch.float32, device=self.dev))
+        hprev = torch.empty(shape, dtype=self.dtype, device=self.dev)
+        hT = torch.empty(self.nh, 64, 128, dtype=torch.float32, device=self.dev)
+        h0 = None if h0 is None else h0.float().contiguous()
+        self._recur(S, h0, hprev, hT)
+        return hprev, hT, h0, hprev0
+
+    def _recur(self, S, h0, hprev, hT):
+        rc = NV.lib().fmsb_ssd_state_fwd(S.data_ptr(), self.Ltot.data_ptr(), NV.ptr(h0), hprev.data_ptr(), hT.data_ptr(),
+                                         self.nc, self.nh, 64 * 128, self.code, NV.stream_ptr())
+        NV.check(rc, "fmsb_ssd_state_fwd")
+
+
+class _SSDScanFused(torch.autograd.Function):
+    """:class:`_SSDScan` for the shapes of :func:`_fused_ok`: same arguments, same results."""
+
+    @staticmethod
+    def forward(ctx, x, dt, A, B, C, D, h0, Q, recompute, cp=None):
+        T, nh, P = x.shape
+        G, N = B.shape[1], B.shape[2]
+        x2 = _rows16(x.reshape(T, nh * P))
+        B2, C2 = _vec_rows(B.reshape(T, G * N)), _vec_rows(C.reshape(T, G * N))
+        dt = dt.float().contiguous()
+        k = _Fused(x2, dt, A.float().contiguous(), B2, C2, T, nh, G, Q)
+        if cp is not None:
+            assert h0 is None, "the entering state of a context-parallel slice comes from the earlier ranks"
+        hprev, hT, h_in, hprev0 = k.states(h0, cp)
+        y = torch.empty(T, nh, P, dtype=x.dtype, device=x.device)
+        k.scan(0, C2, B2, x2, hprev, out=y, D=D.float().contiguous())
+        if recompute:
+            ctx.save_for_backward(x, dt, A, B, C, D, h_in if cp is not None else h0)
+        elif cp is not None:
+            ctx.save_for_backward(x, dt, A, B, C, D, hprev, hprev0)
+        else:
+            ctx.save_for_backward(x, dt, A, B, C, D, hprev)
+        ctx.meta = (Q, h0 is not None, recompute)
+        ctx.cp = cp
+        return y, hT
+
+    @staticmethod
+    def backward(ctx, dy, dhT):
+        Q, has_h0, recompute = ctx.meta
+        saved = ctx.saved_tensors
+        x, dt, A, B, C, D = saved[:6]
+        T, nh, P = x.shape
+        G, N = B.shape[1], B.shape[2]
+        nc, dev, dtp, cp = T // Q, x.device, x.dtype, ctx.cp
+        x2 = _rows16(x.reshape(T, nh * P))
+        B2, C2 = _vec_rows(B.reshape(T, G * N)), _vec_rows(C.reshape(T, G * N))
+        dy2 = _rows16(dy.reshape(T, nh * P))
+        A32 = A.float().contiguous()
+        k = _Fused(x2, dt, A32, B2, C2, T, nh, G, Q)
+        hprev0 = None
+        if recompute:
+            hprev, _, _, hprev0 = k.states(saved[6], want_zero_start=cp is not None)
+        elif cp is not None:
+            hprev, hprev0 = saved[6:]
+        else:
+            hprev = saved[6]
+        # dy . (G x + exp(L) C Hprev^T) per (chunk, head, position): the decay's share of the gradient
+        ydot = torch.empty(nc, nh, Q, dtype=torch.float32, device=dev)
+        k.scan(1, C2, B2, x2, hprev, e=dy2, red=ydot)
+        # gradient of the entering states and, through them, of C
+        dhp, dC_part = k.state(C2, dy2, 1, h=hprev)
+        # ---- recurrence backward
+        dS16 = torch.empty(nc * nh * P, N, dtype=dtp, device=dev)
+        dh0 = torch.empty(nh, P, N, dtype=torch.float32, device=dev) if (has_h0 or cp is not None) else None
+        dLtot = torch.zeros(nc, nh, dtype=torch.float32, device=dev)
+        dhTc = None if dhT is None else dhT.float().contiguous()
+        rc = NV.lib().fmsb_ssd_state_bwd(dhp.data_ptr(), NV.ptr(dhTc), k.Ltot.data_ptr(), hprev.data_ptr(),
+                                         dS16.data_ptr(), NV.ptr(dh0), dLtot.data_ptr(), nc, nh, P * N, k.code,
+                                         NV.stream_ptr())
+        NV.check(rc, "fmsb_ssd_state_bwd")
+        del dhp
+        if cp is not None:  # as in _SSDScan.backward
+            dF, dlogP = cp.backward(dh0, nh, P * N)
+            dS16b = torch.empty_like(dS16)
+            rc = NV.lib().fmsb_ssd_state_bwd(None, dF.data_ptr(), k.Ltot.data_ptr(), hprev0.data_ptr(), dS16b.data_ptr(),
+                                             None, dLtot.data_ptr(), nc, nh, P * N, k.code, NV.stream_ptr())
+            NV.check(rc, "fmsb_ssd_state_bwd")
+            dS16 += dS16b
+            del dS16b
+            dLtot += dlogP[None, :]
+            dh0 = None
+        # ---- dx with its three row dot products, dB through the chunk states, dCB and what it gives to B and C
+        dx = torch.empty(T, nh, P, dtype=dtp, device=dev)
+        red = torch.empty(3, nc, nh, Q, dtype=torch.float32, device=dev)
+        k.scan(2, B2, C2, dy2, dS16, e=x2, out=dx, D=D.float().contiguous(), red=red)
+        _, dB_part = k.state(B2, x2, 0, h=dS16, want_s=False)
+        del dS16
+        dcb = k.dcb(dy2)
+        geo = dict(M=Q, N=N, K=Q, n_batch=nc * G, n_inner=G, a_off=(G * Q, Q, 0, 1), b_off=(Q, 0, N, 1), d_off=(Q, 0, N),
+                   b_mn=True, out_rows=T, out_cols=G * N, out_dtype=torch.float32)
+        dC = k.total(dC_part, batched_gemm(dcb, B2, **geo))
+        dB = k.total(dB_part, batched_gemm(dcb, C2, a_mn=True, **geo))
+        # ---- through the decay
+        ddt = torch.empty(T, nh, dtype=torch.float32, device=dev)
+        sums = torch.empty(2, nc, nh, dtype=torch.float32, device=dev)
+        rc = NV.lib().fmsb_ssdf_decay_bwd(ydot.data_ptr(), red.data_ptr(), k.dtt.data_ptr(), A32.data_ptr(),
+                                          dLtot.data_ptr(), ddt.data_ptr(), sums.data_ptr(), nc, nh, NV.stream_ptr())
+        NV.check(rc, "fmsb_ssdf_decay_bwd")
+        dA, dD = sums.sum(1)
+        return (dx, ddt.to(dt.dtype), dA.to(A.dtype), dB.view(T, G, N), dC.view(T, G, N), dD.to(D.dtype), dh0, None, None,
+                None)
+
+
 class _StateCorrection(torch.autograd.Function):
     """y = y0 + exp(Lg) (C . H_in): what a state ``H_in [nh, P, N]`` entering the slice adds to the outputs of a
     zero-initial-state scan ``y0 [T, nh, P]``, with ``Lg`` the cumulative ``dt*A`` from the start of the slice."""
@@ -490,4 +677,5 @@ def ssd_scan(x, dt, A, B, C, D, h0=None, chunk_size=256, recompute=False, cp=Non
     if not x.is_cuda:
         y, h = ssd_ref(x, dt, A, B, C, D, h0)
         return y.to(x.dtype), h.float()
-    return _SSDScan.apply(x, dt, A, B, C, D, h0, chunk_size, bool(recompute), cp)
+    fn = _SSDScanFused if _fused_ok(x, B, C, chunk_size) else _SSDScan
+    return fn.apply(x, dt, A, B, C, D, h0, chunk_size, bool(recompute), cp)

@@ -95,6 +95,46 @@ def test_ssd_scan_matches_recurrence(T, nh, P, G, N, Q, with_h0, monkeypatch):
         assert _rel(h0.grad.cpu(), h0r.grad) < 5e-2
 
 
+@pytest.mark.parametrize("nc,nh,G,dtype,with_h0,recompute,decay", [
+    (1, 1, 1, torch.bfloat16, False, False, "mild"), (3, 6, 2, torch.float16, True, False, "mild"),
+    (2, 5, 1, torch.bfloat16, True, True, "mild"), (2, 4, 1, torch.bfloat16, False, False, "extreme"),
+    (160, 3, 1, torch.bfloat16, False, False, "mild")])
+def test_fused_scan_matches_recurrence_and_general_path(nc, nh, G, dtype, with_h0, recompute, decay):
+    """The fused kernels (chunk 256, head 64, state 128) against the fp64 recurrence and against the general path on the
+    same inputs.  Products round G, the scaled rows and the entering states to 16 bits (half an ulp each, at most three
+    in a row), sums are fp32: 4 ulp of the result in the 2-norm.  ``extreme``: heads that forget within a step, whose
+    decay takes one exponential per element."""
+    torch.manual_seed(nc + nh)
+    T, P, N, Q = nc * 256, 64, 128, 256
+    x = (torch.randn(T, nh, P, device=DEV) * 0.5).to(dtype)
+    dt = torch.rand(T, nh, device=DEV) * 0.09 + 0.01
+    A = torch.tensor([-0.5, -3.0, -16.0, -2000.0], device=DEV) if decay == "extreme" else -(torch.rand(nh, device=DEV) * 3 + 0.5)
+    BC = (torch.randn(T, 2 * G * N, device=DEV) * 0.3).to(dtype)
+    B, C = BC[:, : G * N].view(T, G, N), BC[:, G * N:].view(T, G, N)  # strided rows, as the mixer's split gives them
+    D = torch.randn(nh, device=DEV)
+    ins = [x, dt, A, B, C, D] + ([torch.randn(nh, P, N, device=DEV) * 0.2] if with_h0 else [])
+    gy, gh = torch.randn(T, nh, P, device=DEV).to(dtype), torch.randn(nh, P, N, device=DEV) * 0.1
+
+    def run(fn):
+        t = [v.detach().requires_grad_() for v in ins]
+        y, h = fn(*t[:6], t[6] if with_h0 else None, Q, recompute)
+        return [y, h] + list(torch.autograd.grad([y, h], t, [gy, gh]))
+
+    assert MB._fused_ok(x, B, C, Q) and not MB._fused_ok(x, B, C, 128)
+    got, general = run(MB._SSDScanFused.apply), run(MB._SSDScan.apply)
+    NV.check_status()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    refs = general
+    if nc <= 3:
+        t = [v.detach().double().cpu().requires_grad_() for v in ins]
+        y, h = MB.ssd_ref(*t[:6], t[6] if with_h0 else None)
+        refs = [y, h] + list(torch.autograd.grad([y, h], t, [gy.double().cpu(), gh.double().cpu()]))
+    for i, (a, g, r) in enumerate(zip(got, general, refs)):
+        assert a.dtype == g.dtype and a.shape == g.shape and torch.isfinite(a.float()).all(), i
+        err = _rel(a.cpu(), r.cpu())
+        assert err < 4 * ulp, (i, err, _rel(g.cpu(), r.cpu()))
+
+
 @pytest.mark.parametrize("Q", [64, 256])
 def test_decay_matrix_kernel_with_moderate_and_extreme_decay(Q):
     """G[c, h, t, s] = CB[c, g, t, s] exp(L_t - L_s) dt_s for s <= t, 0 above the diagonal.  Heads with a moderate
