@@ -16,8 +16,10 @@
 // probabilities of an attention kernel; scaled copies of x and dy exist only in shared memory; the epilogues add the
 // terms and take the row dot products.  What is left is bound by reading x / dy and writing y / dx once.
 //
-// Roles of every kernel here (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute (lane quarter
+// Roles (320 threads; the scan kernel's differ, see there): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute (lane quarter
 // warp % 4, column half (warp - 2) / 4).  Every wait is bounded.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace fmsb {
@@ -71,13 +73,15 @@ __device__ __forceinline__ uint32_t swz(int r, int c16) { return static_cast<uin
 
 // Per-head scalars of a chunk in shared memory, three sets (a set is rewritten only after every compute warp has passed
 // the barrier that follows its last use).  The decay of eight neighbouring columns is factorised around their first
-// one: exp(L_t - L_s) = exp(L_t - L_ref) exp(L_ref - L_s), one exponential per row and eight columns; `ok` says whether
-// the exponents are moderate enough for that, otherwise every element takes its own exponential.
+// one: exp(L_t - L_s) = exp(L_t - L_ref) exp(L_ref - L_s), one exponential per row and eight columns; `ok` (one flag per 32
+// positions) says whether the exponents are moderate enough for that, otherwise every element of the head takes its
+// own exponential.  One branch per head: a test per eight columns kept the loads of the next ones from being issued.
 struct HeadScalars {
   float L[CQ];
   float d[CQ];
-  float cf[CQ];  // rows t: exp(L_ref - L_s) dt_s; rows s (MODE 2): exp(L_t - L_ref)
-  int ok[CQ / 8];
+  float cf[CQ];        // rows t: exp(L_ref - L_s) dt_s; rows s (MODE 2): exp(L_t - L_ref)
+  float ref[CQ / 8];   // L of every eighth position
+  int ok[8];
 };
 
 template <int MODE>
@@ -87,63 +91,83 @@ __device__ __forceinline__ void publish(HeadScalars& hs, int i, float L, float d
   hs.L[i] = L;
   hs.d[i] = d;
   hs.cf[i] = MODE == 2 ? __expf(L - ref) : __expf(ref - L) * d;
-  if ((lane & 7) == 0) hs.ok[i >> 3] = fabsf(ref - last) < kSplitLimit ? 1 : 0;
+  if ((lane & 7) == 0) hs.ref[i >> 3] = L;
+  const int ok = __all_sync(0xffffffffu, fabsf(ref - last) < kSplitLimit);
+  if (lane == 0) hs.ok[i >> 5] = ok;
+}
+__device__ __forceinline__ bool all_ok(const HeadScalars& hs) {
+  const int4 a = *reinterpret_cast<const int4*>(&hs.ok[0]), b = *reinterpret_cast<const int4*>(&hs.ok[4]);
+  return (a.x & a.y & a.z & a.w & b.x & b.y & b.z & b.w) != 0;
 }
 
 // ----------------------------------------------------------------------------------------
-// Scan kernel.  grid (nc * 2, G * splits): one 128-row tile of a chunk, hp heads in turn.
+// Scan kernel.  grid (nc, G * splits): one chunk, hp heads in turn, each head's two 128-row tiles as two units.
 //   MODE 0: rows t; R = C, columns B; V = x, H = Hprev; out = y
 //   MODE 1: the same products, out = dy . (G x + exp(L) C Hprev^T) per row (E = dy)
 //   MODE 2: rows s; R = B, columns C; V = dy, H = dS; out = dx and three row dot products (E = x)
-// Tensor memory: two G buffers of 128 columns (256 contraction indices as 16-bit pairs), two accumulators of 64 + 64.
-// While the tensor core works on head i, the compute warps build G of head i + 1, then drain head i.
+// Both tiles in one CTA read V and H once (one tile per CTA read them 1.5 and 2 times) and are each other's second
+// buffer: while the tensor core works on unit w, the compute warps build G of unit w + 1, then drain unit w.
+// Tensor memory: G of the two tiles 64 + 128 columns (16-bit pairs), accumulators 2 x (64 + 64) from column 256.
+// 384 threads: warps 0 and 1 as above, 2 and 3 idle, 4-11 compute with 232 registers (C B^T is 96 of them).
+// 16384 tokens, 80 heads (one tile per CTA, 168 registers -> this): y 331 -> 144 us, dots 332 -> 141, dx 413 -> 183 us;
+// reading and writing everything once would take 63 us at the copy rate.
 // ----------------------------------------------------------------------------------------
-constexpr int kScanStage = 2 * kTile + kTile + kTile;  // V (256 rows), H (64 x 128), E
-constexpr int kScanSmem = 2 * kTile + 2 * kScanStage + 2 * kTile + 3 * (int)sizeof(HeadScalars) + 2 * 3 * 2 * 128 * 4 + 1024 + 256;
+constexpr int kScanThreads = 384;
+constexpr int kScanRegsMain = 40, kScanRegsCompute = 232;  // 128 * 40 + 256 * 232 = 384 * 168
+constexpr int kScanStage = 3 * kTile;  // V (256 rows), H (64 x 128)
+constexpr int kScanSmem = 4 * kTile + 2 * kScanStage + 3 * kTile + 3 * (int)sizeof(HeadScalars) + 3 * 3 * 128 * 4 + 1024 + 256;
+
+__device__ __forceinline__ void pair_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(quarter + 2) : "memory"); }
 
 template <int MODE, int FMT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kScanThreads, 1)
 ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmCol,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmH,
                 const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmOut, const ScanParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sR = base;
-  auto sV = [&](int s) { return base + 2 * kTile + s * kScanStage; };
+  auto sR = [&](int t) { return base + t * 2 * kTile; };  // [tile][64-column half]
+  auto sV = [&](int s) { return base + 4 * kTile + s * kScanStage; };
   auto sH = [&](int s) { return sV(s) + 2 * kTile; };
-  auto sE = [&](int s) { return sV(s) + 3 * kTile; };
-  const uint32_t sCol = sV(0);  // prologue only: 2 x [128 x 128] = stage 0
-  const uint32_t sOut = base + 2 * kTile + 2 * kScanStage;
-  const uint32_t scal = sOut + 2 * kTile;
+  const uint32_t sCol = sV(0);  // prologue only: [tile][half], 64 KB of the 96 KB of the stages
+  auto sE = [&](int e) { return base + 4 * kTile + 2 * kScanStage + e * kTile; };  // rows in (E) and out, ring of 3
+  const uint32_t scal = sE(3);
   const uint32_t dots = scal + 3 * (uint32_t)sizeof(HeadScalars);
-  const uint32_t bars = dots + 2 * 3 * 2 * 128 * 4;
+  const uint32_t bars = dots + 3 * 3 * 128 * 4;
   const uint32_t bar_r = bars, bar_cb = bars + 8u;
   auto full = [&](int s) { return bars + 16u + 8u * s; };
   auto empty = [&](int s) { return bars + 32u + 8u * s; };
-  auto g_full = [&](int b) { return bars + 48u + 8u * b; };
-  auto acc_full = [&](int b) { return bars + 64u + 8u * b; };
-  const uint32_t holder = bars + 80u;
+  auto g_full = [&](int u) { return bars + 48u + 8u * u; };
+  auto acc_full = [&](int u) { return bars + 64u + 8u * u; };
+  auto e_full = [&](int e) { return bars + 80u + 8u * e; };
+  auto e_empty = [&](int e) { return bars + 104u + 8u * e; };
+  const uint32_t holder = bars + 128u;
   HeadScalars* hs = reinterpret_cast<HeadScalars*>(smem_raw + (scal - smem_u32(smem_raw)));
-  float* sdot = reinterpret_cast<float*>(smem_raw + (dots - smem_u32(smem_raw)));  // [2][3][2][128]
+  float* sdot = reinterpret_cast<float*>(smem_raw + (dots - smem_u32(smem_raw)));  // [3][3][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x >> 1, tile = blockIdx.x & 1;
+  const int c = blockIdx.x;
   const int hpg = p.nh / p.G, spg = gridDim.y / p.G;
   const int g = blockIdx.y / spg;
   const int h_begin = g * hpg + (blockIdx.y % spg) * p.hp;
   const int n_heads = min(p.hp, (g + 1) * hpg - h_begin);
-  const int kt0 = MODE == 2 ? tile : 0;               // first 128-wide contraction tile
-  const int nks = MODE == 2 ? 2 - tile : tile + 1;    // number of them
-  const int own = MODE == 2 ? 0 : tile;               // which of V's tiles holds this CTA's own rows
+  // contraction tiles of row tile u: kt0(u) .. kt0(u) + nks(u) - 1; the first 128-column block of C B^T it owns
+  auto kt0 = [](int u) { return MODE == 2 ? u : 0; };
+  auto nks = [](int u) { return MODE == 2 ? 2 - u : u + 1; };
+  auto cb0 = [](int u) { return u == 0 ? 0 : (MODE == 2 ? 2 : 1); };
 
   if (warp == 1 && lane == 0) {
     mbar_init(bar_r, 1);
     mbar_init(bar_cb, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(full(s), 1);
-      mbar_init(empty(s), 8);
+      mbar_init(empty(s), MODE == 1 ? 1 : 8);
       mbar_init(g_full(s), 8);
       mbar_init(acc_full(s), 1);
+    }
+    for (int e = 0; e < 3; ++e) {
+      mbar_init(e_full(e), 1);
+      mbar_init(e_empty(e), 4);
     }
     fence_barrier_init();
   }
@@ -156,110 +180,133 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
   tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
-  auto tG = [&](int b) { return tmem + 128u * b; };
-  auto tAcc = [&](int b) { return tmem + 256u + 128u * b; };  // [G V: 64 | R H^T: 64]
+  auto tG = [&](int u) { return tmem + 64u * cb0(u); };
+  auto tAcc = [&](int u) { return tmem + 256u + 128u * u; };  // [G V: 64 | R H^T: 64]
 
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(bar_r, 2 * kTile * (1 + nks));
-      for (int k = 0; k < 2; ++k) {
-        tma_load_2d(sR + k * kTile, &tmR, bar_r, g * CN + 64 * k, c * CQ + tile * 128);
-        for (int i = 0; i < nks; ++i)
-          tma_load_2d(sCol + (2 * i + k) * kTile, &tmCol, bar_r, g * CN + 64 * k, c * CQ + (kt0 + i) * 128);
-      }
-      bool ok = mbar_wait(bar_cb, 0, p.status, kTimeoutProducer);  // stage 0 is free once C B^T is done
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kScanRegsMain));
+    if (warp == 0 && lane == 0) {
+      mbar_expect_tx(bar_r, 8 * kTile);
+      for (int t = 0; t < 2; ++t)
+        for (int k = 0; k < 2; ++k) {
+          tma_load_2d(sR(t) + k * kTile, &tmR, bar_r, g * CN + 64 * k, c * CQ + t * 128);
+          tma_load_2d(sCol + (2 * t + k) * kTile, &tmCol, bar_r, g * CN + 64 * k, c * CQ + t * 128);
+        }
+      auto load_e = [&](int w) {  // this CTA's own rows of unit w
+        const int e = w % 3;
+        if (!mbar_wait(e_empty(e), ((w / 3) & 1) ^ 1u, p.status, kTimeoutProducer)) return false;
+        mbar_expect_tx(e_full(e), kTile);
+        tma_load_2d(sE(e), &tmE, e_full(e), (h_begin + (w >> 1)) * CP, c * CQ + (w & 1) * 128);
+        return true;
+      };
+      bool ok = true;
+      if (MODE != 0) ok = load_e(0) && load_e(1);
+      ok = ok && mbar_wait(bar_cb, 0, p.status, kTimeoutProducer);  // the stages are free once C B^T is done
+#pragma unroll 1
       for (int it = 0; it < n_heads && ok; ++it) {
         const int s = it & 1, h = h_begin + it;
         if (!mbar_wait(empty(s), ((it >> 1) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
-        mbar_expect_tx(full(s), kTile * (nks + 1 + (MODE != 0 ? 1 : 0)));
-        for (int i = 0; i < nks; ++i) tma_load_2d(sV(s) + i * kTile, &tmV, full(s), h * CP, c * CQ + (kt0 + i) * 128);
+        mbar_expect_tx(full(s), 3 * kTile);
+        for (int i = 0; i < 2; ++i) tma_load_2d(sV(s) + i * kTile, &tmV, full(s), h * CP, c * CQ + i * 128);
         for (int k = 0; k < 2; ++k)
           tma_load_2d(sH(s) + k * (kTile / 2), &tmH, full(s), 64 * k, (c * p.nh + h) * CP);
-        if (MODE != 0) tma_load_2d(sE(s), &tmE, full(s), h * CP, c * CQ + tile * 128);
+        if (MODE != 0 && it > 0) ok = load_e(2 * it) && load_e(2 * it + 1);
       }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    } else if (warp == 1 && lane == 0) {
       bool ok = mbar_wait(bar_r, 0, p.status, kTimeoutMma);
       if (ok) {
         tc_fence_after();
         const uint32_t idesc = make_idesc_f16(128, 128, FMT, 0, 0);
-        const SmemDescBase a = make_smem_desc_base(sR, 16, 1024);
-        for (int i = 0; i < nks; ++i) {
-          const SmemDescBase b = make_smem_desc_base(sCol + 2 * i * kTile, 16, 1024);
-#pragma unroll
-          for (int ks = 0; ks < CN / 16; ++ks) {
-            const uint32_t off = (ks / 4) * kTile + (ks % 4) * 32;
-            tc_mma_f16(tmem + 128u * i, smem_desc_at(a, off), smem_desc_at(b, off), idesc, ks != 0);
+#pragma unroll 1
+        for (int u = 0; u < 2; ++u)
+#pragma unroll 1
+          for (int i = 0; i < nks(u); ++i) {
+            const SmemDescBase a = make_smem_desc_base(sR(u), 16, 1024);
+            const SmemDescBase b = make_smem_desc_base(sCol + 2 * (kt0(u) + i) * kTile, 16, 1024);
+#pragma unroll 1
+            for (int ks = 0; ks < CN / 16; ++ks) {
+              const uint32_t off = (ks / 4) * kTile + (ks % 4) * 32;
+              tc_mma_f16(tmem + 128u * (cb0(u) + i), smem_desc_at(a, off), smem_desc_at(b, off), idesc, ks != 0);
+            }
           }
-        }
         tc_commit(bar_cb);
       }
       const uint32_t idesc_v = make_idesc_f16(128, CP, FMT, 0, 1), idesc_h = make_idesc_f16(128, CP, FMT, 0, 0);
-      const SmemDescBase r = make_smem_desc_base(sR, 16, 1024);
+      // None of these loops is unrolled: unrolled, the compiler kept the descriptors of all 40 products of a head across
+      // the loop, more than the registers of this warp hold, and every issue waited for a reload from L2 (shared memory
+      // leaves L1 nothing): 296 us instead of 174 us for y at 16384 tokens, 80 heads.
+#pragma unroll 1
       for (int it = 0; it < n_heads && ok; ++it) {
         const int s = it & 1;
         if (!mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutMma)) break;
-        if (!mbar_wait(g_full(s), (it >> 1) & 1, p.status, kTimeoutMma)) break;
-        tc_fence_after();
         const SmemDescBase v = make_smem_desc_base(sV(s), 8192, 1024), hd = make_smem_desc_base(sH(s), 16, 1024);
-        for (int ks = 0; ks < nks * 8; ++ks)
-          tc_mma_f16_ts(tAcc(s), tG(s) + ks * 8, smem_desc_at(v, ks * 2048), idesc_v, ks != 0);
-#pragma unroll
-        for (int ks = 0; ks < CN / 16; ++ks)
-          tc_mma_f16(tAcc(s) + 64u, smem_desc_at(r, (ks / 4) * kTile + (ks % 4) * 32),
-                     smem_desc_at(hd, (ks / 4) * (kTile / 2) + (ks % 4) * 32), idesc_h, ks != 0);
-        tc_commit(acc_full(s));
+#pragma unroll 1
+        for (int u = 0; u < 2; ++u) {
+          if (!mbar_wait(g_full(u), it & 1, p.status, kTimeoutMma)) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int ks = 0; ks < nks(u) * 8; ++ks)
+            tc_mma_f16_ts(tAcc(u), tG(u) + ks * 8, smem_desc_at(v, kt0(u) * kTile + ks * 2048), idesc_v, ks != 0);
+          const SmemDescBase r = make_smem_desc_base(sR(u), 16, 1024);
+#pragma unroll 1
+          for (int ks = 0; ks < CN / 16; ++ks)
+            tc_mma_f16(tAcc(u) + 64u, smem_desc_at(r, (ks / 4) * kTile + (ks % 4) * 32),
+                       smem_desc_at(hd, (ks / 4) * (kTile / 2) + (ks % 4) * 32), idesc_h, ks != 0);
+          tc_commit(acc_full(u));
+        }
+        if (MODE == 1 && ok) tc_commit(empty(s));  // nothing but the tensor core reads V and H
       }
     }
   } else {
-    const int quarter = warp & 3, chalf = (warp - 2) >> 2;
-    const int ctid = threadIdx.x - 64;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kScanRegsCompute));
+    const int quarter = warp & 3, chalf = (warp - 4) >> 2;
+    const int ctid = threadIdx.x - 128;
     const int row = quarter * 32 + lane;
-    const int pos = tile * 128 + row;              // position in the chunk
-    const int rbase = tile * 128 + quarter * 32;   // first position of this warp's rows
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const float* Lg = p.Lt + ((long long)c * p.nh + h_begin) * CQ + ctid;
     const float* dg = p.dtt + ((long long)c * p.nh + h_begin) * CQ + ctid;
     float nL = Lg[0], nd = dg[0];
-    // C B^T of this row, blocks of 32 columns taken in turn by the two column halves (their causal work is then equal)
-    uint32_t cb[4][16];
+    // C B^T of this thread's two rows (one per tile) as 16-bit pairs; blocks of 32 columns are taken in turn by the two
+    // column halves, so that their causal work is equal.  cb[b]: blocks of tile 0, then of tile 1.
+    uint32_t cb[6][16];
     bool ok = mbar_wait(bar_cb, 0, p.status, kTimeoutEpilogue);
     if (ok) {
       tc_fence_after();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i < 2 * nks) {
-          uint32_t r[32];
-          tmem_ld_32x32(tmem + lane_addr + (2 * i + chalf) * 32, r);
-          tmem_ld_wait();
+      for (int i = 0; i < 6; ++i) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem + lane_addr + (2 * i + chalf) * 32, r);
+        tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) cb[i][j] = pack2f<FMT>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-        }
+        for (int j = 0; j < 16; ++j) cb[i][j] = pack2f<FMT>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
       }
       tc_fence_before();
     }
-    auto build = [&](int it) {
-      const HeadScalars& q = hs[it % 3];
+    auto build_as = [&](int u, const HeadScalars& q, auto split) {
+      const int pos = u * 128 + row, rbase = u * 128 + quarter * 32;
       const float Lrow = q.L[pos], drow = MODE == 2 ? q.d[pos] : 1.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i >= 2 * nks) break;
-        const int b = 2 * i + chalf, col0 = kt0 * 128 + b * 32;
+      for (int i = 0; i < 2 * nks(u); ++i) {
+        const int b = 2 * i + chalf, col0 = kt0(u) * 128 + b * 32;
         uint32_t pk[16];
         if (MODE == 2 ? col0 < rbase : col0 > rbase) {  // wholly above the diagonal
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = 0u;
         } else {
+          const float4 r4 = *reinterpret_cast<const float4*>(&q.ref[col0 >> 3]);
+          const float refs[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
           for (int gq = 0; gq < 4; ++gq) {
             const int cg = col0 + gq * 8;
             float f[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) unpack2<FMT>(cb[i][gq * 4 + j], f[2 * j], f[2 * j + 1]);
-            if (q.ok[cg >> 3]) {
-              const float Lref = q.L[cg];
-              const float e = MODE == 2 ? __expf(Lref - Lrow) * drow : __expf(Lrow - Lref);
+            for (int j = 0; j < 4; ++j) {
+              uint32_t w = cb[2 * cb0(u) + i][gq * 4 + j];
+              asm volatile("" : "+r"(w));  // unpack here, not ahead of the loop over the heads: 192 floats spill (174 -> 144 us)
+              unpack2<FMT>(w, f[2 * j], f[2 * j + 1]);
+            }
+            if constexpr (decltype(split)::value) {
+              const float e = MODE == 2 ? __expf(refs[gq] - Lrow) * drow : __expf(Lrow - refs[gq]);
               const uint64_t e2 = pack_f32x2(e, e);
               const float4 c0 = *reinterpret_cast<const float4*>(&q.cf[cg]), c1 = *reinterpret_cast<const float4*>(&q.cf[cg + 4]);
               unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[0], f[1]), e2), pack_f32x2(c0.x, c0.y)), f[0], f[1]);
@@ -267,6 +314,7 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
               unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[4], f[5]), e2), pack_f32x2(c1.x, c1.y)), f[4], f[5]);
               unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(f[6], f[7]), e2), pack_f32x2(c1.z, c1.w)), f[6], f[7]);
             } else {
+              asm volatile("" ::: "memory");  // no loads of later columns ahead of these: registers
 #pragma unroll
               for (int j = 0; j < 8; ++j)
                 f[j] *= MODE == 2 ? __expf(q.L[cg + j] - Lrow) * drow : __expf(Lrow - q.L[cg + j]) * q.d[cg + j];
@@ -280,68 +328,57 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
             for (int j = 0; j < 4; ++j) pk[gq * 4 + j] = pack2f<FMT>(f[2 * j], f[2 * j + 1]);
           }
         }
-        tmem_st_32x16(tG(it & 1) + lane_addr + b * 16, pk);
+        tmem_st_32x16(tG(u) + lane_addr + b * 16, pk);
       }
+    };
+    auto build = [&](int u, int it) {
+      const HeadScalars& q = hs[it % 3];
+      if (all_ok(q)) build_as(u, q, std::true_type{});
+      else build_as(u, q, std::false_type{});
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(g_full(it & 1));
+      if (lane == 0) mbar_arrive(g_full(u));
     };
-    publish<MODE>(hs[0], ctid, nL, nd);
-    if (n_heads > 1) {
-      nL = Lg[CQ];
-      nd = dg[CQ];
-    }
-    compute_sync(1);  // scalars of the first head are there, and C B^T has been read everywhere: G may overwrite it
-    tc_fence_after();
-    if (ok) build(0);
-    for (int it = 0; it < n_heads; ++it) {
-      const int s = it & 1, h = h_begin + it;
-      const bool more = it + 1 < n_heads;
-      if (more) {
-        publish<MODE>(hs[(it + 1) % 3], ctid, nL, nd);
-        if (it + 2 < n_heads) {
-          nL = Lg[(it + 2) * CQ];
-          nd = dg[(it + 2) * CQ];
-        }
-      }
-      compute_sync(1);  // also orders the reuse of sOut and sdot
-      if (more && ok) build(it + 1);
-      if (ok) ok = mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
-      if (ok) ok = mbar_wait(acc_full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+    auto drain = [&](int u, int it) {
+      const int s = it & 1, h = h_begin + it, w = 2 * it + u, e = w % 3;
+      if (ok && u == 0 && MODE != 1) ok = mbar_wait(full(s), (it >> 1) & 1, p.status, kTimeoutEpilogue);
+      if (ok && MODE != 0) ok = mbar_wait(e_full(e), (w / 3) & 1, p.status, kTimeoutEpilogue);
+      if (ok) ok = mbar_wait(acc_full(u), it & 1, p.status, kTimeoutEpilogue);
       const HeadScalars& q = hs[it % 3];
+      float d0 = 0.f, d1 = 0.f, d2 = 0.f;
       if (ok) {
         tc_fence_after();
+        const int pos = u * 128 + row;
         const float Lrow = q.L[pos];
         // weight of the second product: exp(L_t) for rows t, w_s for rows s
-        const float e = MODE == 2 ? __expf(q.L[CQ - 1] - Lrow) * q.d[pos] : __expf(Lrow);
+        const float ew = MODE == 2 ? __expf(q.L[CQ - 1] - Lrow) * q.d[pos] : __expf(Lrow);
         const float dh = MODE == 1 ? 0.f : p.D[h];
-        float d0 = 0.f, d1 = 0.f, d2 = 0.f;
         uint32_t ra[16], ri[16];
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
-          if ((ch & 1) == 0) {  // 16 columns of each product at a time: C B^T keeps 64 registers busy
-            tmem_ld_32x16(tAcc(s) + lane_addr + chalf * 32 + ch * 8, ra);
-            tmem_ld_32x16(tAcc(s) + lane_addr + 64 + chalf * 32 + ch * 8, ri);
+          if ((ch & 1) == 0) {
+            tmem_ld_32x16(tAcc(u) + lane_addr + chalf * 32 + ch * 8, ra);
+            tmem_ld_32x16(tAcc(u) + lane_addr + 64 + chalf * 32 + ch * 8, ri);
             tmem_ld_wait();
           }
           const uint32_t off = swz(row, chalf * 4 + ch);
-          const uint4 u = lds128(sV(s) + own * kTile + off);
-          const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
-          uint4 e4 = make_uint4(0u, 0u, 0u, 0u);
-          if (MODE != 0) e4 = lds128(sE(s) + off);
-          const uint32_t ew[4] = {e4.x, e4.y, e4.z, e4.w};
+          uint4 v4 = make_uint4(0u, 0u, 0u, 0u), e4 = v4;
+          if (MODE != 1) v4 = lds128(sV(s) + u * kTile + off);
+          if (MODE != 0) e4 = lds128(sE(e) + off);
+          const uint32_t vw[4] = {v4.x, v4.y, v4.z, v4.w}, xw[4] = {e4.x, e4.y, e4.z, e4.w};
           uint32_t ow[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            float v0, v1, x0 = 0.f, x1 = 0.f;
-            unpack2<FMT>(uw[j], v0, v1);
-            if (MODE != 0) unpack2<FMT>(ew[j], x0, x1);
+            float v0 = 0.f, v1 = 0.f, x0 = 0.f, x1 = 0.f;
+            if (MODE != 1) unpack2<FMT>(vw[j], v0, v1);
+            if (MODE != 0) unpack2<FMT>(xw[j], x0, x1);
             const int k = (ch & 1) * 8 + j * 2;
             const float a0 = __uint_as_float(ra[k]), a1 = __uint_as_float(ra[k + 1]);
-            const float i0 = e * __uint_as_float(ri[k]), i1 = e * __uint_as_float(ri[k + 1]);
+            const float i0 = ew * __uint_as_float(ri[k]), i1 = ew * __uint_as_float(ri[k + 1]);
             if (MODE == 1) {
-              d0 += x0 * (a0 + i0) + x1 * (a1 + i1);
+              d0 += x0 * (a0 + i0);
+              d1 += x1 * (a1 + i1);
             } else {
               ow[j] = pack2f<FMT>(a0 + i0 + dh * v0, a1 + i1 + dh * v1);
               if (MODE == 2) {
@@ -351,38 +388,71 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
               }
             }
           }
-          if (MODE != 1) sts128(sOut + (it & 1) * kTile + off, ow[0], ow[1], ow[2], ow[3]);
+          if (MODE != 1) sts128(sE(e) + off, ow[0], ow[1], ow[2], ow[3]);
         }
-        if (MODE != 0) {
-          float* sd = sdot + (it & 1) * 768 + chalf * 128 + row;
+        if (MODE == 1) d0 += d1;
+        if (MODE != 0 && chalf == 1) {
+          float* sd = sdot + (w % 3) * 384 + row;
           sd[0] = d0;
           if (MODE == 2) {
-            sd[256] = d1;
-            sd[512] = d2;
+            sd[128] = d1;
+            sd[256] = d2;
           }
         }
         if (MODE != 1) fence_proxy_async_smem();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(empty(s));
+        if (u == 1 && MODE != 1 && lane == 0) mbar_arrive(empty(s));
       }
-      compute_sync(2);
-      if (ok && MODE != 1 && ctid == 0) {
-        tma_store_2d(&tmOut, sOut + (it & 1) * kTile, h * CP, c * CQ + tile * 128);
-        tma_store_commit();
-        tma_store_wait_read<1>();
-      }
-      if (ok && MODE != 0) {
-        const long long o = ((long long)c * p.nh + h) * CQ + tile * 128;
-        const float* sd = sdot + (it & 1) * 768;
-        const long long plane = (long long)p.nc * p.nh * CQ;
-        for (int i = ctid; i < (MODE == 2 ? 384 : 128); i += 256) {
-          const int k = i >> 7, r = i & 127;
-          p.red[k * plane + o + r] = sd[k * 256 + r] + sd[k * 256 + 128 + r];
+      // the two warps of these 32 rows meet; the first one's lane 0 stores the rows and returns the buffer
+      pair_sync(quarter);
+      if (ok && chalf == 0) {
+        if (MODE != 0) {
+          const long long o = ((long long)c * p.nh + h) * CQ + u * 128 + row;
+          const float* sd = sdot + (w % 3) * 384 + row;
+          p.red[o] = d0 + sd[0];
+          if (MODE == 2) {
+            const long long plane = (long long)p.nc * p.nh * CQ;
+            p.red[plane + o] = d1 + sd[128];
+            p.red[2 * plane + o] = d2 + sd[256];
+          }
+        }
+        if (lane == 0) {
+          if (MODE == 1) {
+            mbar_arrive(e_empty(e));
+          } else {
+            tma_store_2d(&tmOut, sE(e) + quarter * 4096, h * CP, c * CQ + u * 128 + quarter * 32);
+            tma_store_commit();
+            tma_store_wait_read<1>();  // the store of the unit before has read its buffer
+            if (MODE == 2 && w > 0) mbar_arrive(e_empty((w - 1) % 3));
+          }
         }
       }
+    };
+    publish<MODE>(hs[0], ctid, nL, nd);
+    if (n_heads > 1) {
+      nL = Lg[CQ];
+      nd = dg[CQ];
     }
-    if (MODE != 1 && ctid == 0) tma_store_wait<0>();
+    compute_sync(1);  // scalars of the first head are there, and C B^T has been read everywhere: G may overwrite it
+    tc_fence_after();
+    if (ok) build(0, 0);
+    for (int it = 0; it < n_heads; ++it) {
+      const bool more = it + 1 < n_heads;
+      if (more) {
+        publish<MODE>(hs[(it + 1) % 3], ctid, nL, nd);
+        if (it + 2 < n_heads) {
+          nL = Lg[(it + 2) * CQ];
+          nd = dg[(it + 2) * CQ];
+        }
+      }
+      if (ok) build(1, it);
+      drain(0, it);
+      compute_sync(1);
+      if (more && ok) build(0, it + 1);
+      drain(1, it);
+    }
+    if (MODE != 1 && chalf == 0 && lane == 0) tma_store_wait<0>();
   }
   __syncwarp();
   tc_fence_before();
@@ -680,6 +750,7 @@ ssd_dcb_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__
       if (!ok) continue;
       tc_fence_after();
       const float Lrow = q.L[pos];
+      const bool split = all_ok(q);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         uint32_t r[32];
@@ -694,8 +765,8 @@ ssd_dcb_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__
         for (int gq = 0; gq < 4; ++gq) {
           const int cg = col0 + k * 32 + gq * 8;
           uint64_t* ac = acc + k * 16 + gq * 4;
-          if (q.ok[cg >> 3]) {
-            const float e = __expf(Lrow - q.L[cg]);
+          if (split) {
+            const float e = __expf(Lrow - q.ref[cg >> 3]);
             const uint64_t e2 = pack_f32x2(e, e);
             const float4 c0 = *reinterpret_cast<const float4*>(&q.cf[cg]), c1 = *reinterpret_cast<const float4*>(&q.cf[cg + 4]);
             const uint64_t cf[4] = {pack_f32x2(c0.x, c0.y), pack_f32x2(c0.z, c0.w), pack_f32x2(c1.x, c1.y), pack_f32x2(c1.z, c1.w)};
@@ -907,10 +978,10 @@ static int pick_heads(long long tiles, int hpg) {
   return hp;
 }
 
-// kind 0: scan tiles (2 per chunk and group), 1: state kernel (1), 2: dCB (3).  Returns heads per CTA.
+// kind 0: scan and 1: state kernel (one CTA per chunk, group and split), 2: dCB (three).  Returns heads per CTA.
 extern "C" int fmsb_ssdf_heads(int kind, int nc, int nh, int G) {
   if (nc <= 0 || G <= 0 || nh % G) return 1;
-  return pick_heads((long long)nc * G * (kind == 0 ? 2 : kind == 1 ? 1 : 3), nh / G);
+  return pick_heads((long long)nc * G * (kind == 2 ? 3 : 1), nh / G);
 }
 
 static int map_rows(CUtensorMap* m, const void* p, long long rows, long long cols, long long ld, int box_rows) {
@@ -920,6 +991,16 @@ static int map_rows(CUtensorMap* m, const void* p, long long rows, long long col
 template <typename K>
 static int set_smem(K kern, int bytes) {
   return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+// The register split of the scan kernel draws on what the block was launched with: a build that gave the kernel fewer
+// registers per thread would wait for them without end, so it is refused here.
+template <typename K>
+static int scan_regs(K kern) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return (int)e;
+  return a.numRegs * kScanThreads >= 128 * kScanRegsMain + 256 * kScanRegsCompute ? 0 : -3;
 }
 
 // mode 0: out = y (v = x, r = C, col = B, hst = entering states); mode 1: red = dy . y-terms (e = dy);
@@ -940,19 +1021,20 @@ extern "C" int fmsb_ssdf_scan(int mode, const void* r, long long ldr, const void
   te = tv;
   to = tv;
   if (mode != 0 && (rc = map_rows(&te, e, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
-  if (mode != 1 && (rc = map_rows(&to, out, T, (long long)nh * CP, (long long)nh * CP, 128))) return rc;
+  if (mode != 1 && (rc = map_rows(&to, out, T, (long long)nh * CP, (long long)nh * CP, 32))) return rc;
   ScanParams p{};
   p.nc = nc; p.nh = nh; p.G = G; p.hp = hp; p.Lt = Lt; p.dtt = dtt; p.D = D; p.red = red; p.T = (int)T; p.status = status;
   const int hpg = nh / G;
-  const dim3 grid(nc * 2, G * ((hpg + hp - 1) / hp));
+  const dim3 grid(nc, G * ((hpg + hp - 1) / hp));
 #define FMSB_SCAN(MM, FF)                                                                              \
   do {                                                                                                 \
     static bool cfg = false;                                                                           \
     if (!cfg) {                                                                                        \
       if ((rc = set_smem(ssd_scan_kernel<MM, FF>, kScanSmem))) return rc;                              \
+      if ((rc = scan_regs(ssd_scan_kernel<MM, FF>))) return rc;                                        \
       cfg = true;                                                                                      \
     }                                                                                                  \
-    ssd_scan_kernel<MM, FF><<<grid, 320, kScanSmem, stream>>>(tr, tc, tv, th, te, to, p);              \
+    ssd_scan_kernel<MM, FF><<<grid, kScanThreads, kScanSmem, stream>>>(tr, tc, tv, th, te, to, p);              \
   } while (0)
   if (fmt == 1) { if (mode == 0) FMSB_SCAN(0, 1); else if (mode == 1) FMSB_SCAN(1, 1); else FMSB_SCAN(2, 1); }
   else { if (mode == 0) FMSB_SCAN(0, 0); else if (mode == 1) FMSB_SCAN(1, 0); else FMSB_SCAN(2, 0); }
