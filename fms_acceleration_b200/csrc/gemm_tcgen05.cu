@@ -319,14 +319,29 @@ __device__ __forceinline__ void epilogue_store_tile_tma(const GemmParams& p, con
     for (int i = 0; i < CH; ++i) v[i] = (empty_k ? 0.f : __uint_as_float(r[i])) * p.alpha;
     const int gn = n0 + c * CH;
     if (p.C != nullptr && p.beta != 0.f && gm < p.M && gn < p.N) {
-      if (p.fmt == 1) {
-        const __nv_bfloat16* crow = reinterpret_cast<const __nv_bfloat16*>(p.C) + (long long)gm * p.ldc + gn;
+      const uint16_t* crow = reinterpret_cast<const uint16_t*>(p.C) + (long long)gm * p.ldc + gn;
+      if (gn + CH <= p.N && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
+        // four 16-byte loads, all in flight: lanes are rows, so 32 loads of two bytes touched 32 lines each
+        uint4 u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) u[j] = *reinterpret_cast<const uint4*>(crow + 8 * j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t w[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 f = p.fmt == 1 ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]))
+                                        : __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+            v[8 * j + 2 * k] += p.beta * f.x;
+            v[8 * j + 2 * k + 1] += p.beta * f.y;
+          }
+        }
+      } else if (p.fmt == 1) {
         for (int i = 0; i < CH; ++i)
-          if (gn + i < p.N) v[i] += p.beta * __bfloat162float(crow[i]);
+          if (gn + i < p.N) v[i] += p.beta * __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(crow)[i]);
       } else {
-        const __half* crow = reinterpret_cast<const __half*>(p.C) + (long long)gm * p.ldc + gn;
         for (int i = 0; i < CH; ++i)
-          if (gn + i < p.N) v[i] += p.beta * __half2float(crow[i]);
+          if (gn + i < p.N) v[i] += p.beta * __half2float(reinterpret_cast<const __half*>(crow)[i]);
       }
     }
     const uint32_t buf = slots + static_cast<uint32_t>(slot) * 2048u;
@@ -899,7 +914,7 @@ int launch_gemm_pair(const CUtensorMap& a1, const CUtensorMap& b1, const CUtenso
 static int g_pair_tma_store = 1;
 static int g_single_tma_store = 1;
 
-// 0: never, 1: when there are enough 256 x 256 tiles to fill the machine about twice (default), 2: whenever M and N
+// 0: never, 1: by the rule in gemm_impl (default), 2: whenever M and N
 // reach 256; set through fmsb_gemm_set_pair_mode (tests compare both kernels on small shapes)
 static int g_pair_mode = 1;
 
@@ -960,10 +975,17 @@ static int gemm_impl(const void* A1, long long lda1, const void* B1, long long l
   if (b_mn && bn < 64) return -3;
   CUtensorMap ta1, tb1, ta2, tb2, tbalt;
   int rc;
-  // CTA pairs: plain mode, 256-column tiles, enough 256 x 256 tiles to fill the machine about twice
-  const bool use_pair = mode == 0 && bn == 256 && g_pair_mode != 0 && M >= 256 && N >= 256 &&
-                        (g_pair_mode == 2 ||
-                         (long long)((M + 255) / 256) * ((N + 255) / 256) >= 2LL * (sm_count() / 2));
+  // CTA pairs: plain mode, 256-column tiles, and either enough 256 x 256 tiles to fill the machine about twice, or a
+  // grid that takes no more turns with pairs than with single CTAs (a ragged M can cost the pairs a turn: 1111 x 4096 x
+  // 4096 40 us single, 68 us pairs) and is long enough for the pair's longer start: two turns (2048 x 4096 x 14336:
+  // 207 -> 189 us; 5376 x 1536 x 49160: 724 -> 622 us) or a contraction of 8192 (256 x 4096 x 14336: 111 -> 100 us, while
+  // 4096 x 1024 x 4096 goes from 36 to 38 us).
+  bool use_pair = false;
+  if (mode == 0 && bn == 256 && g_pair_mode != 0 && M >= 256 && N >= 256) {
+    const long long t2 = (long long)((M + 255) / 256) * ((N + 255) / 256), t1 = (long long)((M + 127) / 128) * ((N + 255) / 256);
+    const long long turns1 = (t1 + sm_count() - 1) / sm_count(), turns2 = (t2 + sm_count() / 2 - 1) / (sm_count() / 2);
+    use_pair = g_pair_mode == 2 || t2 >= 2LL * (sm_count() / 2) || (turns2 <= turns1 && (turns2 >= 2 || K1 + K2 >= 8192));
+  }
   const int b_box_rows = use_pair ? fmsb::BNH : bn;
   // a_rows / b_rows: number of rows of the stored A / B matrices when it differs from the per-tile view
   // (grouped modes address several segments / expert matrices through one tensor map)
