@@ -98,6 +98,22 @@ __device__ __forceinline__ uint32_t q4_pack2(float a, float b, int fmt) {
   return fmt == 1 ? pack_bf16x2(a, b) : pack_f16x2(a, b);
 }
 
+// 32 accumulator columns of one row to D
+__device__ __forceinline__ void q4_store32(const Q4Params& p, int row, int col, const uint32_t (&v)[32]) {
+  uint16_t* dst = reinterpret_cast<uint16_t*>(p.D) + (long long)row * p.ldd + col;
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) {
+    if (col + i < p.N) {  // N % 8 == 0: a group of 8 columns is in range as a whole
+      uint4 u;
+      u.x = q4_pack2(__uint_as_float(v[i]) * p.alpha, __uint_as_float(v[i + 1]) * p.alpha, p.fmt);
+      u.y = q4_pack2(__uint_as_float(v[i + 2]) * p.alpha, __uint_as_float(v[i + 3]) * p.alpha, p.fmt);
+      u.z = q4_pack2(__uint_as_float(v[i + 4]) * p.alpha, __uint_as_float(v[i + 5]) * p.alpha, p.fmt);
+      u.w = q4_pack2(__uint_as_float(v[i + 6]) * p.alpha, __uint_as_float(v[i + 7]) * p.alpha, p.fmt);
+      *reinterpret_cast<uint4*>(dst + i) = u;
+    }
+  }
+}
+
 template <int BN, int GPTQ>
 __global__ void __launch_bounds__(64 + Q4_DQ_THREADS, 1)
 gemm_q4_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmXa,
@@ -285,20 +301,236 @@ gemm_q4_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         uint32_t v[32];
         tmem_ld_32x32(tmem + lane_addr + c * 32, v);
         tmem_ld_wait();
-        if (row < p.M) {
-          uint16_t* dst = reinterpret_cast<uint16_t*>(p.D) + (long long)row * p.ldd + n0 + c * 32;
+        if (row < p.M) q4_store32(p, row, n0 + c * 32, v);
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 128);
+  }
+}
+
+// ----------------------------------------------------------------------------------------
+// The same product for one local, double-quantised NF4 / FP4 weight without a LoRA pair (a plain 4-bit layer), laid out
+// for latency.  In the kernel above all eight dequant warps work on one K block at a time, so a block costs one warp's
+// whole chain (load, look-up, convert, store, fence, arrive: about 2000 cycles whatever the tile).  Here four groups of
+// four warps take K blocks in turn, a thread expands a longer piece of a row (64 values at 128 wide) and nothing is
+// outstanding when it fences: the packed bytes come in by TMA (a W stage is [BN rows x 128 bytes] = four K blocks,
+// 128-byte swizzle) and the 8-bit scale codes of the tile (BN * K / 64 bytes) are copied to shared memory once.
+// 77 x 14336 x 4096: 66.6 -> 37.7 us, 77 x 4096 x 4096 (32 wide): 30.8 -> 22.7 us; what is left at 128 wide is shared memory (look-ups,
+// operand writes and the tensor core's reads: about 850 of 1000 cycles per K block).
+// ----------------------------------------------------------------------------------------
+constexpr int Q4T_GROUPS = 4;           // dequant groups of four warps
+constexpr int Q4T_DQ_THREADS = Q4T_GROUPS * 128;
+
+template <int BN>
+struct Q4tCfg {
+  static constexpr int kABytes = Q4_BM * Q4_BK * 2;
+  static constexpr int kBBytes = 2 * BN * Q4_BK * 2;  // two K blocks
+  // separate rings: a group may expand its next K block while the tensor core still has to read its last one
+  static constexpr int kAStages = 4;
+  static constexpr int kBStages = BN == 128 ? 2 : 4;
+  static constexpr int kWBytes = BN * 128;
+  static constexpr int kWStages = BN == 128 ? 2 : 3;
+  static constexpr int kFixed = kAStages * kABytes + kBStages * kBBytes + kWStages * kWBytes + 1024 + 512;
+  static constexpr int kStatic = 256 * 16 * 8 + 2048;  // the pair table and the small ones
+  static constexpr int kScaleBytes = 227 * 1024 - kStatic - kFixed;  // room for the codes and the second-level scales
+};
+
+template <int BN, int FMT>
+__global__ void __launch_bounds__(96 + Q4T_DQ_THREADS, 1)
+gemm_q4_tma_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Q4Params p) {
+  using Cfg = Q4tCfg<BN>;
+  constexpr int AS = Cfg::kAStages, BS = Cfg::kBStages, WS = Cfg::kWStages;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  auto sA = [&](int s) { return base + s * Cfg::kABytes; };
+  auto sB = [&](int s) { return base + AS * Cfg::kABytes + s * Cfg::kBBytes; };
+  auto sW = [&](int s) { return base + AS * Cfg::kABytes + BS * Cfg::kBBytes + s * Cfg::kWBytes; };
+  const uint32_t bars = sW(WS);
+  auto bar_a_full = [&](int s) { return bars + 8u * s; };
+  auto bar_a_empty = [&](int s) { return bars + 8u * (AS + s); };
+  auto bar_b_full = [&](int s) { return bars + 8u * (2 * AS + s); };
+  auto bar_b_empty = [&](int s) { return bars + 8u * (2 * AS + BS + s); };
+  auto bar_w_full = [&](int s) { return bars + 8u * (2 * AS + 2 * BS + s); };
+  auto bar_w_empty = [&](int s) { return bars + 8u * (2 * AS + 2 * BS + WS + s); };
+  const uint32_t bar_acc = bars + 8u * (2 * AS + 2 * BS + 2 * WS);
+  const uint32_t holder = bar_acc + 8u;
+  uint8_t* codes = smem_raw + (bars - smem_u32(smem_raw)) + 512;  // [BN][K / 64]
+  // value pairs of a byte, sixteen copies side by side: lane l reads copy l % 16, so the 8-byte reads of a half warp
+  // never meet in a bank.  One look-up gives two values (two 4-byte look-ups cost six instructions more per byte).
+  __shared__ float2 s_pair[256 * 16];
+  __shared__ float s_code[16];
+  __shared__ float s_code256[256];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * BN;
+  const int m0 = blockIdx.y * Q4_BM;
+  const int kbt = p.kblocks1;
+  const int rows = min(BN, p.N - n0);
+  float* s_abs2 = reinterpret_cast<float*>(codes + ((BN * kbt + 15) & ~15));
+  const long long blk0 = (long long)n0 * kbt;  // first scale block of the tile
+  const long long grp0 = blk0 >> 8;
+
+  if (warp == 1 && lane == 0) {
+    for (int s = 0; s < AS; ++s) {
+      mbar_init(bar_a_full(s), 1);
+      mbar_init(bar_a_empty(s), 1);
+    }
+    for (int s = 0; s < BS; ++s) {
+      mbar_init(bar_b_full(s), 8);  // four warps for each of the two K blocks
+      mbar_init(bar_b_empty(s), 1);
+    }
+    for (int s = 0; s < WS; ++s) {
+      mbar_init(bar_w_full(s), 1);
+      mbar_init(bar_w_empty(s), Q4T_DQ_THREADS / 32);
+    }
+    mbar_init(bar_acc, 1);
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(holder, 128);
+    tmem_relinquish();
+  }
+  if (threadIdx.x < 16) s_code[threadIdx.x] = p.code16[threadIdx.x];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) s_code256[i] = p.code256[i];
+  {
+    const int nb = rows * kbt;
+    const uint8_t* src = p.absmax_q + blk0;
+    int i0 = 0;
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+      i0 = nb & ~15;
+      for (int i = threadIdx.x * 16; i < i0; i += blockDim.x * 16)
+        *reinterpret_cast<uint4*>(codes + i) = *reinterpret_cast<const uint4*>(src + i);
+    }
+    for (int i = i0 + threadIdx.x; i < nb; i += blockDim.x) codes[i] = src[i];
+    const int ng = (int)(((blk0 + nb - 1) >> 8) - grp0) + 1;
+    for (int i = threadIdx.x; i < ng; i += blockDim.x) s_abs2[i] = p.absmax2[grp0 + i];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4096; i += blockDim.x) s_pair[i] = make_float2(s_code[i >> 8], s_code[(i >> 4) & 15]);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = 0; kb < kbt; ++kb) {
+        const int s = kb % AS;
+        if (!mbar_wait(bar_a_empty(s), ((kb / AS) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(bar_a_full(s), Cfg::kABytes);
+        tma_load_2d(sA(s), &tmX, bar_a_full(s), kb * Q4_BK, m0);
+      }
+    }
+  } else if (warp == 2) {
+    // W has a producer of its own: behind the waits for free activation stages it was asked for too late
+    if (lane == 0) {
+      for (int wi = 0; 4 * wi < kbt; ++wi) {
+        const int s = wi % WS;
+        if (!mbar_wait(bar_w_empty(s), ((wi / WS) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(bar_w_full(s), Cfg::kWBytes);
+        tma_load_2d(sW(s), &tmW, bar_w_full(s), wi * 64, n0);  // 64 16-bit units = 128 bytes = 256 weights
+      }
+    }
+  } else if (warp == 1) {
+    // Two K blocks per hand-off: the issuing thread needs about 700 cycles for two waits, four short products and two
+    // commits, more than four products of 128 x BN x 16 take.
+    const bool leader = elect_one();
+    const uint32_t idesc = make_idesc_f16(128, BN, FMT, 0, 0);
+    bool ok = true;
+    for (int st = 0; 2 * st < kbt && ok; ++st) {
+      const int sb = st % BS;
+      if (!mbar_wait(bar_b_full(sb), (st / BS) & 1, p.status, kTimeoutMma)) { ok = false; break; }
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            if (n0 + c * 32 + i < p.N) {  // N % 8 == 0: a group of 8 columns is in range as a whole
-              uint4 u;
-              u.x = q4_pack2(__uint_as_float(v[i]) * p.alpha, __uint_as_float(v[i + 1]) * p.alpha, p.fmt);
-              u.y = q4_pack2(__uint_as_float(v[i + 2]) * p.alpha, __uint_as_float(v[i + 3]) * p.alpha, p.fmt);
-              u.z = q4_pack2(__uint_as_float(v[i + 4]) * p.alpha, __uint_as_float(v[i + 5]) * p.alpha, p.fmt);
-              u.w = q4_pack2(__uint_as_float(v[i + 6]) * p.alpha, __uint_as_float(v[i + 7]) * p.alpha, p.fmt);
-              *reinterpret_cast<uint4*>(dst + i) = u;
-            }
-          }
+      for (int j = 0; j < 2; ++j) {
+        const int kb = 2 * st + j;
+        if (kb >= kbt) break;
+        const int sa = kb % AS;
+        if (!mbar_wait(bar_a_full(sa), (kb / AS) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+        tc_fence_after();
+        const SmemDescBase da = make_smem_desc_base(sA(sa), 16, 1024);
+        const SmemDescBase db = make_smem_desc_base(sB(sb) + j * (BN * 128), 16, 1024);
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < Q4_BK / 16; ++ks)
+            tc_mma_f16(tmem, smem_desc_at(da, ks * 32), smem_desc_at(db, ks * 32), idesc, (kb | ks) != 0);
+          tc_commit(bar_a_empty(sa));
         }
+      }
+      if (ok && leader) tc_commit(bar_b_empty(sb));
+    }
+    if (ok && leader) tc_commit(bar_acc);
+  } else {
+    // ------------------------------------------------------------------ dequantise W tiles [BN rows x 64]
+    constexpr int TPR = 128 / BN;   // threads per weight row
+    constexpr int CPT = 8 / TPR;    // 16-byte output chunks (= 4-byte packed words) per thread and K block
+    const int tid = threadIdx.x - 96;
+    const int group = tid >> 7;
+    const int r = (tid & 127) / TPR, part = (tid & 127) % TPR;
+    const uint32_t copy = (lane & 15) * 8;
+    const bool row_ok = r < rows;
+    const long long rb0 = blk0 + (long long)r * kbt;
+    bool ok = true;
+    const int kb_end = (kbt + 1) & ~1;  // an odd last block: its partner only arrives
+    for (int kb = group; kb < kb_end; kb += Q4T_GROUPS) {  // group g of a W stage takes its K block g
+      const int wi = kb >> 2, ws = wi % WS;
+      if (!mbar_wait(bar_w_full(ws), (wi / WS) & 1, p.status, kTimeoutDequant)) { ok = false; break; }
+      // packed bytes of this thread: 4 * CPT of the row's 32 for this K block, in the swizzled 128-byte row
+      const int byte = group * 32 + part * (4 * CPT);
+      uint32_t w[CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; i += 4) {
+        const int bi = byte + 4 * i;
+        const uint32_t wa = sW(ws) + static_cast<uint32_t>(r * 128 + (((bi >> 4) ^ (r & 7)) << 4) + (bi & 15));
+        if constexpr (CPT >= 4)
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]) : "r"(wa));
+        else
+          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w[i]), "=r"(w[i + 1]) : "r"(wa));
+      }
+      float scale = 0.f;
+      if (row_ok && kb < kbt) scale = s_code256[codes[r * kbt + kb]] * s_abs2[(int)(((rb0 + kb) >> 8) - grp0)] + p.offset;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_w_empty(ws));
+      const int st = kb >> 1, s = st % BS;
+      if (!mbar_wait(bar_b_empty(s), ((st / BS) & 1) ^ 1u, p.status, kTimeoutDequant)) { ok = false; break; }
+      const uint64_t scale2 = pack_f32x2(scale, scale);
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) {
+        uint32_t o[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const uint32_t off = ((b == 0 ? w[i] << 7 : w[i] >> (8 * b - 7)) & 0x7f80u) | copy;
+          const float2 v = *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(s_pair) + off);
+          float v0, v1;
+          unpack_f32x2(mul_f32x2(pack_f32x2(v.x, v.y), scale2), v0, v1);
+          o[b] = q4_pack2(v0, v1, FMT);
+        }
+        const int chunk = part * CPT + i;
+        const uint32_t addr = sB(s) + static_cast<uint32_t>((kb & 1) * (BN * 128) + r * 128 + ((chunk ^ (r & 7)) << 4));
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3])
+                     : "memory");
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_b_full(s));
+    }
+    if (ok && mbar_wait(bar_acc, 0, p.status, kTimeoutEpilogue)) {
+      tc_fence_after();
+      const int q = warp & 3;
+      const int row = m0 + q * 32 + lane;
+      const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+#pragma unroll 1
+      for (int c = (warp - 3) >> 2; c < BN / 32; c += Q4T_GROUPS) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem + lane_addr + c * 32, v);
+        tmem_ld_wait();
+        if (row < p.M) q4_store32(p, row, n0 + c * 32, v);
       }
     }
   }
@@ -488,6 +720,24 @@ static int q4_maps(CUtensorMap* tx, CUtensorMap* txa, CUtensorMap* tbl, const vo
   return 0;
 }
 
+// bytes of the codes and second-level scales of a tile in shared memory
+static int q4t_scale_bytes(int bn, int K) { return bn * (K / 64) + 16 + (bn * (K / 64) / 256 + 2) * 4; }
+
+template <int BN, int FMT>
+static int q4t_launch(const CUtensorMap& tx, const CUtensorMap& tw, const Q4Params& p, cudaStream_t stream) {
+  const int smem = Q4tCfg<BN>::kFixed + q4t_scale_bytes(BN, p.K);
+  static bool cfg = false;
+  if (!cfg) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_q4_tma_kernel<BN, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         Q4tCfg<BN>::kFixed + Q4tCfg<BN>::kScaleBytes);
+    if (e != cudaSuccess) return (int)e;
+    cfg = true;
+  }
+  dim3 grid((p.N + BN - 1) / BN, (p.M + Q4_BM - 1) / Q4_BM);
+  gemm_q4_tma_kernel<BN, FMT><<<grid, 96 + Q4T_DQ_THREADS, smem, stream>>>(tx, tw, p);
+  return (int)cudaGetLastError();
+}
+
 // x [M, K] (ldx), packed shards (world pointers, shard_bytes each; world = 1: one local pointer), scales either
 // `absmax` (fp32 per 64-block) or the double-quantised triple (absmax_q, code256, absmax2, offset); code16 = the
 // 16-entry NF4 / FP4 table (host pointer); optional LoRA pair xa [M, R] (ldxa), bl [N, R] (ldbl), R = r2;
@@ -535,6 +785,18 @@ extern "C" int fmsb_gemm_q4_fused(const void* x, long long ldx, void* const* pac
   }
   CUtensorMap tx, txa, tbl;
   if (int rc = q4_maps(&tx, &txa, &tbl, x, ldx, xa, ldxa, bl, ldbl, r2, M, N, K, bn)) return rc;
+  // One local, double-quantised weight without a LoRA pair: the packed bytes by TMA (16-byte aligned; the scale codes of a
+  // tile have to fit beside the stages: K up to about 15000 at 128 wide, 25000 at 64, more at 32).
+  const int room = bn == 128 ? Q4tCfg<128>::kScaleBytes : bn == 64 ? Q4tCfg<64>::kScaleBytes : Q4tCfg<32>::kScaleBytes;
+  if (world == 1 && xa == nullptr && absmax_q != nullptr && (reinterpret_cast<uintptr_t>(p.shard[0]) & 15u) == 0 &&
+      q4t_scale_bytes(bn, K) <= room) {
+    CUtensorMap tw;  // rows of K / 2 bytes, seen as K / 4 16-bit units
+    if (int rc = make_tmap_2d_16b(&tw, p.shard[0], N, K / 4, K / 4, bn, 64)) return rc;
+    if (bn == 128) return fmt == 1 ? q4t_launch<128, 1>(tx, tw, p, stream) : q4t_launch<128, 0>(tx, tw, p, stream);
+    if (bn == 64) return fmt == 1 ? q4t_launch<64, 1>(tx, tw, p, stream) : q4t_launch<64, 0>(tx, tw, p, stream);
+    if (bn == 32) return fmt == 1 ? q4t_launch<32, 1>(tx, tw, p, stream) : q4t_launch<32, 0>(tx, tw, p, stream);
+    return -2;
+  }
   if (bn == 128) return q4_launch<128, 0>(tx, txa, tbl, p, stream);
   if (bn == 64) return q4_launch<64, 0>(tx, txa, tbl, p, stream);
   if (bn == 32) return q4_launch<32, 0>(tx, txa, tbl, p, stream);

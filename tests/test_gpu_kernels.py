@@ -363,7 +363,8 @@ def test_fused_q4_gemm_matches_dequant_then_gemm(M, Nn, K, bn, double_quant, lor
 @pytest.mark.parametrize("M,Nn,K,dtype,double_quant", [
     (1, 8, 64, torch.bfloat16, True), (4, 4104, 64, torch.float16, False), (3, 4096, 4096, torch.bfloat16, True),
     (1, 1032, 14336, torch.float16, True), (3, 4096, 14336, torch.bfloat16, True), (4, 256, 14336, torch.bfloat16, True),
-    (5, 264, 192, torch.bfloat16, True), (77, 14336, 512, torch.bfloat16, True), (129, 4104, 256, torch.float16, False)])
+    (5, 264, 192, torch.bfloat16, True), (6, 1032, 64, torch.float16, True), (128, 4104, 14336, torch.bfloat16, True),
+    (40, 4736, 4160, torch.bfloat16, True), (130, 64, 320, torch.float16, True), (77, 14336, 512, torch.bfloat16, True), (129, 4104, 256, torch.float16, False)])
 def test_fused_q4_gemm_chosen_kernel_matches_fp64(M, Nn, K, dtype, double_quant):
     """The kernel the library chooses (few rows on the CUDA cores, else a tile width by size) against 64 bits.  The
     result is rounded to the 16-bit type once (half an ulp); the tensor-core form also rounds every weight (half an
