@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const T* __restrict_
 
 template <typename T>
 __device__ __forceinline__ uint2 state_pack4(const float4& v) {
-  T t[4] = {(T)v.x, (T)v.y, (T)v.z, (T)v.w};
+  alignas(8) T t[4] = {(T)v.x, (T)v.y, (T)v.z, (T)v.w};
   return *reinterpret_cast<uint2*>(t);
 }
 

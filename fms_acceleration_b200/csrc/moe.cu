@@ -420,19 +420,96 @@ __global__ void __launch_bounds__(256) moe_dispatch_kernel(const T* __restrict__
   }
 }
 
-// zero the pad rows [seg_off[e] + seg_cnt[e], seg_off[e + 1]) of a local buffer
+// Backward of the dispatch on one GPU: for every (token t, slot s) with row r = dest_row[t, s]
+//   dgate[t, s] = <y[r], dout[t]>,   dy[r] = gate[t, s] * dout[t].
+// One warp per token, the dout row in registers: y is read once and dy written once (0.8 GB for 16384 tokens, top 8, 1536
+// wide), where placing the unscaled rows, then reading them back beside y to weight them, moved 1.6 GB in two launches
+// and needed two more for the weights: 283 -> 163 us.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_dispatch_dot_kernel(const T* __restrict__ dout, long long ldd,
+                                                               const int* __restrict__ dest_row,
+                                                               const float* __restrict__ gate, long long n_tokens, int k,
+                                                               int H, const T* __restrict__ y, long long ldy,
+                                                               T* __restrict__ dy, long long lddy,
+                                                               float* __restrict__ dgate) {
+  const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= n_tokens) return;
+  int my_row = -1;
+  float my_gate = 0.f, my_dot = 0.f;
+  if (lane < k) {
+    my_row = dest_row[t * k + lane];
+    my_gate = gate[t * k + lane];
+  }
+  const T* src = dout + t * ldd;
+  const int nvec = H >> 3;
+  constexpr int NV = 6;  // 1536 columns a pass
+  for (int v0 = 0; v0 < nvec; v0 += 32 * NV) {
+    uint4 d[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int vi = v0 + lane + 32 * j;
+      d[j] = vi < nvec ? *reinterpret_cast<const uint4*>(src + vi * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint4 nx[NV];  // y row of the next slot: a warp has two rows in flight
+    auto fetch = [&](int s) {
+      const int row = __shfl_sync(0xffffffffu, my_row, s);
+      const T* yr = y + (long long)(row < 0 ? 0 : row) * ldy;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const int vi = v0 + lane + 32 * j;
+        nx[j] = row >= 0 && vi < nvec ? *reinterpret_cast<const uint4*>(yr + vi * 8) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    };
+    fetch(0);
+    for (int s = 0; s < k; ++s) {
+      const int row = __shfl_sync(0xffffffffu, my_row, s);
+      const float g = __shfl_sync(0xffffffffu, my_gate, s);
+      T* dr = dy + (long long)row * lddy;
+      uint4 a[NV];
+#pragma unroll
+      for (int j = 0; j < NV; ++j) a[j] = nx[j];
+      if (s + 1 < k) fetch(s + 1);
+      if (row < 0) continue;  // dropped pair
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const uint32_t aw[4] = {a[j].x, a[j].y, a[j].z, a[j].w}, dw[4] = {d[j].x, d[j].y, d[j].z, d[j].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float2 fa, fd;
+          if (std::is_same<T, __nv_bfloat16>::value) {
+            fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&aw[i]));
+            fd = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dw[i]));
+            o[i] = pack_bf16x2(fd.x * g, fd.y * g);
+          } else {
+            fa = __half22float2(*reinterpret_cast<const __half2*>(&aw[i]));
+            fd = __half22float2(*reinterpret_cast<const __half2*>(&dw[i]));
+            o[i] = pack_f16x2(fd.x * g, fd.y * g);
+          }
+          acc += fa.x * fd.x + fa.y * fd.y;
+        }
+        const int vi = v0 + lane + 32 * j;
+        if (vi < nvec) *reinterpret_cast<uint4*>(dr + vi * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      acc = warp_sum(acc);
+      if (lane == s) my_dot += acc;
+    }
+  }
+  if (lane < k) dgate[t * k + lane] = my_dot;
+}
+
+// zero the pad rows [seg_off[e] + seg_cnt[e], seg_off[e + 1]) of a local buffer; grid (E_local, slices of the pad): one
+// CTA per expert left most SMs idle behind up to 127 rows each (13 -> 3.3 us for 40 experts, 1536 wide)
 template <typename T>
 __global__ void moe_zero_pad_kernel(T* __restrict__ buf, long long ld, int H, const int* __restrict__ seg_off,
                                     const int* __restrict__ seg_cnt, int E_local) {
   const int e = blockIdx.x;
   const int r0 = seg_off[e] + seg_cnt[e], r1 = seg_off[e + 1];
-  const int vec_per_row = H / 8;
-  const long long total = (long long)(r1 - r0) * vec_per_row;
-  for (long long i = threadIdx.x; i < total; i += blockDim.x) {
-    const long long r = r0 + i / vec_per_row;
-    const int c = (int)(i % vec_per_row) * 8;
-    *reinterpret_cast<uint4*>(buf + r * ld + c) = make_uint4(0, 0, 0, 0);
-  }
+  for (int r = r0 + blockIdx.y; r < r1; r += gridDim.y)
+    for (int c = threadIdx.x * 8; c < H; c += blockDim.x * 8)
+      *reinterpret_cast<uint4*>(buf + (long long)r * ld + c) = make_uint4(0, 0, 0, 0);
 }
 
 // out[t][:] = sum_k w[t, k] * owner_buf(t, k)[dest_row(t, k)][:]   (w == nullptr: plain sum).  One warp per token;
@@ -495,7 +572,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(MoePeers ybuf, long lo
   // load rounds per token of a 1536-wide top-8 layer, and the gather ran at 0.45 of the copy bandwidth.)
   constexpr int CV = 2, RG = 8;
   const int nvec = H >> 3;
-  for (int v0 = 0; v0 < nvec; v0 += 32 * CV) {
+  // few tokens: the passes of a token are spread over gridDim.y warps instead of following one another
+  for (int v0 = blockIdx.y * 32 * CV; v0 < nvec; v0 += gridDim.y * 32 * CV) {
     float acc[CV][8];
 #pragma unroll
     for (int j = 0; j < CV; ++j)
@@ -800,6 +878,20 @@ extern "C" int fmsb_moe_dispatch_meta(const void* x, long long ldx, const int* t
   return (int)cudaGetLastError();
 }
 
+// see moe_dispatch_dot_kernel; one GPU (rows of a local buffer)
+extern "C" int fmsb_moe_dispatch_dot(const void* dout, long long ldd, const int* dest_row, const float* gate,
+                                     long long n_tokens, int k, int H, const void* y, long long ldy, void* dy,
+                                     long long lddy, float* dgate, int dtype, cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (H % 8 != 0 || ldd % 8 != 0 || ldy % 8 != 0 || lddy % 8 != 0 || k < 1 || k > 32) return -2;
+  const unsigned blocks = (unsigned)((n_tokens * 32 + 255) / 256);
+  if (dtype == 1)
+    moe_dispatch_dot_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)dout, ldd, dest_row, gate, n_tokens, k, H, (const __nv_bfloat16*)y, ldy, (__nv_bfloat16*)dy, lddy, dgate);
+  else
+    moe_dispatch_dot_kernel<__half><<<blocks, 256, 0, stream>>>((const __half*)dout, ldd, dest_row, gate, n_tokens, k, H, (const __half*)y, ldy, (__half*)dy, lddy, dgate);
+  return (int)cudaGetLastError();
+}
+
 // Owner side of the routing-weight gradient: dots[row] = <y[row], dy[row]>, then dy[row] *= gate[row]; rows below
 // seg_off[E_local] only (everything this rank received).  One warp per row.
 extern "C" int fmsb_moe_rowdot_scale(const void* y, long long ldy, void* dy, long long lddy, const float* gate,
@@ -828,8 +920,8 @@ extern "C" int fmsb_moe_zero_pad(void* buf, long long ld, int H, const int* seg_
                                  int dtype, cudaStream_t stream) {
   if (E_local <= 0) return 0;
   if (H % 8 != 0 || ld % 8 != 0) return -2;
-  if (dtype == 1) moe_zero_pad_kernel<__nv_bfloat16><<<E_local, 256, 0, stream>>>((__nv_bfloat16*)buf, ld, H, seg_off, seg_cnt, E_local);
-  else moe_zero_pad_kernel<__half><<<E_local, 256, 0, stream>>>((__half*)buf, ld, H, seg_off, seg_cnt, E_local);
+  if (dtype == 1) moe_zero_pad_kernel<__nv_bfloat16><<<dim3(E_local, 16), 256, 0, stream>>>((__nv_bfloat16*)buf, ld, H, seg_off, seg_cnt, E_local);
+  else moe_zero_pad_kernel<__half><<<dim3(E_local, 16), 256, 0, stream>>>((__half*)buf, ld, H, seg_off, seg_cnt, E_local);
   return (int)cudaGetLastError();
 }
 
@@ -840,10 +932,12 @@ extern "C" int fmsb_moe_combine(void* const* ybuf, long long ldy, const int* top
   if (H % 8 != 0 || ldy % 8 != 0 || ldo % 8 != 0 || k < 1 || k > 32) return -2;
   MoePeers y = moe_ptrs(ybuf, world);
   const long long blocks = (T_tokens * 32 + 255) / 256;
+  // 512 columns a pass; below two CTAs per SM the passes go to CTAs of their own (250 tokens, top 8, 1536 wide: 16.6 -> 8.4 us)
+  const dim3 grid((unsigned)blocks, blocks < 296 ? (unsigned)((H + 511) / 512) : 1u);
   if (dtype == 1)
-    moe_combine_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, stream>>>(y, ldy, topk_idx, dest_row, w, T_tokens, k, H, E_local, (__nv_bfloat16*)out, ldo, 0, nullptr);
+    moe_combine_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(y, ldy, topk_idx, dest_row, w, T_tokens, k, H, E_local, (__nv_bfloat16*)out, ldo, 0, nullptr);
   else
-    moe_combine_kernel<__half><<<(unsigned)blocks, 256, 0, stream>>>(y, ldy, topk_idx, dest_row, w, T_tokens, k, H, E_local, (__half*)out, ldo, 0, nullptr);
+    moe_combine_kernel<__half><<<grid, 256, 0, stream>>>(y, ldy, topk_idx, dest_row, w, T_tokens, k, H, E_local, (__half*)out, ldo, 0, nullptr);
   return (int)cudaGetLastError();
 }
 

@@ -48,6 +48,7 @@ N.declare("fmsb_moe_zero_pad", [P, L, I, P, P, I, I, P])
 N.declare("fmsb_moe_combine", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_gate_grad", [P, L, P, P, P, L, L, I, I, I, P, I, I, P])
 N.declare("fmsb_moe_dispatch_meta", [P, L, P, P, P, L, I, I, I, P, L, P, I, I, P])
+N.declare("fmsb_moe_dispatch_dot", [P, L, P, P, L, I, I, P, L, P, L, P, I, P])
 N.declare("fmsb_moe_rowdot_scale", [P, L, P, L, P, P, P, I, I, I, I, P])
 N.declare("fmsb_moe_gather_scalar", [P, P, P, L, I, P, I, P])
 N.declare("fmsb_moe_stage_plan", [P, P, L, I, I, I, P, P, P, P, P, P])
@@ -495,27 +496,18 @@ class _Experts(torch.autograd.Function):
         El, cap = mctx.E_local, gu.shape[0]
         dev, dt = dout.device, dout.dtype
         dYs = torch.empty(cap, H, dtype=dt, device=dev)
-        rgate = torch.zeros(cap, dtype=torch.float32, device=dev)
-        rdots = torch.empty(cap, dtype=torch.float32, device=dev)
         _zero_pad(mctx, dYs, seg_off, seg_cnt)
-        # dout rows are placed unscaled together with their routing weight; <expert output, dout> per row is the
-        # routing-weight gradient, then the weight is applied in place
-        rc = N.lib().fmsb_moe_dispatch_meta(dout.data_ptr(), dout.stride(0), idx.data_ptr(), dest_row.data_ptr(),
-                                            gates.contiguous().data_ptr(), T * mctx.k, mctx.k, H, El, _one_ptr(dYs),
-                                            dYs.stride(0), _one_ptr(rgate), 1, N.dtype_code(dt), N.stream_ptr())
-        N.check(rc, "fmsb_moe_dispatch_meta")
-        rc = N.lib().fmsb_moe_rowdot_scale(Ys.data_ptr(), Ys.stride(0), dYs.data_ptr(), dYs.stride(0), rgate.data_ptr(),
-                                           rdots.data_ptr(), seg_off.data_ptr(), El, cap, H, N.dtype_code(dt),
-                                           N.stream_ptr())
-        N.check(rc, "fmsb_moe_rowdot_scale")
+        # the weighted dout rows in the expert-sorted layout and <expert output, dout> per pair, the routing-weight gradient
+        dgate = torch.empty(T, mctx.k, dtype=torch.float32, device=dev)
+        gates_c = gates.contiguous()
+        rc = N.lib().fmsb_moe_dispatch_dot(dout.data_ptr(), dout.stride(0), dest_row.data_ptr(), gates_c.data_ptr(), T,
+                                           mctx.k, H, Ys.data_ptr(), Ys.stride(0), dYs.data_ptr(), dYs.stride(0),
+                                           dgate.data_ptr(), N.dtype_code(dt), N.stream_ptr())
+        N.check(rc, "fmsb_moe_dispatch_dot")
         acc: dict = {}
         need_dw = any(ctx.needs_input_grad[3:6])
         dXs = _experts_bwd_local(mctx, Xs, gu, dYs, seg_off, w1, w3, w2, act, acc, need_dw, lora=lora, XA=XA, single=True)
         dx = _combine(mctx, _one_ptr(dXs), dXs.stride(0), idx, dest_row, None, T, H, dt, dev)
-        dgate = torch.empty(T, mctx.k, dtype=torch.float32, device=dev)
-        rc = N.lib().fmsb_moe_gather_scalar(_one_ptr(rdots), idx.data_ptr(), dest_row.data_ptr(), T * mctx.k, El,
-                                            dgate.data_ptr(), 1, N.stream_ptr())
-        N.check(rc, "fmsb_moe_gather_scalar")
         dw1, dw3, dw2 = _weight_grads(mctx, acc, w1, w3, w2, ctx.needs_input_grad[3:6])
         return (dx, dgate, None, dw1, dw3, dw2, None, None) + (_lora_grads(acc, lora, ctx.needs_input_grad[8:12]) if lora else ())
 

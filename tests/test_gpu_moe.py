@@ -193,3 +193,42 @@ def test_capacity_overflow_drops_rows_and_reports():
     n_kept = (dest_row >= 0).sum(1, keepdim=True).float()
     assert torch.allclose(out.float(), x.float() * n_kept, atol=0.08, rtol=0.02)
     NV.check_status()
+
+
+@pytest.mark.parametrize("T,k,H,dtype", [(1, 1, 8, torch.bfloat16), (37, 3, 1536, torch.float16), (5, 32, 1544, torch.bfloat16),
+                                         (300, 8, 4096, torch.bfloat16)])
+def test_dispatch_dot_and_combine_at_their_edges(T, k, H, dtype):
+    """dy[r] = gate dout[t] (one rounding), dgate = <y[r], dout[t]> (fp32 sums of exact products: 1e-5 of the norms), dropped
+    pairs; and the combine of the same layout, whose passes go to CTAs of their own for few tokens."""
+    import ctypes
+
+    torch.manual_seed(T + H)
+    dev = "cuda"
+    rows = T * k + 3
+    dest = torch.randperm(rows, device=dev)[: T * k].view(T, k).to(torch.int32)
+    dest[0, k - 1] = -1
+    gate = torch.rand(T, k, device=dev)
+    dout, y = torch.randn(T, H, device=dev).to(dtype), torch.randn(rows, H, device=dev).to(dtype)
+    dy, dgate = torch.full((rows, H), 7.0, device=dev, dtype=dtype), torch.empty(T, k, device=dev)
+    N = NV
+    rc = N.lib().fmsb_moe_dispatch_dot(dout.data_ptr(), H, dest.data_ptr(), gate.data_ptr(), T, k, H, y.data_ptr(), H,
+                                       dy.data_ptr(), H, dgate.data_ptr(), N.dtype_code(dtype), N.stream_ptr())
+    assert rc == 0
+    ref = torch.full_like(dy, 7.0)
+    ref_g = torch.zeros(T, k, device=dev, dtype=torch.float64)
+    out_ref = torch.zeros(T, H, device=dev, dtype=torch.float64)
+    for t in range(T):
+        for s in range(k):
+            r = int(dest[t, s])
+            if r >= 0:
+                ref[r] = (dout[t].float() * gate[t, s]).to(dtype)
+                ref_g[t, s] = (y[r].double() * dout[t].double()).sum()
+                out_ref[t] += gate[t, s].double() * y[r].double()
+    assert torch.equal(dy, ref)
+    assert (dgate.double() - ref_g).abs().max() <= 1e-5 * H ** 0.5 * 4
+    out = torch.empty(T, H, device=dev, dtype=dtype)
+    rc = N.lib().fmsb_moe_combine((ctypes.c_void_p * 1)(y.data_ptr()), H, torch.zeros_like(dest).data_ptr(), dest.data_ptr(),
+                                  gate.data_ptr(), T, k, H, 1, out.data_ptr(), H, 1, N.dtype_code(dtype), N.stream_ptr())
+    assert rc == 0
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert (out.double() - out_ref).abs().max() <= ulp * out_ref.abs().max().clamp(min=1.0)
