@@ -12,6 +12,7 @@ states [nh, P, N] fp32.  T must be a multiple of the chunk size Q.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 import torch.nn.functional as F
@@ -419,6 +420,12 @@ def _fused_ok(x, B, C, Q):
             and x.dtype in (torch.bfloat16, torch.float16) and B.dtype == x.dtype and C.dtype == x.dtype)
 
 
+@functools.lru_cache(maxsize=256)
+def _fused_heads(kind, nc, nh, G):
+    hp = NV.lib().fmsb_ssdf_heads(kind, nc, nh, G)
+    return hp, -(-(nh // G) // hp)
+
+
 class _Fused:
     """Launches of the fused kernels for one call's geometry."""
 
@@ -435,8 +442,7 @@ class _Fused:
 
     def heads(self, kind):
         """(heads per CTA, number of head splits of a group) of a kernel."""
-        hp = NV.lib().fmsb_ssdf_heads(kind, self.nc, self.nh, self.G)
-        return hp, -(-(self.nh // self.G) // hp)
+        return _fused_heads(kind, self.nc, self.nh, self.G)
 
     def scan(self, mode, r, col, v, h, e=None, out=None, D=None, red=None):
         rc = NV.lib().fmsb_ssdf_scan(mode, r.data_ptr(), r.stride(0), col.data_ptr(), col.stride(0), v.data_ptr(),
