@@ -11,13 +11,17 @@
 //     compute order            A(j): P^T = exp2(S^T..) -> packed over S^T      (needs S^T(j))
 //                              B(j): dS^T = P^T o (dP^T - delta) -> over dP^T  (needs dP^T(j))
 //     dV(j) waits for A(j), dK(j) for B(j); A(j+1) runs while dK(j), dP^T(j+1) execute.
-//   dQ kernel (fixed query tile; Q and dO are copied ONCE into tensor memory as packed 16-bit and serve as the
-//     A operand of S = Q K^T and dP = dO V^T, so those products read only the K / V tile from shared memory)
-//     MMA order      S(j) dP(j) | S(j+1) | dQ(j) dP(j+1) | S(j+2) ...
+//   dQ kernel (fixed query tile; keys are streamed)
+//     MMA order      S(j) dP(j) | S(j+1) dP(j+1) | dQ(j) | S(j+2) dP(j+2) | dQ(j+1) ...
 //     compute order  load S(j) (then S(j+1) may overwrite it), P in registers, B(j): dS over dP(j)
+//     dP has two buffers: with one, dP(j+1) waited for dQ(j), which waits for B(j), and every block was that chain.
+//     The second one takes the room that Q and dO had in tensor memory as A operands; they are read from shared memory.
+//     V is released by dP(j), K by dQ(j), so half of the next loads start a product earlier.
 //
-// Tensor memory (512 columns): dK/dV: S^T 128 | dP^T 128 | dV D | dK D.   dQ: Q D/2 | dO D/2 | S 128 | dP 128 | dQ D.
+// Tensor memory (512 columns): dK/dV: S^T 128 | dP^T 128 | dV D | dK D.   dQ: S 128 | dP 2 x 128 | dQ D.
 // P is kept as packed 16-bit between the stages (it is the operand of dV in that precision anyway).
+// T = 16384 packed, 32/8 heads, d = 128: dQ 919 -> 874 us, dK/dV 1050 -> 886 us (heads fastest in the grids, fp32 pairs);
+// T = 1500, d = 64: dQ 29.4 -> 22.9 us.
 // Warp roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute; a compute warp owns lane
 // quarter `warp % 4` and 64 of the 128 columns.  Every wait is bounded.
 #include "common.cuh"
@@ -118,8 +122,8 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   float* scal_f = reinterpret_cast<float*>(smem_raw + (scal - smem_u32(smem_raw)));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x;
-  const int hk = blockIdx.y;
+  const int kt = blockIdx.y;  // early tiles have the most queries: they start first, heads fastest
+  const int hk = blockIdx.x;
   const int G = p.nh / p.nkv;
   const int k0 = kt * B3_T;
   const int k_last = min(k0 + B3_T - 1, p.T - 1);
@@ -237,6 +241,7 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const float LOG2E = 1.4426950408889634f;
     const float sl2 = p.scale * LOG2E;
+    const uint64_t sl2x2 = pack_f32x2(sl2, sl2);
     auto fetch = [&](int it, float& f, int& i) {
       const int head = hk * G + it / nq;
       const int t = (qb_lo + it % nq) * B3_T + (ctid & 127);
@@ -250,7 +255,7 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     };
     auto publish = [&](int buf, float f, int i) {
       float* b = scal_f + buf * 384;
-      b[ctid] = f;  // [0,128): lse*log2e, [128,256): delta
+      b[ctid] = -f;  // [0,128): -lse*log2e, [128,256): -delta
       if (ctid < 128) reinterpret_cast<int*>(b)[256 + ctid] = i;
     };
     float nf;
@@ -282,10 +287,10 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             const int col = c0 + c * 32 + i;
             const float4 l4 = *reinterpret_cast<const float4*>(b + col);
             float pv[4];
-            pv[0] = fast_exp2(__uint_as_float(rs[i]) * sl2 - l4.x);
-            pv[1] = fast_exp2(__uint_as_float(rs[i + 1]) * sl2 - l4.y);
-            pv[2] = fast_exp2(__uint_as_float(rs[i + 2]) * sl2 - l4.z);
-            pv[3] = fast_exp2(__uint_as_float(rs[i + 3]) * sl2 - l4.w);
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), sl2x2, pack_f32x2(l4.x, l4.y)), pv[0], pv[1]);
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i + 2]), __uint_as_float(rs[i + 3])), sl2x2, pack_f32x2(l4.z, l4.w)), pv[2], pv[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) pv[e] = fast_exp2(pv[e]);
             if (need_mask) {
               const int4 s4 = *reinterpret_cast<const int4*>(bi + col);
               const int t = q0 + col;
@@ -320,9 +325,10 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             float p0, p1, p2, p3;
             b3_unpack2(pk[c * 16 + i / 2], FMT, p0, p1);
             b3_unpack2(pk[c * 16 + i / 2 + 1], FMT, p2, p3);
-            dk[c * 16 + i / 2] = b3_pack2(p0 * (__uint_as_float(rp[i]) - d4.x), p1 * (__uint_as_float(rp[i + 1]) - d4.y), FMT);
-            dk[c * 16 + i / 2 + 1] =
-                b3_pack2(p2 * (__uint_as_float(rp[i + 2]) - d4.z), p3 * (__uint_as_float(rp[i + 3]) - d4.w), FMT);
+            unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), add_f32x2(pack_f32x2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), pack_f32x2(d4.x, d4.y))), p0, p1);
+            unpack_f32x2(mul_f32x2(pack_f32x2(p2, p3), add_f32x2(pack_f32x2(__uint_as_float(rp[i + 2]), __uint_as_float(rp[i + 3])), pack_f32x2(d4.z, d4.w))), p2, p3);
+            dk[c * 16 + i / 2] = b3_pack2(p0, p1, FMT);
+            dk[c * 16 + i / 2 + 1] = b3_pack2(p2, p3, FMT);
           }
         }
         tmem_st_32x32(tdP + lane_addr + c0, dk);
@@ -379,16 +385,18 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   auto sV = [&](int s) { return base + Cfg::kTileBytes * (3 + 2 * s); };
   const uint32_t bars = base + Cfg::kTileBytes * 6 + Cfg::kScalarBytes;
   const uint32_t bar_q = bars;
-  auto bar_kv_full = [&](int s) { return bars + 8u * (1 + s); };
-  auto bar_kv_empty = [&](int s) { return bars + 8u * (3 + s); };
-  const uint32_t bar_s_full = bars + 8u * 5, bar_dp_full = bars + 8u * 6;
-  const uint32_t bar_sa_done = bars + 8u * 7, bar_pb_full = bars + 8u * 8;
-  const uint32_t bar_acc_done = bars + 8u * 9, bar_qtm_full = bars + 8u * 10;
-  const uint32_t holder = bars + 8u * 11;
+  auto bar_k_full = [&](int s) { return bars + 8u * (1 + s); };
+  auto bar_k_empty = [&](int s) { return bars + 8u * (3 + s); };
+  auto bar_v_full = [&](int s) { return bars + 8u * (5 + s); };
+  auto bar_v_empty = [&](int s) { return bars + 8u * (7 + s); };
+  const uint32_t bar_s_full = bars + 8u * 9, bar_sa_done = bars + 8u * 10, bar_acc_done = bars + 8u * 11;
+  auto bar_dp_full = [&](int b) { return bars + 8u * (12 + b); };
+  auto bar_pb_full = [&](int b) { return bars + 8u * (14 + b); };
+  const uint32_t holder = bars + 8u * 16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // long tiles (late in their document) first
-  const int head = blockIdx.y;
+  const int qt = gridDim.y - 1 - blockIdx.y;  // long tiles (late in their document) first, heads fastest
+  const int head = blockIdx.x;
   const int hk = head / (p.nh / p.nkv);
   const int q0 = qt * B3_T;
   const int q_last = min(q0 + B3_T - 1, p.T - 1);
@@ -399,15 +407,16 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == 1 && lane == 0) {
     mbar_init(bar_q, 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(bar_kv_full(s), 1);
-      mbar_init(bar_kv_empty(s), 1);
+      mbar_init(bar_k_full(s), 1);
+      mbar_init(bar_k_empty(s), 1);
+      mbar_init(bar_v_full(s), 1);
+      mbar_init(bar_v_empty(s), 1);
+      mbar_init(bar_dp_full(s), 1);
+      mbar_init(bar_pb_full(s), 8);
     }
     mbar_init(bar_s_full, 1);
-    mbar_init(bar_dp_full, 1);
     mbar_init(bar_sa_done, 8);
-    mbar_init(bar_pb_full, 8);
     mbar_init(bar_acc_done, 1);
-    mbar_init(bar_qtm_full, 8);
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -419,7 +428,8 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(holder));
-  const uint32_t tQ = tmem, tdO = tmem + D / 2, tS = tmem + D, tdP = tmem + D + 128u, tdQ = tmem + D + 256u;
+  const uint32_t tS = tmem, tdQ = tmem + 384u;
+  auto tdP = [&](int b) { return tmem + 128u + 128u * b; };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -431,67 +441,69 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       for (int j = 0; j < nblk; ++j) {
         const int s = j & 1;
-        if (!mbar_wait(bar_kv_empty(s), ((j >> 1) & 1) ^ 1u, p.status, kTimeoutProducer)) break;
+        const uint32_t par = ((j >> 1) & 1) ^ 1u;
         const int k0 = (kb_lo + j) * B3_T;
-        mbar_expect_tx(bar_kv_full(s), 2 * Cfg::kTileBytes);
+        if (!mbar_wait(bar_v_empty(s), par, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(bar_v_full(s), Cfg::kTileBytes);
 #pragma unroll
-        for (int h = 0; h < NH; ++h) {
-          tma_load_2d(sK(s) + h * Cfg::kHalfBytes, &tmK, bar_kv_full(s), hk * D + 64 * h, k0);
-          tma_load_2d(sV(s) + h * Cfg::kHalfBytes, &tmV, bar_kv_full(s), hk * D + 64 * h, k0);
-        }
+        for (int h = 0; h < NH; ++h) tma_load_2d(sV(s) + h * Cfg::kHalfBytes, &tmV, bar_v_full(s), hk * D + 64 * h, k0);
+        if (!mbar_wait(bar_k_empty(s), par, p.status, kTimeoutProducer)) break;
+        mbar_expect_tx(bar_k_full(s), Cfg::kTileBytes);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) tma_load_2d(sK(s) + h * Cfg::kHalfBytes, &tmK, bar_k_full(s), hk * D + 64 * h, k0);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc_s = make_idesc_f16(128, 128, FMT, 0, 0);
       const uint32_t idesc_g = make_idesc_f16(128, D, FMT, 0, 1);
-      auto issue_scores = [&](uint32_t acc, uint32_t a_tmem, uint32_t b_tile, uint32_t bar) {  // acc = A[tmem] . B^T
-        const SmemDescBase b = make_smem_desc_base(b_tile, 16, 1024);
+      auto issue_scores = [&](uint32_t acc, uint32_t a_tile, uint32_t b_tile, uint32_t bar) {  // acc = A . B^T
+        const SmemDescBase a = make_smem_desc_base(a_tile, 16, 1024), b = make_smem_desc_base(b_tile, 16, 1024);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const uint32_t off = (ks / 4) * Cfg::kHalfBytes + (ks % 4) * 32;
-          tc_mma_f16_ts(acc, a_tmem + ks * 8, smem_desc_at(b, off), idesc_s, ks != 0 ? 1u : 0u);
+          tc_mma_f16(acc, smem_desc_at(a, off), smem_desc_at(b, off), idesc_s, ks != 0 ? 1u : 0u);
         }
         tc_commit(bar);
       };
       auto issue_dq = [&](int s, bool first) {  // dQ += dS K
         const SmemDescBase b = make_smem_desc_base(sK(s), Cfg::kHalfBytes, 1024);
-        tc_mma_f16_ts(tdQ, tdP + b3_pcol(0), smem_desc_at(b, 0), idesc_g, first ? 0u : 1u);
+        const uint32_t ds = tdP(s);
+        tc_mma_f16_ts(tdQ, ds + b3_pcol(0), smem_desc_at(b, 0), idesc_g, first ? 0u : 1u);
 #pragma unroll
-        for (int ks = 1; ks < 8; ++ks) tc_mma_f16_ts(tdQ, tdP + b3_pcol(ks), smem_desc_at(b, ks * 2048), idesc_g, 1u);
+        for (int ks = 1; ks < 8; ++ks) tc_mma_f16_ts(tdQ, ds + b3_pcol(ks), smem_desc_at(b, ks * 2048), idesc_g, 1u);
       };
-      const bool tr = blockIdx.x == gridDim.x / 2 && blockIdx.y == 0;
+      const bool tr = blockIdx.y == gridDim.y / 2 && blockIdx.x == 0;
       FMSB_TRACE3(tr, 4000);
-      bool ok = mbar_wait(bar_qtm_full, 0, p.status, kTimeoutMma);
+      bool ok = mbar_wait(bar_q, 0, p.status, kTimeoutMma);
       FMSB_TRACE3(tr, 4001);
-      if (ok) ok = mbar_wait(bar_kv_full(0), 0, p.status, kTimeoutMma);
-      if (ok) {
-        tc_fence_after();
-        issue_scores(tS, tQ, sK(0), bar_s_full);
-        issue_scores(tdP, tdO, sV(0), bar_dp_full);
-      }
-      FMSB_TRACE3(tr, 4002);
-      for (int j = 0; j < nblk && ok; ++j) {
-        const int s = j & 1;
-        const bool more = j + 1 < nblk;
-        FMSB_TRACE3(tr, 4096 + 8 * j + 0);
-        if (more) {
+      for (int j = -1; j < nblk && ok; ++j) {
+        FMSB_TRACE3(tr, 4096 + 8 * (j + 1) + 0);
+        if (j + 1 < nblk) {
+          const int n = j + 1, s = n & 1;
+          const uint32_t par = (n >> 1) & 1;
           // S(j) is in the compute warps' registers: S(j+1) may overwrite it while they work
-          if (!mbar_wait(bar_sa_done, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
-          if (!mbar_wait(bar_kv_full(s ^ 1), ((j + 1) >> 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+          if (j >= 0 && !mbar_wait(bar_sa_done, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
+          if (!mbar_wait(bar_k_full(s), par, p.status, kTimeoutMma)) { ok = false; break; }
           tc_fence_after();
-          FMSB_TRACE3(tr, 4096 + 8 * j + 1);
-          issue_scores(tS, tQ, sK(s ^ 1), bar_s_full);
-          FMSB_TRACE3(tr, 4096 + 8 * j + 2);
+          FMSB_TRACE3(tr, 4096 + 8 * (j + 1) + 1);
+          issue_scores(tS, sQ, sK(s), bar_s_full);
+          if (!mbar_wait(bar_v_full(s), par, p.status, kTimeoutMma)) { ok = false; break; }
+          tc_fence_after();
+          // dS(j-1) in this buffer has been read: dQ(j-1) was issued before this product
+          issue_scores(tdP(s), sdO, sV(s), bar_dp_full(s));
+          tc_commit(bar_v_empty(s));
+          FMSB_TRACE3(tr, 4096 + 8 * (j + 1) + 2);
         }
-        if (!mbar_wait(bar_pb_full, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
-        tc_fence_after();
-        FMSB_TRACE3(tr, 4096 + 8 * j + 3);
-        issue_dq(s, j == 0);
-        tc_commit(bar_kv_empty(s));
-        FMSB_TRACE3(tr, 4096 + 8 * j + 4);
-        if (more) issue_scores(tdP, tdO, sV(s ^ 1), bar_dp_full);
-        FMSB_TRACE3(tr, 4096 + 8 * j + 5);
+        if (j >= 0) {
+          const int s = j & 1;
+          if (!mbar_wait(bar_pb_full(s), (j >> 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+          tc_fence_after();
+          FMSB_TRACE3(tr, 4096 + 8 * (j + 1) + 3);
+          issue_dq(s, j == 0);
+          tc_commit(bar_k_empty(s));
+          FMSB_TRACE3(tr, 4096 + 8 * (j + 1) + 4);
+        }
       }
       if (ok) tc_commit(bar_acc_done);
       FMSB_TRACE3(tr, 4003);
@@ -508,45 +520,10 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float sl2 = p.scale * LOG2E;
     const float lse2 = row_ok ? p.lse[(long long)head * p.T + t] * LOG2E : 0.f;
     const float dlt = row_ok ? p.delta[(long long)head * p.T + t] : 0.f;
+    const uint64_t sl2x2 = pack_f32x2(sl2, sl2), nlse2 = pack_f32x2(-lse2, -lse2), ndlt2 = pack_f32x2(-dlt, -dlt);
     const int c0 = chalf * 64;
-    const bool trc = blockIdx.x == gridDim.x / 2 && blockIdx.y == 0 && threadIdx.x == 64;
-    FMSB_TRACE3(trc, 10);
-    bool ok = mbar_wait(bar_q, 0, p.status, kTimeoutEpilogue);
-    FMSB_TRACE3(trc, 11);
-    // ---- Q and dO rows into tensor memory as packed 16-bit A operands (row = lane)
-    if (ok) {
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const uint32_t src = (m == 0 ? sQ : sdO);
-        const uint32_t dst = (m == 0 ? tQ : tdO);
-        if constexpr (D == 128) {
-          uint32_t w[32];
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch) {
-            const uint32_t addr = src + chalf * Cfg::kHalfBytes + static_cast<uint32_t>(row * 128 + ((ch ^ (row & 7)) << 4));
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(w[ch * 4]), "=r"(w[ch * 4 + 1]), "=r"(w[ch * 4 + 2]), "=r"(w[ch * 4 + 3])
-                         : "r"(addr));
-          }
-          tmem_st_32x32(dst + lane_addr + chalf * 32, w);
-        } else {
-          uint32_t w[16];
-#pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            const int ch = chalf * 4 + c4;
-            const uint32_t addr = src + static_cast<uint32_t>(row * 128 + ((ch ^ (row & 7)) << 4));
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(w[c4 * 4]), "=r"(w[c4 * 4 + 1]), "=r"(w[c4 * 4 + 2]), "=r"(w[c4 * 4 + 3])
-                         : "r"(addr));
-          }
-          tmem_st_32x16(dst + lane_addr + chalf * 16, w);
-        }
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_qtm_full);
-    }
+    const bool trc = blockIdx.y == gridDim.y / 2 && blockIdx.x == 0 && threadIdx.x == 64;
+    bool ok = true;
     FMSB_TRACE3(trc, 12);
     for (int j = 0; j < nblk && ok; ++j) {
       const int k0 = (kb_lo + j) * B3_T;
@@ -566,10 +543,13 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (lane == 0) mbar_arrive(bar_sa_done);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0 = fast_exp2(__uint_as_float(rs0[i]) * sl2 - lse2);
-          float p1 = fast_exp2(__uint_as_float(rs0[i + 1]) * sl2 - lse2);
-          float p2 = fast_exp2(__uint_as_float(rs1[i]) * sl2 - lse2);
-          float p3 = fast_exp2(__uint_as_float(rs1[i + 1]) * sl2 - lse2);
+          float p0, p1, p2, p3;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs0[i]), __uint_as_float(rs0[i + 1])), sl2x2, nlse2), p0, p1);
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs1[i]), __uint_as_float(rs1[i + 1])), sl2x2, nlse2), p2, p3);
+          p0 = fast_exp2(p0);
+          p1 = fast_exp2(p1);
+          p2 = fast_exp2(p2);
+          p3 = fast_exp2(p3);
           if (need_mask) {
             const int kk = k0 + c0 + i;
             if (!(row_ok && kk >= ds && kk <= t)) p0 = 0.f;
@@ -582,27 +562,29 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       FMSB_TRACE3(trc, 64 + 8 * j + 2);
-      if (!mbar_wait(bar_dp_full, j & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
+      if (!mbar_wait(bar_dp_full(j & 1), (j >> 1) & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
       tc_fence_after();
       FMSB_TRACE3(trc, 64 + 8 * j + 3);
       uint32_t dk[32];
+      const uint32_t tdp = tdP(j & 1) + lane_addr + c0;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t rp[32];
-        tmem_ld_32x32(tdP + lane_addr + c0 + c * 32, rp);
+        tmem_ld_32x32(tdp + c * 32, rp);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float p0, p1;
           b3_unpack2(pk[c * 16 + i / 2], FMT, p0, p1);
-          dk[c * 16 + i / 2] = b3_pack2(p0 * (__uint_as_float(rp[i]) - dlt), p1 * (__uint_as_float(rp[i + 1]) - dlt), FMT);
+          unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), add_f32x2(pack_f32x2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), ndlt2)), p0, p1);
+          dk[c * 16 + i / 2] = b3_pack2(p0, p1, FMT);
         }
       }
-      tmem_st_32x32(tdP + lane_addr + c0, dk);
+      tmem_st_32x32(tdp, dk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_pb_full);
+      if (lane == 0) mbar_arrive(bar_pb_full(j & 1));
       FMSB_TRACE3(trc, 64 + 8 * j + 4);
     }
     FMSB_TRACE3(trc, 13);
@@ -673,7 +655,7 @@ extern "C" int fmsb_attn_bwd_dq3(const void* q, long long ldq, const void* k, lo
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end; p.lse = lse; p.delta = delta;
   p.dq = dq; p.lddq = lddq; p.fmt = fmt; p.status = status;
-  dim3 grid((T + B3_T - 1) / B3_T, nh);
+  dim3 grid(nh, (T + B3_T - 1) / B3_T);
 #define FMSB_B3(DD, FF)                                                                                          \
   do {                                                                                                           \
     static bool cfg = false;                                                                                     \
@@ -706,7 +688,7 @@ extern "C" int fmsb_attn_bwd_dkv3(const void* q, long long ldq, const void* k, l
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end; p.lse = lse; p.delta = delta;
   p.dk = dk; p.lddk = lddk; p.dv = dv; p.lddv = lddv; p.fmt = fmt; p.status = status;
-  dim3 grid((T + B3_T - 1) / B3_T, nkv);
+  dim3 grid(nkv, (T + B3_T - 1) / B3_T);
 #define FMSB_B3(DD, FF)                                                                                          \
   do {                                                                                                           \
     static bool cfg = false;                                                                                     \

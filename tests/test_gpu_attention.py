@@ -56,6 +56,31 @@ def test_attention_forward_extreme_scores(d, lens):
     assert _rel(o, ref) < 2 * 2.0 ** -8
 
 
+@pytest.mark.parametrize("d,dtype", [(128, torch.float16), (64, torch.float16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("lens", [[1], [127, 1], [1150], [129, 640, 1, 257]])
+def test_attention_backward_ring_lengths(d, dtype, lens):
+    """One to nine key blocks per query tile (the buffers and rings of the backward wrap at two), three query heads per
+    key head, against fp32.  P and dS are rounded to 16 bits, sums are fp32: 4 ulp of the gradient in the 2-norm."""
+    T, nh, nkv = sum(lens), 6, 2
+    qkv, ds, de = _make(T, nh, nkv, d, lens, dtype, seed=5)
+    q = qkv[:, : nh * d].reshape(T, nh, d).clone().requires_grad_()
+    k = qkv[:, nh * d: (nh + nkv) * d].reshape(T, nkv, d).clone().requires_grad_()
+    v = qkv[:, (nh + nkv) * d:].reshape(T, nkv, d).clone().requires_grad_()
+    o = AT.varlen_attention(q, k, v, ds, de)
+    g = torch.randn_like(o)
+    got = torch.autograd.grad(o, (q, k, v), g)
+    NV.check_status()
+    qf, kf, vf = (t.detach().double().requires_grad_() for t in (q, k, v))
+    rep = nh // nkv
+    mask = (torch.arange(T, device=DEV)[None] <= torch.arange(T, device=DEV)[:, None]) & (
+        torch.arange(T, device=DEV)[None] >= ds.long()[:, None])
+    s = torch.einsum("thd,shd->hts", qf, kf.repeat_interleave(rep, 1)) * d ** -0.5
+    ref = torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(~mask, float("-inf")), -1), vf.repeat_interleave(rep, 1))
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, r in zip(got, torch.autograd.grad(ref, (qf, kf, vf), g.double())):
+        assert (a.double() - r).norm() <= 4 * ulp * r.norm() + 1e-6 * g.double().norm()
+
+
 @pytest.mark.parametrize("d", [128, 64])
 @pytest.mark.parametrize("lens", [[256], [100, 156, 7, 249], [640, 129, 255]])
 def test_attention_backward(d, lens):
