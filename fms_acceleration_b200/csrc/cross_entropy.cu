@@ -129,7 +129,10 @@ ce_kernel(T* logits, long long row_stride, const long long* __restrict__ labels,
 #pragma unroll
       for (int i = 0; i < n; ++i) {
         s += __expf(f[u][i] - nm);  // exp(-inf) = 0 for the slots beyond the row
-        if (ok) acc.t += f[u][i];
+      }
+      if (label_smoothing > 0.f && ok) {  // the plain sum serves label smoothing only
+#pragma unroll
+        for (int i = 0; i < n; ++i) acc.t += f[u][i];
       }
     }
     acc.m = nm;
@@ -183,16 +186,33 @@ ce_kernel(T* logits, long long row_stride, const long long* __restrict__ labels,
     if (scale_ptr != nullptr) sc *= *scale_ptr;
     if (row_scale != nullptr) sc *= row_scale[row];
     const float eps_v = label_smoothing / (float)V;
-    for (int v = threadIdx.x; v < nvec; v += CE_THREADS) {
-      float f[n];
-      load_vec<T>(x + v * n, f);
+    // four vectors a trip, their loads (L2: this CTA has just read the row) in flight together; one test per vector for
+    // the label instead of a 64-bit comparison per element
+    const long long lv = label / n;
+    for (int v0 = threadIdx.x; v0 < nvec; v0 += CE_THREADS * U) {
+      uint4 raw[U];
 #pragma unroll
-      for (int i = 0; i < n; ++i) {
-        float g = __expf(f[i] - lse) - eps_v;
-        if ((long long)(v * n + i) == label) g -= (1.f - label_smoothing);
-        f[i] = g * sc;
+      for (int u = 0; u < U; ++u) {
+        const int v = v0 + u * CE_THREADS;
+        if (v < nvec) raw[u] = *reinterpret_cast<const uint4*>(x + v * n);
       }
-      store_vec<T>(x + v * n, f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int v = v0 + u * CE_THREADS;
+        if (v >= nvec) continue;
+        const T* e = reinterpret_cast<const T*>(&raw[u]);
+        float f[n];
+#pragma unroll
+        for (int i = 0; i < n; ++i) f[i] = __expf(ld_as_float<T>(e + i) - lse) - eps_v;
+        if (v == lv) {
+#pragma unroll
+          for (int i = 0; i < n; ++i)
+            if (i == (int)(label - lv * n)) f[i] -= (1.f - label_smoothing);
+        }
+#pragma unroll
+        for (int i = 0; i < n; ++i) f[i] *= sc;
+        store_vec<T>(x + v * n, f);
+      }
     }
     for (int i = nvec * n + threadIdx.x; i < V; i += CE_THREADS) {
       float g = __expf(ld_as_float<T>(x + i) - lse) - eps_v;

@@ -595,6 +595,21 @@ glu_bwd_kernel(const T* __restrict__ dh, const T* e, const T* g, T* de, T* dg, T
 }
 
 // y = a + b (residual add), 16-bit
+// out (16-bit) = src (fp32) * *factor: the gradient of a weight that was accumulated in fp32, scaled and rounded in one pass
+// (a broadcast product and a cast, each a pass of its own, took 262 us for 75.5 M elements; 450 MB are 68 us).
+template <typename T>
+__global__ void __launch_bounds__(256) scale_cast_kernel(const float* __restrict__ src, const float* __restrict__ factor,
+                                                         T* __restrict__ out, long long n8, long long n) {
+  const float f = *factor;
+  const long long stride = (long long)gridDim.x * blockDim.x, i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = i0; i < n8; i += stride) {
+    const float4 a = reinterpret_cast<const float4*>(src)[2 * i], b = reinterpret_cast<const float4*>(src)[2 * i + 1];
+    alignas(16) T t[8] = {(T)(a.x * f), (T)(a.y * f), (T)(a.z * f), (T)(a.w * f), (T)(b.x * f), (T)(b.y * f), (T)(b.z * f), (T)(b.w * f)};
+    reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(t);
+  }
+  for (long long i = n8 * 8 + i0; i < n; i += stride) out[i] = (T)(src[i] * f);
+}
+
 template <typename T>
 __global__ void add_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long n8) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n8;
@@ -888,5 +903,17 @@ extern "C" int fmsb_adamw(void* p, const void* g, void* m, void* v, long long n,
   else if (dtype == 2) FMSB_ADAMW(float, 2);
   else return -2;
 #undef FMSB_ADAMW
+  return (int)cudaGetLastError();
+}
+
+extern "C" int fmsb_scale_cast(const float* src, const float* factor, void* out, long long n, int dtype, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  const long long n8 = aligned ? n / 8 : 0;
+  long long blocks = ((aligned ? n8 + 7 : n) + 255) / 256;
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (dtype == 1) scale_cast_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, stream>>>(src, factor, (__nv_bfloat16*)out, n8, n);
+  else if (dtype == 0) scale_cast_kernel<__half><<<(unsigned)blocks, 256, 0, stream>>>(src, factor, (__half*)out, n8, n);
+  else return -2;
   return (int)cudaGetLastError();
 }

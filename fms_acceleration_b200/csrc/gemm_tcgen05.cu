@@ -1093,8 +1093,11 @@ extern "C" int fmsb_gemm(const void* A1, long long lda1, const void* B1, long lo
                          void* D, long long ldd, int d_fp32, const void* C, long long ldc,        //
                          float alpha, float beta, int M, int N, int fmt, int bn, int max_ctas, int* status,
                          cudaStream_t stream) {
-  return gemm_impl(A1, lda1, B1, ldb1, K1, A2, lda2, B2, ldb2, K2, a_mn, b_mn, D, ldd, d_fp32, C, ldc, alpha, beta, M,
-                   N, fmt, bn, max_ctas, status, stream, 0, 0, nullptr, 0, 0, 0, 0);
+  // d_fp32: bit 0 = D in fp32, bit 1 = C in fp32 (accumulation over calls: C = D, beta = 1)
+  GroupExtra gx;
+  gx.c_fp32 = (d_fp32 >> 1) & 1;
+  return gemm_impl(A1, lda1, B1, ldb1, K1, A2, lda2, B2, ldb2, K2, a_mn, b_mn, D, ldd, d_fp32 & 1, C, ldc, alpha, beta, M,
+                   N, fmt, bn, max_ctas, status, stream, 0, 0, nullptr, 0, 0, 0, 0, nullptr, &gx);
 }
 
 // Grouped GEMM for mixture-of-experts layers.  seg_off[g] (device, n_groups + 1 ints, multiples of 128) are the

@@ -10,6 +10,8 @@ Reference behaviour:
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 import torch.nn.functional as F
 
@@ -138,7 +140,7 @@ class _FusedLinearCE(torch.autograd.Function):
             scale = torch.full((1,), 1.0 / float(num_items), dtype=torch.float32, device=x.device) \
                 if not torch.is_tensor(num_items) else (1.0 / num_items.float().reshape(1))
         dx = torch.empty_like(x)
-        dw = torch.zeros(V, H, dtype=torch.float32, device=x.device) if need_dw else None
+        dw = None
         loss_rows = torch.empty(T, dtype=torch.float32, device=x.device)
         C = _chunk_rows(T, V, x.element_size())
         # rows of the logits chunk start on 16-byte boundaries whatever the vocabulary size (49155 for Granite)
@@ -151,7 +153,11 @@ class _FusedLinearCE(torch.autograd.Function):
             loss_rows[s:e] = l
             gemm(lg, weight, b_mn=True, out=dx[s:e])  # dx = dlogits @ W
             if need_dw:
-                _accumulate_dw(dw, lg, x[s:e])  # dW[V,H] += dlogits^T[V,rows] @ x[rows,H]
+                # dW[V,H] += dlogits^T[V,rows] @ x[rows,H]; the first chunk writes, the others add in the epilogue
+                if dw is None:
+                    dw = gemm(lg, x[s:e], a_mn=True, b_mn=True, out_dtype=torch.float32)
+                else:
+                    gemm(lg, x[s:e], a_mn=True, b_mn=True, c=dw, beta=1.0, out=dw)
         loss = loss_rows.sum() * scale[0]
         ctx.save_for_backward(dx, dw)
         ctx.wdtype = weight.dtype
@@ -161,13 +167,22 @@ class _FusedLinearCE(torch.autograd.Function):
     def backward(ctx, dloss):
         dx, dw = ctx.saved_tensors
         gx = dx * dloss.to(dx.dtype)
-        gw = None if dw is None else (dw * dloss).to(ctx.wdtype)
+        gw = None if dw is None else _scaled_cast(dw, dloss, ctx.wdtype)
         return gx, gw, None, None, None, None, None
 
 
-def _accumulate_dw(dw, dlogits, x):
-    part = gemm(dlogits, x, a_mn=True, b_mn=True, out_dtype=torch.float32)
-    dw.add_(part)
+N.declare("fmsb_scale_cast", [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p])
+
+
+def _scaled_cast(src, factor, dtype):
+    """``(src * factor).to(dtype)`` for a dense fp32 ``src`` and a device scalar, in one pass."""
+    if dtype not in (torch.bfloat16, torch.float16) or factor.dtype != torch.float32 or not src.is_contiguous():
+        return (src * factor).to(dtype)
+    out = torch.empty(src.shape, dtype=dtype, device=src.device)
+    rc = N.lib().fmsb_scale_cast(src.data_ptr(), factor.data_ptr(), out.data_ptr(), src.numel(), N.dtype_code(dtype),
+                                 N.stream_ptr())
+    N.check(rc, "fmsb_scale_cast")
+    return out
 
 
 def fused_linear_cross_entropy(x, weight, labels, ignore_index=IGNORE_INDEX, num_items=None, label_smoothing=0.0):

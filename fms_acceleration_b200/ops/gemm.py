@@ -114,7 +114,8 @@ def gemm(
     if out.dtype not in (a.dtype, torch.float32):
         raise TypeError("output must have the operand dtype or fp32")
     if c is not None:
-        if c.shape != (M, Nn) or c.stride(1) != 1 or c.dtype != a.dtype:
+        # an fp32 `c` (with an fp32 `out`, usually the same tensor) accumulates over calls
+        if c.shape != (M, Nn) or c.stride(1) != 1 or (c.dtype != a.dtype and not (c.dtype == out.dtype == torch.float32)):
             raise ValueError("bad `c`")
     if bn is None:
         bn = _pick_bn(Nn, b_mn)
@@ -127,7 +128,7 @@ def gemm(
         a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), K,
         N.ptr(a2), a2.stride(0) if a2 is not None else 0, N.ptr(b2), b2.stride(0) if b2 is not None else 0, K2,
         int(a_mn), int(b_mn),
-        out.data_ptr(), out.stride(0), int(out.dtype == torch.float32),
+        out.data_ptr(), out.stride(0), int(out.dtype == torch.float32) + 2 * int(c is not None and c.dtype == torch.float32),
         N.ptr(c), c.stride(0) if c is not None else 0,
         float(alpha), float(beta), M, Nn, N.dtype_code(a.dtype), bn, int(max_ctas),
         status.data_ptr(), N.stream_ptr(),

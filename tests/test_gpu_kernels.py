@@ -530,3 +530,54 @@ def test_adamw_kernel_matches_torch_fused(dtype, n):
     o2.step()
     o3.step()
     assert (a2.float() - b2.float()).abs().max() <= tol * (1 + b2.float().abs().max())
+
+
+@pytest.mark.parametrize("M,Nn,K", [(256, 512, 64), (300, 776, 192), (4099, 264, 136), (2050, 1536, 200)])
+@pytest.mark.parametrize("trans", [False, True])
+def test_gemm_accumulates_in_fp32_over_calls(M, Nn, K, trans):
+    """``out = c = dw`` in fp32 with ``beta = 1``: two products summed in the epilogue equal their fp32 sum (the
+    accumulation order inside a product is the kernel's; 1e-5 of the result's scale)."""
+    from fms_acceleration_b200.ops.gemm import gemm
+
+    torch.manual_seed(M)
+    rows = lambda n, c: torch.randn(n, (c + 7) // 8 * 8, device=DEV).bfloat16()[:, :c]
+    a, a2 = (rows(K, M), rows(K, M)) if trans else (rows(M, K), rows(M, K))
+    b, b2 = (rows(K, Nn), rows(K, Nn)) if trans else (rows(Nn, K), rows(Nn, K))
+    acc = gemm(a, b, a_mn=trans, b_mn=trans, out_dtype=torch.float32)
+    gemm(a2, b2, a_mn=trans, b_mn=trans, c=acc, beta=1.0, out=acc)
+    NV.check_status()
+    f = (lambda x, y: x.double().t() @ y.double()) if trans else (lambda x, y: x.double() @ y.double().t())
+    ref = f(a, b) + f(a2, b2)
+    assert (acc.double() - ref).abs().max() <= 1e-5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("M,Nn,K", [(300, 520, 64), (257, 264, 4096), (2048, 512, 8256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_residual_over_ragged_tiles_and_both_kernels(M, Nn, K, dtype):
+    """The residual in the store epilogue: whole and clipped chunks, aligned and unaligned residual rows, single CTAs and
+    pairs.  One rounding of the 16-bit result (half an ulp of the largest value)."""
+    from fms_acceleration_b200.ops import gemm as G
+
+    torch.manual_seed(M + K)
+    x, w = torch.randn(M, K, device=DEV).to(dtype) * 0.1, torch.randn(Nn, K, device=DEV).to(dtype) * 0.1
+    for off in (0, 3):
+        c = torch.randn(M, Nn + 8, device=DEV).to(dtype)[:, off: off + Nn]
+        ref = x.double() @ w.double().t() + c.double()
+        ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        for mode in (0, 1, 2):
+            old = G.set_pair_mode(mode)
+            try:
+                y = G.gemm(x, w, c=c, beta=1.0)
+                NV.check_status()
+            finally:
+                G.set_pair_mode(old)
+            assert (y.double() - ref).abs().max() <= ulp * ref.abs().max(), (off, mode)
+
+
+@pytest.mark.parametrize("n,dtype", [(1, torch.bfloat16), (8, torch.float16), (100003, torch.bfloat16)])
+def test_scale_cast_rounds_once(n, dtype):
+    from fms_acceleration_b200.ops.cross_entropy import _scaled_cast
+
+    src, factor = torch.randn(n, device=DEV), torch.tensor(0.37, device=DEV)
+    assert torch.equal(_scaled_cast(src, factor, dtype), (src * factor).to(dtype))
+    assert torch.equal(_scaled_cast(torch.randn(n + 1, device=DEV)[1:].copy_(src), factor, dtype), (src * factor).to(dtype))
