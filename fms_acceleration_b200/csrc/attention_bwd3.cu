@@ -20,15 +20,18 @@
 //
 // Tensor memory (512 columns): dK/dV: S^T 128 | dP^T 128 | dV D | dK D.   dQ: S 128 | dP 2 x 128 | dQ D.
 // P is kept as packed 16-bit between the stages (it is the operand of dV in that precision anyway).
-// T = 16384 packed, 32/8 heads, d = 128: dQ 919 -> 874 us, dK/dV 1050 -> 886 us (heads fastest in the grids, fp32 pairs);
-// T = 1500, d = 64: dQ 29.4 -> 22.9 us.
-// Warp roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute; a compute warp owns lane
-// quarter `warp % 4` and 64 of the 128 columns.  Every wait is bounded.
+// T = 16384 packed, 32/8 heads, d = 128: dQ 919 -> 874 us, dK/dV 1050 -> 886 us (heads fastest in the grids, fp32 pairs),
+// then 842 and 884 us with sixteen compute warps instead of eight;
+// T = 1500, d = 64: dQ 29.4 -> 21.2 us.
+// Warp roles (576 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-17 compute; a compute warp owns lane
+// quarter `warp % 4` and 32 of the 128 columns.  Every wait is bounded.
 #include "common.cuh"
 
 namespace fmsb {
 
 constexpr int B3_T = 128;  // tile edge (queries and keys)
+constexpr int B3_CW = 16;   // compute warps: four per scheduler, 32 of the 128 columns each (eight of 64 left latency exposed)
+constexpr int B3_THREADS = 64 + 32 * B3_CW;
 
 struct AttnBwd3Params {
   int T, nh, nkv, d;
@@ -68,9 +71,10 @@ __device__ __forceinline__ void b3_unpack2(uint32_t w, int fmt, float& a, float&
     b = f.y;
   }
 }
-__device__ __forceinline__ void b3_store_row_chunk(uint16_t* dst, const uint32_t (&r)[32], float mul, int fmt) {
+template <int NC>
+__device__ __forceinline__ void b3_store_row_chunk(uint16_t* dst, const uint32_t (&r)[NC], float mul, int fmt) {
 #pragma unroll
-  for (int i = 0; i < 32; i += 8) {
+  for (int i = 0; i < NC; i += 8) {
     uint4 u;
     u.x = b3_pack2(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul, fmt);
     u.y = b3_pack2(__uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul, fmt);
@@ -88,17 +92,33 @@ __device__ long long g_trace3[8192];
 #define FMSB_TRACE3(cond, slot) do { } while (0)
 #endif
 
-__device__ __forceinline__ void b3_compute_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void b3_compute_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
-// Column of K-step `ks` (16 elements = 8 packed columns) of a packed 128-element row: the warp of columns 0-63
-// packs into columns 0-31, the warp of columns 64-127 into columns 64-95 (each overwrites only what it has read).
-__device__ __forceinline__ uint32_t b3_pcol(int ks) { return static_cast<uint32_t>((ks >> 2) * 64 + (ks & 3) * 8); }
+// Column of K-step `ks` (16 elements = 8 packed columns) of a packed 128-element row: the warp of columns 32 q .. 32 q + 31
+// packs into columns 32 q .. 32 q + 15 (each overwrites only what it has read).
+__device__ __forceinline__ uint32_t b3_pcol(int ks) { return static_cast<uint32_t>((ks >> 1) * 32 + (ks & 1) * 8); }
+
+// This warp's quarter of an accumulator row (D / 4 columns from `col`), multiplied, to global memory.
+template <int D, int FMT>
+__device__ __forceinline__ void b3_store_quarter(uint16_t* dst, uint32_t taddr, float mul, bool on) {
+  if constexpr (D == 128) {
+    uint32_t r[32];
+    tmem_ld_32x32(taddr, r);
+    tmem_ld_wait();
+    if (on) b3_store_row_chunk(dst, r, mul, FMT);
+  } else {
+    uint32_t r[16];
+    tmem_ld_32x16(taddr, r);
+    tmem_ld_wait();
+    if (on) b3_store_row_chunk(dst, r, mul, FMT);
+  }
+}
 
 // ----------------------------------------------------------------------------------------
 // dV[kv tile, kv head] = sum P^T dO ,  dK = scale * sum dS^T Q
 // ----------------------------------------------------------------------------------------
 template <int D, int FMT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(B3_THREADS, 1)
 attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                      const AttnBwd3Params p) {
@@ -141,8 +161,8 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     mbar_init(bar_s_full, 1);
     mbar_init(bar_dp_full, 1);
-    mbar_init(bar_pa_full, 8);
-    mbar_init(bar_pb_full, 8);
+    mbar_init(bar_pa_full, B3_CW);
+    mbar_init(bar_pb_full, B3_CW);
     mbar_init(bar_acc_done, 1);
     fence_barrier_init();
   }
@@ -235,7 +255,7 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
   } else {
     const int quarter = warp & 3;
-    const int chalf = (warp - 2) >> 2;  // columns [64*chalf, 64*chalf + 64)
+    const int cq = (warp - 2) >> 2;  // columns [32 cq, 32 cq + 32)
     const int ctid = threadIdx.x - 64;
     const int kr = k0 + quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
@@ -248,23 +268,23 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (ctid < 128) {
         f = t < p.T ? p.lse[(long long)head * p.T + t] * LOG2E : 0.f;
         i = t < p.T ? p.doc_start[t] : 0x7fffffff;
-      } else {
+      } else if (ctid < 256) {
         f = t < p.T ? p.delta[(long long)head * p.T + t] : 0.f;
         i = 0;
       }
     };
     auto publish = [&](int buf, float f, int i) {
       float* b = scal_f + buf * 384;
-      b[ctid] = -f;  // [0,128): -lse*log2e, [128,256): -delta
+      if (ctid < 256) b[ctid] = -f;  // [0,128): -lse*log2e, [128,256): -delta
       if (ctid < 128) reinterpret_cast<int*>(b)[256 + ctid] = i;
     };
-    float nf;
-    int ni;
+    float nf = 0.f;
+    int ni = 0;
     fetch(0, nf, ni);
     publish(0, nf, ni);
     b3_compute_sync();
     bool ok = true;
-    const int c0 = chalf * 64;
+    const int c0 = cq * 32;
     for (int it = 0; it < niter; ++it) {
       const bool more = it + 1 < niter;
       if (more) fetch(it + 1, nf, ni);
@@ -272,19 +292,18 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int* bi = reinterpret_cast<const int*>(b) + 256;
       const int q0 = (qb_lo + it % nq) * B3_T;
       const bool need_mask = !(q0 >= k0 + B3_T - 1 && bi[127] <= k0);
-      uint32_t pk[32];
+      uint32_t pk[16];
       // ---- stage A: P^T from S^T
       if (ok && !mbar_wait(bar_s_full, it & 1, p.status, kTimeoutEpilogue)) ok = false;
       if (ok) {
         tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        {
           uint32_t rs[32];
-          tmem_ld_32x32(tS + lane_addr + c0 + c * 32, rs);
+          tmem_ld_32x32(tS + lane_addr + c0, rs);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            const int col = c0 + c * 32 + i;
+            const int col = c0 + i;
             const float4 l4 = *reinterpret_cast<const float4*>(b + col);
             float pv[4];
             unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), sl2x2, pack_f32x2(l4.x, l4.y)), pv[0], pv[1]);
@@ -299,11 +318,11 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
               if (!(kr >= s4.z && kr <= t + 2)) pv[2] = 0.f;
               if (!(kr >= s4.w && kr <= t + 3)) pv[3] = 0.f;
             }
-            pk[c * 16 + i / 2] = b3_pack2(pv[0], pv[1], FMT);
-            pk[c * 16 + i / 2 + 1] = b3_pack2(pv[2], pv[3], FMT);
+            pk[i / 2] = b3_pack2(pv[0], pv[1], FMT);
+            pk[i / 2 + 1] = b3_pack2(pv[2], pv[3], FMT);
           }
         }
-        tmem_st_32x32(tS + lane_addr + c0, pk);
+        tmem_st_32x16(tS + lane_addr + c0, pk);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -313,25 +332,24 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (ok && !mbar_wait(bar_dp_full, it & 1, p.status, kTimeoutEpilogue)) ok = false;
       if (ok) {
         tc_fence_after();
-        uint32_t dk[32];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        uint32_t dk[16];
+        {
           uint32_t rp[32];
-          tmem_ld_32x32(tdP + lane_addr + c0 + c * 32, rp);
+          tmem_ld_32x32(tdP + lane_addr + c0, rp);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            const float4 d4 = *reinterpret_cast<const float4*>(b + 128 + c0 + c * 32 + i);
+            const float4 d4 = *reinterpret_cast<const float4*>(b + 128 + c0 + i);
             float p0, p1, p2, p3;
-            b3_unpack2(pk[c * 16 + i / 2], FMT, p0, p1);
-            b3_unpack2(pk[c * 16 + i / 2 + 1], FMT, p2, p3);
+            b3_unpack2(pk[i / 2], FMT, p0, p1);
+            b3_unpack2(pk[i / 2 + 1], FMT, p2, p3);
             unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), add_f32x2(pack_f32x2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), pack_f32x2(d4.x, d4.y))), p0, p1);
             unpack_f32x2(mul_f32x2(pack_f32x2(p2, p3), add_f32x2(pack_f32x2(__uint_as_float(rp[i + 2]), __uint_as_float(rp[i + 3])), pack_f32x2(d4.z, d4.w))), p2, p3);
-            dk[c * 16 + i / 2] = b3_pack2(p0, p1, FMT);
-            dk[c * 16 + i / 2 + 1] = b3_pack2(p2, p3, FMT);
+            dk[i / 2] = b3_pack2(p0, p1, FMT);
+            dk[i / 2 + 1] = b3_pack2(p2, p3, FMT);
           }
         }
-        tmem_st_32x32(tdP + lane_addr + c0, dk);
+        tmem_st_32x16(tdP + lane_addr + c0, dk);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -342,20 +360,12 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     if (ok && mbar_wait(bar_acc_done, 0, p.status, kTimeoutEpilogue)) {
       tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        const int col = chalf * (D / 2) + c * 32;
-        uint32_t r[32];
-        tmem_ld_32x32(tdV + lane_addr + col, r);
-        tmem_ld_wait();
-        if (kr < p.T)
-          b3_store_row_chunk(reinterpret_cast<uint16_t*>(p.dv) + (long long)kr * p.lddv + hk * D + col, r, 1.f, FMT);
-        tmem_ld_32x32(tdK + lane_addr + col, r);
-        tmem_ld_wait();
-        if (kr < p.T)
-          b3_store_row_chunk(reinterpret_cast<uint16_t*>(p.dk) + (long long)kr * p.lddk + hk * D + col, r, p.scale,
-                             FMT);
-      }
+      const int col = cq * (D / 4);
+      const bool on = kr < p.T;
+      b3_store_quarter<D, FMT>(reinterpret_cast<uint16_t*>(p.dv) + (long long)kr * p.lddv + hk * D + col, tdV + lane_addr + col,
+                               1.f, on);
+      b3_store_quarter<D, FMT>(reinterpret_cast<uint16_t*>(p.dk) + (long long)kr * p.lddk + hk * D + col, tdK + lane_addr + col,
+                               p.scale, on);
     }
   }
   __syncwarp();
@@ -371,7 +381,7 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // dQ[q tile, head] = scale * sum_j dS_j K_j
 // ----------------------------------------------------------------------------------------
 template <int D, int FMT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(B3_THREADS, 1)
 attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                     const AttnBwd3Params p) {
@@ -412,10 +422,10 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(bar_v_full(s), 1);
       mbar_init(bar_v_empty(s), 1);
       mbar_init(bar_dp_full(s), 1);
-      mbar_init(bar_pb_full(s), 8);
+      mbar_init(bar_pb_full(s), B3_CW);
     }
     mbar_init(bar_s_full, 1);
-    mbar_init(bar_sa_done, 8);
+    mbar_init(bar_sa_done, B3_CW);
     mbar_init(bar_acc_done, 1);
     fence_barrier_init();
   }
@@ -510,7 +520,7 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else {
     const int quarter = warp & 3;
-    const int chalf = (warp - 2) >> 2;
+    const int cq = (warp - 2) >> 2;  // columns [32 cq, 32 cq + 32)
     const int row = quarter * 32 + lane;
     const int t = q0 + row;
     const bool row_ok = t < p.T;
@@ -521,7 +531,7 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float lse2 = row_ok ? p.lse[(long long)head * p.T + t] * LOG2E : 0.f;
     const float dlt = row_ok ? p.delta[(long long)head * p.T + t] : 0.f;
     const uint64_t sl2x2 = pack_f32x2(sl2, sl2), nlse2 = pack_f32x2(-lse2, -lse2), ndlt2 = pack_f32x2(-dlt, -dlt);
-    const int c0 = chalf * 64;
+    const int c0 = cq * 32;
     const bool trc = blockIdx.y == gridDim.y / 2 && blockIdx.x == 0 && threadIdx.x == 64;
     bool ok = true;
     FMSB_TRACE3(trc, 12);
@@ -532,55 +542,47 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!mbar_wait(bar_s_full, j & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
       tc_fence_after();
       FMSB_TRACE3(trc, 64 + 8 * j + 1);
-      uint32_t pk[32];
+      uint32_t pk[16];
       {
-        uint32_t rs0[32], rs1[32];
-        tmem_ld_32x32(tS + lane_addr + c0, rs0);
-        tmem_ld_32x32(tS + lane_addr + c0 + 32, rs1);
+        uint32_t rs[32];
+        tmem_ld_32x32(tS + lane_addr + c0, rs);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_sa_done);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0, p1, p2, p3;
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs0[i]), __uint_as_float(rs0[i + 1])), sl2x2, nlse2), p0, p1);
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs1[i]), __uint_as_float(rs1[i + 1])), sl2x2, nlse2), p2, p3);
+          float p0, p1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), sl2x2, nlse2), p0, p1);
           p0 = fast_exp2(p0);
           p1 = fast_exp2(p1);
-          p2 = fast_exp2(p2);
-          p3 = fast_exp2(p3);
           if (need_mask) {
             const int kk = k0 + c0 + i;
             if (!(row_ok && kk >= ds && kk <= t)) p0 = 0.f;
             if (!(row_ok && kk + 1 >= ds && kk + 1 <= t)) p1 = 0.f;
-            if (!(row_ok && kk + 32 >= ds && kk + 32 <= t)) p2 = 0.f;
-            if (!(row_ok && kk + 33 >= ds && kk + 33 <= t)) p3 = 0.f;
           }
           pk[i / 2] = b3_pack2(p0, p1, FMT);
-          pk[16 + i / 2] = b3_pack2(p2, p3, FMT);
         }
       }
       FMSB_TRACE3(trc, 64 + 8 * j + 2);
       if (!mbar_wait(bar_dp_full(j & 1), (j >> 1) & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
       tc_fence_after();
       FMSB_TRACE3(trc, 64 + 8 * j + 3);
-      uint32_t dk[32];
+      uint32_t dk[16];
       const uint32_t tdp = tdP(j & 1) + lane_addr + c0;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      {
         uint32_t rp[32];
-        tmem_ld_32x32(tdp + c * 32, rp);
+        tmem_ld_32x32(tdp, rp);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float p0, p1;
-          b3_unpack2(pk[c * 16 + i / 2], FMT, p0, p1);
+          b3_unpack2(pk[i / 2], FMT, p0, p1);
           unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), add_f32x2(pack_f32x2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), ndlt2)), p0, p1);
-          dk[c * 16 + i / 2] = b3_pack2(p0, p1, FMT);
+          dk[i / 2] = b3_pack2(p0, p1, FMT);
         }
       }
-      tmem_st_32x32(tdp, dk);
+      tmem_st_32x16(tdp, dk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -591,16 +593,9 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (ok && mbar_wait(bar_acc_done, 0, p.status, kTimeoutEpilogue)) {
       tc_fence_after();
       FMSB_TRACE3(trc, 14);
-#pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        const int col = chalf * (D / 2) + c * 32;
-        uint32_t r[32];
-        tmem_ld_32x32(tdQ + lane_addr + col, r);
-        tmem_ld_wait();
-        if (row_ok)
-          b3_store_row_chunk(reinterpret_cast<uint16_t*>(p.dq) + (long long)t * p.lddq + head * D + col, r, p.scale,
-                             FMT);
-      }
+      const int col = cq * (D / 4);
+      b3_store_quarter<D, FMT>(reinterpret_cast<uint16_t*>(p.dq) + (long long)t * p.lddq + head * D + col,
+                               tdQ + lane_addr + col, p.scale, row_ok);
     }
   }
   __syncwarp();
@@ -663,7 +658,7 @@ extern "C" int fmsb_attn_bwd_dq3(const void* q, long long ldq, const void* k, lo
       if ((rc = b3_set_smem(attn_bwd_dq3_kernel<DD, FF>, AttnBwd3Cfg<DD>::kSmemBytes))) return rc;             \
       cfg = true;                                                                                                \
     }                                                                                                            \
-    attn_bwd_dq3_kernel<DD, FF><<<grid, 320, AttnBwd3Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);       \
+    attn_bwd_dq3_kernel<DD, FF><<<grid, B3_THREADS, AttnBwd3Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);       \
   } while (0)
   if (d == 128 && fmt == 1) FMSB_B3(128, 1);
   else if (d == 128) FMSB_B3(128, 0);
@@ -696,7 +691,7 @@ extern "C" int fmsb_attn_bwd_dkv3(const void* q, long long ldq, const void* k, l
       if ((rc = b3_set_smem(attn_bwd_dkv3_kernel<DD, FF>, AttnBwd3Cfg<DD>::kSmemBytes))) return rc;             \
       cfg = true;                                                                                                \
     }                                                                                                            \
-    attn_bwd_dkv3_kernel<DD, FF><<<grid, 320, AttnBwd3Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);       \
+    attn_bwd_dkv3_kernel<DD, FF><<<grid, B3_THREADS, AttnBwd3Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, tdo, p);       \
   } while (0)
   if (d == 128 && fmt == 1) FMSB_B3(128, 1);
   else if (d == 128) FMSB_B3(128, 0);
