@@ -700,3 +700,21 @@ extern "C" int fmsb_attn_bwd_dkv3(const void* q, long long ldq, const void* k, l
 #undef FMSB_B3
   return (int)cudaGetLastError();
 }
+
+extern "C" int fmsb_attn_delta(const void* o, const void* dout, long long ldo, long long lddo, float* delta, int T, int nh, int d,
+                               int fmt, cudaStream_t stream);
+
+// The whole backward (delta, dQ, dK/dV) in one call: three launches from Python cost the host more than the kernels take at
+// 1500 tokens.  delta: scratch of nh * T floats.
+extern "C" int fmsb_attn_bwd(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
+                             const void* o, long long ldo, const void* dout, long long lddo, void* dq, long long lddq,
+                             void* dk, long long lddk, void* dv, long long lddv, const float* lse, float* delta,
+                             const int* doc_start, const int* doc_end, int T, int nh, int nkv, int d, float scale, int fmt,
+                             int* status, cudaStream_t stream) {
+  int rc;
+  if ((rc = fmsb_attn_delta(o, dout, ldo, lddo, delta, T, nh, d, fmt, stream))) return rc;
+  if ((rc = fmsb_attn_bwd_dq3(q, ldq, k, ldk, v, ldv, dout, lddo, dq, lddq, lse, delta, doc_start, doc_end, T, nh, nkv, d, scale,
+                              fmt, status, stream))) return rc;
+  return fmsb_attn_bwd_dkv3(q, ldq, k, ldk, v, ldv, dout, lddo, dk, lddk, dv, lddv, lse, delta, doc_start, doc_end, T, nh, nkv,
+                            d, scale, fmt, status, stream);
+}

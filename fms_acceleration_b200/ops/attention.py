@@ -7,6 +7,7 @@ structure is handed to the kernels as per-token ``doc_start`` / ``doc_end`` arra
 """
 from __future__ import annotations
 
+import ctypes
 import math
 import os
 
@@ -35,6 +36,26 @@ def cu_seqlens_from_position_ids(position_ids: torch.Tensor) -> torch.Tensor:
     return torch.cat([starts, end]).to(torch.int32)
 
 
+N.declare("fmsb_doc_bounds", [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
+                              ctypes.c_void_p])
+
+
+def doc_bounds_from_position_ids(position_ids: torch.Tensor):
+    """(positions, doc_start, doc_end), int32 ``[T]`` each, of a flattened batch: a new document starts wherever the
+    position is 0.  One launch on a GPU, no host synchronisation."""
+    flat = position_ids.reshape(-1)
+    T = flat.numel()
+    if not flat.is_cuda or flat.dtype not in (torch.int64, torch.int32) or T >= 1 << 31 or T == 0:
+        ds, de = doc_bounds_from_cu_seqlens(cu_seqlens_from_position_ids(flat), T)
+        return flat.to(torch.int32).contiguous(), ds, de
+    flat = flat.contiguous()
+    pos, ds, de = torch.empty(3, T, dtype=torch.int32, device=flat.device).unbind(0)
+    rc = N.lib().fmsb_doc_bounds(flat.data_ptr(), int(flat.dtype == torch.int64), pos.data_ptr(), ds.data_ptr(),
+                                 de.data_ptr(), T, N.stream_ptr())
+    N.check(rc, "fmsb_doc_bounds")
+    return pos, ds, de
+
+
 def attention_ref(q, k, v, doc_start, scale=None):
     """fp32 oracle.  q [T, nh, d], k/v [T, nkv, d]."""
     T, nh, d = q.shape
@@ -58,6 +79,10 @@ def attention_ref(q, k, v, doc_start, scale=None):
 DETERMINISTIC_BACKWARD = True
 
 
+_P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+N.declare("fmsb_attn_bwd", [_P, _L] * 8 + [_P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P])
+
+
 def _fwd(q2, k2, v2, doc_start, doc_end, nh, nkv, d, scale):
     T = q2.shape[0]
     o = torch.empty(T, nh * d, dtype=q2.dtype, device=q2.device)
@@ -74,10 +99,6 @@ def _bwd(q2, k2, v2, o, lse, dout, doc_start, doc_end, nh, nkv, d, scale, dq=Non
     T = q2.shape[0]
     dev = q2.device
     delta = torch.empty(nh, T, dtype=torch.float32, device=dev)
-    fmt = N.dtype_code(q2.dtype)
-    rc = N.lib().fmsb_attn_delta(o.data_ptr(), dout.data_ptr(), o.stride(0), dout.stride(0), delta.data_ptr(), T, nh,
-                                 d, fmt, N.stream_ptr())
-    N.check(rc, "fmsb_attn_delta")
     if dq is None:
         dq = torch.empty(T, nh * d, dtype=q2.dtype, device=dev)
     if dk is None:
@@ -85,18 +106,12 @@ def _bwd(q2, k2, v2, o, lse, dout, doc_start, doc_end, nh, nkv, d, scale, dq=Non
     if dv is None:
         dv = torch.empty(T, nkv * d, dtype=q2.dtype, device=dev)
     st = N.status_word(dev)
-    dq_fn, dkv_fn = N.lib().fmsb_attn_bwd_dq3, N.lib().fmsb_attn_bwd_dkv3
-    rc = dq_fn(q2.data_ptr(), q2.stride(0), k2.data_ptr(), k2.stride(0), v2.data_ptr(),
-                                  v2.stride(0), dout.data_ptr(), dout.stride(0), dq.data_ptr(), dq.stride(0),
-                                  lse.data_ptr(), delta.data_ptr(), doc_start.data_ptr(), doc_end.data_ptr(), T, nh,
-                                  nkv, d, float(scale), fmt, st.data_ptr(), N.stream_ptr())
-    N.check(rc, "fmsb_attn_bwd_dq")
-    rc = dkv_fn(q2.data_ptr(), q2.stride(0), k2.data_ptr(), k2.stride(0), v2.data_ptr(),
-                v2.stride(0), dout.data_ptr(), dout.stride(0), dk.data_ptr(), dk.stride(0),
-                dv.data_ptr(), dv.stride(0), lse.data_ptr(), delta.data_ptr(), doc_start.data_ptr(),
-                doc_end.data_ptr(), T, nh, nkv, d, float(scale), fmt, st.data_ptr(),
-                N.stream_ptr())
-    N.check(rc, "fmsb_attn_bwd_dkv")
+    rc = N.lib().fmsb_attn_bwd(q2.data_ptr(), q2.stride(0), k2.data_ptr(), k2.stride(0), v2.data_ptr(), v2.stride(0),
+                               o.data_ptr(), o.stride(0), dout.data_ptr(), dout.stride(0), dq.data_ptr(), dq.stride(0),
+                               dk.data_ptr(), dk.stride(0), dv.data_ptr(), dv.stride(0), lse.data_ptr(), delta.data_ptr(),
+                               doc_start.data_ptr(), doc_end.data_ptr(), T, nh, nkv, d, float(scale),
+                               N.dtype_code(q2.dtype), st.data_ptr(), N.stream_ptr())
+    N.check(rc, "fmsb_attn_bwd")
     return dq, dk, dv
 
 

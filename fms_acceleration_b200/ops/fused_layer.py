@@ -38,10 +38,8 @@ class PackedBatch:
 
     @classmethod
     def from_position_ids(cls, position_ids: torch.Tensor, cos, sin) -> "PackedBatch":
-        flat = position_ids.reshape(-1)
-        cu = ATT.cu_seqlens_from_position_ids(flat)
-        ds, de = ATT.doc_bounds_from_cu_seqlens(cu, flat.numel())
-        return cls(flat.to(torch.int32).contiguous(), ds, de, cos, sin)
+        pos, ds, de = ATT.doc_bounds_from_position_ids(position_ids)
+        return cls(pos, ds, de, cos, sin)
 
     @classmethod
     def from_cu_seqlens(cls, cu_seqlens: torch.Tensor, total: int, cos, sin) -> "PackedBatch":

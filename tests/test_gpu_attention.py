@@ -140,3 +140,16 @@ def test_backward_is_bitwise_reproducible():
         grads.append((o.detach().clone(), q.grad.clone(), k.grad.clone(), v.grad.clone()))
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("lens,lead", [([1], 0), ([1023, 1, 1025, 7], 0), ([5000, 3, 2], 0), ([1, 1, 1, 1], 0), ([2048, 2048], 0),
+                                       ([100, 3000], 5), ([1500], 2100), ([], 1030)])
+def test_doc_bounds_from_position_ids_equal_the_host_form(lens, lead, dtype):
+    """Documents across and inside the 1024-token tiles; ``lead`` tokens before the first position 0 (or no 0 at all)."""
+    pos = torch.cat([torch.arange(7, 7 + lead)] + [torch.arange(n) for n in lens]).to(dtype)
+    got = AT.doc_bounds_from_position_ids(pos.to(DEV))
+    cu = AT.cu_seqlens_from_position_ids(pos)
+    ds, de = AT.doc_bounds_from_cu_seqlens(cu, pos.numel())
+    assert torch.equal(got[0].cpu(), pos.to(torch.int32))
+    assert torch.equal(got[1].cpu(), ds) and torch.equal(got[2].cpu(), de)
