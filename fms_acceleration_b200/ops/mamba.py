@@ -37,6 +37,9 @@ NV.declare("fmsb_ssdf_scan", [I_, P_, L_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_
 NV.declare("fmsb_ssdf_state", [P_, L_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, P_, P_])
 NV.declare("fmsb_ssdf_dcb", [P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, P_, P_])
 NV.declare("fmsb_ssdf_sum", [P_, P_, P_, I_, L_, I_, P_])
+NV.declare("fmsb_ssdf_workspace", [I_, I_, I_, I_])
+NV.declare("fmsb_ssdf_forward", [P_, P_, P_, P_, L_, P_, L_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, P_, P_])
+NV.declare("fmsb_ssdf_backward", [P_, P_, P_, P_, P_, L_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, P_, P_])
 NV.declare("fmsb_ssdf_decay", [P_, P_, P_, P_, P_, I_, I_, P_])
 NV.declare("fmsb_ssdf_decay_bwd", [P_, P_, P_, P_, P_, P_, P_, I_, I_, P_])
 
@@ -502,6 +505,28 @@ class _Fused:
         NV.check(rc, "fmsb_ssd_state_fwd")
 
 
+@functools.lru_cache(maxsize=256)
+def _fused_workspace(backward, nc, nh, G):
+    fn = NV.lib()._handle.fmsb_ssdf_workspace
+    fn.restype = ctypes.c_longlong
+    return max(1, fn(backward, nc, nh, G))
+
+
+def _fused_forward(x2, dt, A32, B2, C2, D32, h0, y, nh, G):
+    """(hprev, hT), and ``y`` unless it is None; all launches of the forward in one native call."""
+    nc, dev = x2.shape[0] // 256, x2.device
+    hprev = torch.empty(nc * nh * 64, 128, dtype=x2.dtype, device=dev)
+    hT = torch.empty(nh, 64, 128, dtype=torch.float32, device=dev)
+    h0 = None if h0 is None else h0.float().contiguous()
+    ws = torch.empty(_fused_workspace(0, nc, nh, G), dtype=torch.uint8, device=dev)
+    rc = NV.lib().fmsb_ssdf_forward(x2.data_ptr(), dt.data_ptr(), A32.data_ptr(), B2.data_ptr(), B2.stride(0), C2.data_ptr(),
+                                    C2.stride(0), NV.ptr(D32), NV.ptr(h0), NV.ptr(y), hT.data_ptr(), hprev.data_ptr(),
+                                    ws.data_ptr(), nc, nh, G, NV.dtype_code(x2.dtype), NV.status_word(dev).data_ptr(),
+                                    NV.stream_ptr())
+    NV.check(rc, "fmsb_ssdf_forward")
+    return hprev, hT
+
+
 class _SSDScanFused(torch.autograd.Function):
     """:class:`_SSDScan` for the shapes of :func:`_fused_ok`: same arguments, same results."""
 
@@ -512,12 +537,15 @@ class _SSDScanFused(torch.autograd.Function):
         x2 = _rows16(x.reshape(T, nh * P))
         B2, C2 = _vec_rows(B.reshape(T, G * N)), _vec_rows(C.reshape(T, G * N))
         dt = dt.float().contiguous()
-        k = _Fused(x2, dt, A.float().contiguous(), B2, C2, T, nh, G, Q)
+        A32, D32 = A.float().contiguous(), D.float().contiguous()
+        y = torch.empty(T, nh, P, dtype=x.dtype, device=x.device)
         if cp is not None:
             assert h0 is None, "the entering state of a context-parallel slice comes from the earlier ranks"
-        hprev, hT, h_in, hprev0 = k.states(h0, cp)
-        y = torch.empty(T, nh, P, dtype=x.dtype, device=x.device)
-        k.scan(0, C2, B2, x2, hprev, out=y, D=D.float().contiguous())
+            k = _Fused(x2, dt, A32, B2, C2, T, nh, G, Q)
+            hprev, hT, h_in, hprev0 = k.states(h0, cp)
+            k.scan(0, C2, B2, x2, hprev, out=y, D=D32)
+        else:
+            hprev, hT = _fused_forward(x2, dt, A32, B2, C2, D32, h0, y, nh, G)
         if recompute:
             ctx.save_for_backward(x, dt, A, B, C, D, h_in if cp is not None else h0)
         elif cp is not None:
@@ -539,60 +567,65 @@ class _SSDScanFused(torch.autograd.Function):
         x2 = _rows16(x.reshape(T, nh * P))
         B2, C2 = _vec_rows(B.reshape(T, G * N)), _vec_rows(C.reshape(T, G * N))
         dy2 = _rows16(dy.reshape(T, nh * P))
-        A32 = A.float().contiguous()
+        A32, D32 = A.float().contiguous(), D.float().contiguous()
+        dhTc = None if dhT is None else dhT.float().contiguous()
+        dx = torch.empty(T, nh, P, dtype=dtp, device=dev)
+        ddt = torch.empty(T, nh, dtype=torch.float32, device=dev)
+        sums = torch.empty(2, nc, nh, dtype=torch.float32, device=dev)
+        if cp is None:
+            hprev = saved[6] if not recompute else _fused_forward(x2, dt, A32, B2, C2, None, saved[6], None, nh, G)[0]
+            dB, dC = torch.empty(T, G, N, dtype=dtp, device=dev), torch.empty(T, G, N, dtype=dtp, device=dev)
+            dh0 = torch.empty(nh, P, N, dtype=torch.float32, device=dev) if has_h0 else None
+            ws = torch.empty(_fused_workspace(1, nc, nh, G), dtype=torch.uint8, device=dev)
+            rc = NV.lib().fmsb_ssdf_backward(x2.data_ptr(), dy2.data_ptr(), dt.data_ptr(), A32.data_ptr(), B2.data_ptr(),
+                                             B2.stride(0), C2.data_ptr(), C2.stride(0), D32.data_ptr(), hprev.data_ptr(),
+                                             NV.ptr(dhTc), dx.data_ptr(), ddt.data_ptr(), dB.data_ptr(), dC.data_ptr(),
+                                             sums.data_ptr(), NV.ptr(dh0), ws.data_ptr(), nc, nh, G, NV.dtype_code(dtp),
+                                             NV.status_word(dev).data_ptr(), NV.stream_ptr())
+            NV.check(rc, "fmsb_ssdf_backward")
+            dA, dD = sums.sum(1)
+            return (dx, ddt, dA.to(A.dtype), dB, dC, dD.to(D.dtype), dh0, None, None, None)
+        # context parallelism: the same launches around the exchange
         k = _Fused(x2, dt, A32, B2, C2, T, nh, G, Q)
-        hprev0 = None
         if recompute:
-            hprev, _, _, hprev0 = k.states(saved[6], want_zero_start=cp is not None)
-        elif cp is not None:
-            hprev, hprev0 = saved[6:]
+            hprev, _, _, hprev0 = k.states(saved[6], want_zero_start=True)
         else:
-            hprev = saved[6]
+            hprev, hprev0 = saved[6:]
         # dy . (G x + exp(L) C Hprev^T) per (chunk, head, position): the decay's share of the gradient
         ydot = torch.empty(nc, nh, Q, dtype=torch.float32, device=dev)
         k.scan(1, C2, B2, x2, hprev, e=dy2, red=ydot)
         # gradient of the entering states and, through them, of C
         dhp, dC_part = k.state(C2, dy2, 1, h=hprev)
         # ---- recurrence backward
-        dS16 = torch.empty(nc * nh * P, N, dtype=dtp, device=dev)
-        dh0 = torch.empty(nh, P, N, dtype=torch.float32, device=dev) if (has_h0 or cp is not None) else None
+        dS16, dS16b = torch.empty(2, nc * nh * P, N, dtype=dtp, device=dev).unbind(0)
+        dh0 = torch.empty(nh, P, N, dtype=torch.float32, device=dev)
         dLtot = torch.zeros(nc, nh, dtype=torch.float32, device=dev)
-        dhTc = None if dhT is None else dhT.float().contiguous()
         rc = NV.lib().fmsb_ssd_state_bwd(dhp.data_ptr(), NV.ptr(dhTc), k.Ltot.data_ptr(), hprev.data_ptr(),
-                                         dS16.data_ptr(), NV.ptr(dh0), dLtot.data_ptr(), nc, nh, P * N, k.code,
+                                         dS16.data_ptr(), dh0.data_ptr(), dLtot.data_ptr(), nc, nh, P * N, k.code,
                                          NV.stream_ptr())
         NV.check(rc, "fmsb_ssd_state_bwd")
         del dhp
-        if cp is not None:  # as in _SSDScan.backward
-            dF, dlogP = cp.backward(dh0, nh, P * N)
-            dS16b = torch.empty_like(dS16)
-            rc = NV.lib().fmsb_ssd_state_bwd(None, dF.data_ptr(), k.Ltot.data_ptr(), hprev0.data_ptr(), dS16b.data_ptr(),
-                                             None, dLtot.data_ptr(), nc, nh, P * N, k.code, NV.stream_ptr())
-            NV.check(rc, "fmsb_ssd_state_bwd")
-            dS16 += dS16b
-            del dS16b
-            dLtot += dlogP[None, :]
-            dh0 = None
+        dF, dlogP = cp.backward(dh0, nh, P * N)  # as in _SSDScan.backward
+        rc = NV.lib().fmsb_ssd_state_bwd(None, dF.data_ptr(), k.Ltot.data_ptr(), hprev0.data_ptr(), dS16b.data_ptr(),
+                                         None, dLtot.data_ptr(), nc, nh, P * N, k.code, NV.stream_ptr())
+        NV.check(rc, "fmsb_ssd_state_bwd")
+        dS16 += dS16b
+        dLtot += dlogP[None, :]
         # ---- dx with its three row dot products, dB through the chunk states, dCB and what it gives to B and C
-        dx = torch.empty(T, nh, P, dtype=dtp, device=dev)
         red = torch.empty(3, nc, nh, Q, dtype=torch.float32, device=dev)
-        k.scan(2, B2, C2, dy2, dS16, e=x2, out=dx, D=D.float().contiguous(), red=red)
+        k.scan(2, B2, C2, dy2, dS16, e=x2, out=dx, D=D32, red=red)
         _, dB_part = k.state(B2, x2, 0, h=dS16, want_s=False)
-        del dS16
         dcb = k.dcb(dy2)
         geo = dict(M=Q, N=N, K=Q, n_batch=nc * G, n_inner=G, a_off=(G * Q, Q, 0, 1), b_off=(Q, 0, N, 1), d_off=(Q, 0, N),
                    b_mn=True, out_rows=T, out_cols=G * N, out_dtype=torch.float32)
         dC = k.total(dC_part, batched_gemm(dcb, B2, **geo))
         dB = k.total(dB_part, batched_gemm(dcb, C2, a_mn=True, **geo))
         # ---- through the decay
-        ddt = torch.empty(T, nh, dtype=torch.float32, device=dev)
-        sums = torch.empty(2, nc, nh, dtype=torch.float32, device=dev)
         rc = NV.lib().fmsb_ssdf_decay_bwd(ydot.data_ptr(), red.data_ptr(), k.dtt.data_ptr(), A32.data_ptr(),
                                           dLtot.data_ptr(), ddt.data_ptr(), sums.data_ptr(), nc, nh, NV.stream_ptr())
         NV.check(rc, "fmsb_ssdf_decay_bwd")
         dA, dD = sums.sum(1)
-        return (dx, ddt.to(dt.dtype), dA.to(A.dtype), dB.view(T, G, N), dC.view(T, G, N), dD.to(D.dtype), dh0, None, None,
-                None)
+        return (dx, ddt, dA.to(A.dtype), dB.view(T, G, N), dC.view(T, G, N), dD.to(D.dtype), None, None, None, None)
 
 
 class _StateCorrection(torch.autograd.Function):

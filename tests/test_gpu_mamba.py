@@ -135,6 +135,42 @@ def test_fused_scan_matches_recurrence_and_general_path(nc, nh, G, dtype, with_h
         assert err < 4 * ulp, (i, err, _rel(g.cpu(), r.cpu()))
 
 
+@pytest.mark.parametrize("recompute", [False, True])
+def test_fused_scan_with_an_exchange_around_it(recompute):
+    """The launch sequence of a context-parallel slice (states, exchange, scan; backward likewise) with an exchange that
+    hands in a fixed state and returns zero gradients: the same numbers as the one-call sequence from that state."""
+    torch.manual_seed(3)
+    nc, nh, G, P, N, Q = 3, 4, 2, 64, 128, 256
+    T = nc * Q
+    h_in = torch.randn(nh, P, N, device=DEV) * 0.2
+
+    class Exchange:
+        def forward(self, S, Ltot, hprev0, nc_, nh_, PN, dtype):
+            scratch = torch.empty(nh_, PN, device=DEV)
+            NV.check(NV.lib().fmsb_ssd_state_fwd(S.data_ptr(), Ltot.data_ptr(), None, hprev0.data_ptr(), scratch.data_ptr(),
+                                                 nc_, nh_, PN, NV.dtype_code(dtype), NV.stream_ptr()), "state_fwd")
+            return h_in
+
+        def backward(self, dh0, nh_, PN):
+            self.dh0 = dh0
+            return torch.zeros(nh_, PN, device=DEV), torch.zeros(nh_, device=DEV)
+
+    ins = [torch.randn(T, nh, P, device=DEV).bfloat16() * 0.5, torch.rand(T, nh, device=DEV) * 0.09 + 0.01,
+           -(torch.rand(nh, device=DEV) * 3 + 0.5), torch.randn(T, G, N, device=DEV).bfloat16() * 0.3,
+           torch.randn(T, G, N, device=DEV).bfloat16() * 0.3, torch.randn(nh, device=DEV)]
+    gy = torch.randn(T, nh, P, device=DEV).bfloat16()
+    t = [v.detach().requires_grad_() for v in ins] + [h_in.clone().requires_grad_()]
+    y, _ = MB._SSDScanFused.apply(*t, Q, False)
+    want = [y] + list(torch.autograd.grad(y, t, gy))
+    t2 = [v.detach().requires_grad_() for v in ins]
+    ex = Exchange()
+    y2, _ = MB._SSDScanFused.apply(*t2, None, Q, recompute, ex)
+    got = [y2] + list(torch.autograd.grad(y2, t2, gy)) + [ex.dh0]
+    NV.check_status()
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert _rel(a, b) < 1e-5, (i, _rel(a, b))
+
+
 @pytest.mark.parametrize("Q", [64, 256])
 def test_decay_matrix_kernel_with_moderate_and_extreme_decay(Q):
     """G[c, h, t, s] = CB[c, g, t, s] exp(L_t - L_s) dt_s for s <= t, 0 above the diagonal.  Heads with a moderate
