@@ -48,6 +48,8 @@ N.declare("fmsb_moe_zero_pad", [P, L, I, P, P, I, I, P])
 N.declare("fmsb_moe_combine", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_gate_grad", [P, L, P, P, P, L, L, I, I, I, P, I, I, P])
 N.declare("fmsb_moe_dispatch_meta", [P, L, P, P, P, L, I, I, I, P, L, P, I, I, P])
+N.declare("fmsb_moe_local_fwd", [P, L, P, P, L, I, I, I, I, P, P, P, I, P, P, P, P, I, P, P, P, P, P, P, P, I, I, P, P])
+N.declare("fmsb_moe_local_bwd", [P, L, P, P, P, P, P, P, P, P, L, I, I, I, I, P, P, P, I, I, P, P, P, P, P, P, P, P, P, I, I, P, P])
 N.declare("fmsb_moe_dispatch_dot", [P, L, P, P, L, I, I, P, L, P, L, P, I, P])
 N.declare("fmsb_moe_rowdot_scale", [P, L, P, L, P, P, P, I, I, I, I, P])
 N.declare("fmsb_moe_gather_scalar", [P, P, P, L, I, P, I, P])
@@ -467,6 +469,51 @@ def _weight_grads(mctx, acc, w1, w3, w2, needs):
     return dw1, dw3, dw2
 
 
+def _local_fwd(mctx, x, gates, idx, w1, w3, w2, act, cap):
+    """Forward of :class:`_Experts` without low-rank factors, all launches in one native call (``csrc/moe_local.cu``)."""
+    T, H = x.shape
+    E, k, I_ = mctx.E_local, mctx.k, mctx.I
+    dev, dt = x.device, x.dtype
+    ints = torch.empty(2 * E + 1 + 3 * E + max(1, -(-T * k // 1024)) * E, dtype=torch.int32, device=dev)
+    seg_off, seg_cnt, ws = ints.split([E + 1, E, ints.numel() - 2 * E - 1])
+    dest_row = torch.empty(T, k, dtype=torch.int32, device=dev)
+    Xs, Ys = torch.empty(cap, H, dtype=dt, device=dev), torch.empty(cap, H, dtype=dt, device=dev)
+    gu, hs = torch.empty(cap, 2 * I_, dtype=dt, device=dev), torch.empty(cap, I_, dtype=dt, device=dev)
+    out = torch.empty(T, H, dtype=dt, device=dev)
+    rc = N.lib().fmsb_moe_local_fwd(x.data_ptr(), x.stride(0), idx.data_ptr(), gates.data_ptr(), T, k, H, I_, E,
+                                    w1.view(E * H, I_).data_ptr(), w3.view(E * H, I_).data_ptr(),
+                                    w2.view(E * I_, H).data_ptr(), ACT.ACT_CODES[act], ws.data_ptr(), seg_off.data_ptr(),
+                                    seg_cnt.data_ptr(), dest_row.data_ptr(), cap, Xs.data_ptr(), gu.data_ptr(),
+                                    hs.data_ptr(), Ys.data_ptr(), out.data_ptr(), MoEContext.needed_counter(dev).data_ptr(),
+                                    _counter(_overflow, dev).data_ptr(), N.dtype_code(dt), mctx.gemm_ctas,
+                                    N.status_word(dev).data_ptr(), N.stream_ptr())
+    N.check(rc, "fmsb_moe_local_fwd")
+    return out, (seg_off, seg_cnt, dest_row, gu, Xs, Ys)
+
+
+def _local_bwd(mctx, dout, gates, idx, w1, w3, w2, act, seg_off, seg_cnt, dest_row, gu, Xs, Ys, need_dw):
+    """Backward of :func:`_local_fwd`: (dx, dgate, (dw1, dw3, dw2))."""
+    T, H = dout.shape
+    E, k, I_, cap = mctx.E_local, mctx.k, mctx.I, gu.shape[0]
+    dev, dt = dout.device, dout.dtype
+    dYs, dXs = torch.empty(cap, H, dtype=dt, device=dev), torch.empty(cap, H, dtype=dt, device=dev)
+    dhs = torch.empty(cap, I_, dtype=dt, device=dev)
+    hs = torch.empty(cap, I_, dtype=dt, device=dev) if need_dw else None
+    dgate = torch.empty(T, k, dtype=torch.float32, device=dev)
+    dx = torch.empty(T, H, dtype=dt, device=dev)
+    dws = tuple(torch.empty(w.shape, dtype=w.dtype, device=dev) for w in (w1, w3, w2)) if need_dw else (None,) * 3
+    gates_c = gates.contiguous()
+    rc = N.lib().fmsb_moe_local_bwd(dout.data_ptr(), dout.stride(0), idx.data_ptr(), gates_c.data_ptr(), seg_off.data_ptr(),
+                                    seg_cnt.data_ptr(), dest_row.data_ptr(), Xs.data_ptr(), gu.data_ptr(), Ys.data_ptr(), T, k,
+                                    H, I_, E, w1.view(E * H, I_).data_ptr(), w3.view(E * H, I_).data_ptr(),
+                                    w2.view(E * I_, H).data_ptr(), ACT.ACT_CODES[act], cap, dYs.data_ptr(), N.ptr(hs),
+                                    dhs.data_ptr(), dXs.data_ptr(), dgate.data_ptr(), dx.data_ptr(), N.ptr(dws[0]),
+                                    N.ptr(dws[1]), N.ptr(dws[2]), N.dtype_code(dt), mctx.gemm_ctas,
+                                    N.status_word(dev).data_ptr(), N.stream_ptr())
+    N.check(rc, "fmsb_moe_local_bwd")
+    return dx, dgate, dws
+
+
 class _Experts(torch.autograd.Function):
     """One rank owns every expert.  x [T,H], gates fp32 [T,k], idx int32 [T,k], w1/w3 [E,H,I], w2 [E,I,H] -> [T,H]."""
 
@@ -476,6 +523,11 @@ class _Experts(torch.autograd.Function):
         T, H = x.shape
         dev, dt = x.device, x.dtype
         cap = mctx.cap = _round_up(T * mctx.k + mctx.E_local * 128, 128)  # exact upper bound: never overflows
+        if lora is None:
+            out, saved = _local_fwd(mctx, x, gates, idx, w1, w3, w2, act, cap)
+            ctx.mctx, ctx.act, ctx.has_lora = mctx, act, False
+            ctx.save_for_backward(gates, idx, w1, w3, w2, *saved)
+            return out
         seg_off, seg_cnt, dest_row = _plan(mctx, idx, T, dev)
         Xs = torch.empty(cap, H, dtype=dt, device=dev)
         _zero_pad(mctx, Xs, seg_off, seg_cnt)
@@ -495,6 +547,10 @@ class _Experts(torch.autograd.Function):
         T, H = dout.shape
         El, cap = mctx.E_local, gu.shape[0]
         dev, dt = dout.device, dout.dtype
+        if lora is None:
+            dx, dgate, dws = _local_bwd(mctx, dout, gates, idx, w1, w3, w2, act, seg_off, seg_cnt, dest_row, gu, Xs, Ys,
+                                        any(ctx.needs_input_grad[3:6]))
+            return (dx, dgate, None) + tuple(w if n else None for w, n in zip(dws, ctx.needs_input_grad[3:6])) + (None, None)
         dYs = torch.empty(cap, H, dtype=dt, device=dev)
         _zero_pad(mctx, dYs, seg_off, seg_cnt)
         # the weighted dout rows in the expert-sorted layout and <expert output, dout> per pair, the routing-weight gradient
