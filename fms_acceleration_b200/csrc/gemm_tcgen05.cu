@@ -306,8 +306,8 @@ __device__ __forceinline__ void epilogue_store_tile(const GemmParams& p, const T
 // ragged edges of M and N.  Two slots per warp alternate; a slot is rewritten only after the store that read it.
 template <int BN>
 __device__ __forceinline__ void epilogue_store_tile_tma(const GemmParams& p, const CUtensorMap* tmD, uint32_t taddr,
-                                                        int cpar, int row0, int gm, int n0, bool empty_k, uint32_t slots,
-                                                        int lane, int& slot) {
+                                                        int cpar, int row0, int row_end, int gm, int n0, bool empty_k,
+                                                        uint32_t slots, int lane, int& slot) {
   constexpr int CH = 32;
 #pragma unroll 1
   for (int c = cpar; c < BN / CH; c += 2) {
@@ -364,7 +364,7 @@ __device__ __forceinline__ void epilogue_store_tile_tma(const GemmParams& p, con
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && gn < p.N && row0 < p.M) {
+    if (lane == 0 && gn < p.N && row0 < row_end) {
       tma_store_2d(tmD, buf, gn, row0);
       tma_store_commit();
     }
@@ -539,7 +539,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_const
       if constexpr (BN == 256) {
         // a box store writes 32 whole rows: only for tiles whose rows all belong to the segment
         if (p.tma_store && ti.m_store + BM <= ti.m_end) {
-          epilogue_store_tile_tma<BN>(p, &tmD, taddr, cpar, ti.m_store + q * 32, gm, n0, empty_k, my_slots, lane, slot);
+          // mode 2: the groups' outputs lie one below the other in one map
+          const int below = p.mode == 2 ? (int)(ti.d_off / p.ldd) : 0;
+          epilogue_store_tile_tma<BN>(p, &tmD, taddr, cpar, below + ti.m_store + q * 32, below + ti.m_end, gm, n0, empty_k,
+                                      my_slots, lane, slot);
           stored = true;
         }
       }
@@ -760,7 +763,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN2);
       if (p.tma_store)
-        epilogue_store_tile_tma<BN2>(p, &tmD, taddr, cpar, row0, gm, n0, kblocks == 0, my_slots, lane, slot);
+        epilogue_store_tile_tma<BN2>(p, &tmD, taddr, cpar, row0, p.M, gm, n0, kblocks == 0, my_slots, lane, slot);
       else
         epilogue_store_tile<BN2>(p, ti, taddr, cpar, gm, n0, kblocks == 0);
       tc_fence_before();
@@ -1063,11 +1066,17 @@ static int gemm_impl(const void* A1, long long lda1, const void* B1, long long l
     if (!a_mn && b_mn) return launch_gemm_pair<0, 1>(ta1, tb1, ta2, tb2, td, p, max_ctas, stream);
     return launch_gemm_pair<1, 1>(ta1, tb1, ta2, tb2, td, p, max_ctas, stream);
   }
-  // single-CTA kernel: the store epilogue through shared memory serves BN = 256 in the plain and grouped-M modes
+  // single-CTA kernel: the store epilogue through shared memory serves BN = 256 in the plain and grouped modes.  Grouped
+  // contractions (weight gradients, one [M, N] output per group, dense one below the other, nothing to add) are seen as
+  // one matrix of n_groups * M rows; a box store writes 32 whole rows, so whole tiles only, and an M that is no multiple
+  // of the tile leaves its last tile of every group to the per-thread stores.  Those touch half a sector per lane and
+  // instruction, and with 128 rows per expert they were most of the kernel (40 experts, 1536 x 512: 98 -> 60 us for three).
   CUtensorMap td1 = ta1;
-  if (bn == 256 && (mode == 0 || mode == 1) && bd == nullptr && g_single_tma_store && !d_fp32 && ldd % 8 == 0 &&
+  const bool stacked = mode == 2 && C == nullptr && d_group_stride == (long long)M * ldd &&
+                       (long long)n_groups * M <= 0x7fffffffLL;
+  if (bn == 256 && (mode == 0 || mode == 1 || stacked) && bd == nullptr && g_single_tma_store && !d_fp32 && ldd % 8 == 0 &&
       (reinterpret_cast<uintptr_t>(D) & 15) == 0 &&
-      make_tmap_2d_16b_sw64(&td1, D, (uint64_t)M, (uint64_t)N, (uint64_t)ldd, 32, 32) == 0)
+      make_tmap_2d_16b_sw64(&td1, D, (uint64_t)M * (stacked ? n_groups : 1), (uint64_t)N, (uint64_t)ldd, 32, 32) == 0)
     p.tma_store = 1;
 #define FMSB_DISPATCH(BNV)                                                                          \
   if (bn == BNV) {                                                                                  \

@@ -232,3 +232,25 @@ def test_dispatch_dot_and_combine_at_their_edges(T, k, H, dtype):
     assert rc == 0
     ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     assert (out.double() - out_ref).abs().max() <= ulp * out_ref.abs().max().clamp(min=1.0)
+
+
+@pytest.mark.parametrize("m,n,dtype", [(128, 256, torch.bfloat16), (256, 520, torch.float16), (192, 512, torch.bfloat16),
+                                       (1536, 512, torch.bfloat16)])
+def test_grouped_weight_gradients_store_whole_and_ragged_tiles(m, n, dtype):
+    """One output per group, dense one below the other: whole tiles leave by box stores, the last tile of an ``m`` that is
+    no multiple of 128 by per-thread stores; empty groups give zeros.  One rounding of the result (half an ulp)."""
+    torch.manual_seed(m + n)
+    sizes = [128, 0, 384, 128, 0]
+    seg_off = torch.tensor([0] + sizes, device=DEV).cumsum(0).to(torch.int32)
+    rows = int(seg_off[-1])
+    a, b = torch.randn(rows, m, device=DEV).to(dtype), torch.randn(rows, n, device=DEV).to(dtype)
+    guard = torch.full((len(sizes) * m + 256, n), 3.0, device=DEV, dtype=dtype)
+    out = guard[: len(sizes) * m].view(len(sizes), m, n)
+    MOE.grouped_gemm(a, b, seg_off, len(sizes), mode=2, m=m, n=n, out=out)
+    NV.check_status()
+    assert torch.all(guard[len(sizes) * m:] == 3.0)
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for g in range(len(sizes)):
+        s, e = int(seg_off[g]), int(seg_off[g + 1])
+        ref = a[s:e].double().t() @ b[s:e].double()
+        assert (out[g].double() - ref).abs().max() <= ulp * ref.abs().max().clamp(min=1e-9)
