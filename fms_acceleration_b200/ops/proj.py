@@ -11,13 +11,20 @@ GEMM's second operand pair (A2 = s * x A_cat^T, B2 = block-diagonal lora_B), so 
 """
 from __future__ import annotations
 
+import ctypes
 from typing import List, Optional
 
 import torch
 from torch import nn
 
+from .. import _native as N
 from . import workspace as WS
 from .gemm import gemm
+
+
+_P, _I = ctypes.c_void_p, ctypes.c_int
+N.declare("fmsb_lora_pack", [_I, _P, _P, _P, _P, _I, _I, _I, _P])
+N.declare("fmsb_lora_unpack", [_I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P])
 
 
 def _unwrap(mod: nn.Module):
@@ -129,6 +136,15 @@ class ProjGroup:
         if Rp != R:
             As.append(torch.zeros(Rp - R, self.in_features, dtype=dtype, device=device))
         A_cat = As[0] if len(As) == 1 else torch.cat(As, dim=0)
+        desc = self._native_desc(slices, dtype, device)
+        if desc is not None:
+            B_blk = torch.empty(self.total_out, Rp, dtype=dtype, device=device)
+            ptrs = (ctypes.c_void_p * desc[0])(*[_lora_parts(l)[1].data_ptr() for l in self.loras if l is not None])
+            rc = N.lib().fmsb_lora_pack(desc[0], ptrs, desc[1], desc[2], B_blk.data_ptr(), self.total_out, Rp,
+                                        N.dtype_code(dtype), N.stream_ptr())
+            N.check(rc, "fmsb_lora_pack")
+            self._lora_cat_cache = (key, (A_cat, B_blk, slices))
+            return A_cat, B_blk, slices
         B_blk = torch.zeros(self.total_out, Rp, dtype=dtype, device=device)
         for l, sl, o0, o1 in zip(self.loras, slices, self.offsets[:-1], self.offsets[1:]):
             if l is None:
@@ -137,6 +153,19 @@ class ProjGroup:
             B_blk[o0:o1, sl[0]:sl[1]] = B.to(dtype) * s
         self._lora_cat_cache = (key, (A_cat, B_blk, slices))
         return A_cat, B_blk, slices
+
+    def _native_desc(self, slices, dtype, device):
+        """(count, [o0, o1, r0, r1] per adapter, scalings) for the packing kernels of ``csrc/lora.cu``, or None when they do
+        not apply: factors on a GPU, dense, in the 16-bit dtype of the group, at most eight of them."""
+        mods = [(sl, o0, o1, _lora_parts(l)) for l, sl, o0, o1 in zip(self.loras, slices, self.offsets[:-1], self.offsets[1:])
+                if l is not None]
+        if not 1 <= len(mods) <= 8 or device.type != "cuda" or dtype not in (torch.bfloat16, torch.float16):
+            return None
+        for _, _, _, (A, B, _) in mods:
+            if A.dtype != dtype or B.dtype != dtype or not B.is_cuda or not B.is_contiguous() or type(B.data) is not torch.Tensor:
+                return None
+        flat = [v for sl, o0, o1, _ in mods for v in (o0, o1, sl[0], sl[1])]
+        return (len(mods), (ctypes.c_int * len(flat))(*flat), (ctypes.c_float * len(mods))(*[p[2] for _, _, _, p in mods]))
 
     # ------------------------------------------------------------------ forward
     def dropout_p(self) -> float:
@@ -204,6 +233,21 @@ class ProjGroup:
         y = gemm(x, W, b_mn=b_mn, a2=a2, b2=b2, c=residual, beta=beta, out=out)
         return y, xa
 
+    def _unpack_grads(self, dA_cat, dB_blk, slices, dtype, device):
+        """Per projection ``[dA, dB]`` in the factors' dtype from the packed fp32 gradients, one launch; None where the
+        packing kernels do not apply."""
+        desc = self._native_desc(slices, dtype, device)
+        if desc is None or not (dA_cat.is_contiguous() and dB_blk.is_contiguous()):
+            return None
+        out = [None if l is None else [torch.empty(p.shape, dtype=dtype, device=device) for p in _lora_parts(l)[:2]]
+               for l in self.loras]
+        live = [g for g in out if g is not None]
+        ga, gb = ((ctypes.c_void_p * len(live))(*[g[k].data_ptr() for g in live]) for k in (0, 1))
+        rc = N.lib().fmsb_lora_unpack(desc[0], ga, gb, desc[1], desc[2], dA_cat.data_ptr(), dB_blk.data_ptr(),
+                                      self.in_features, dB_blk.shape[1], N.dtype_code(dtype), N.stream_ptr())
+        N.check(rc, "fmsb_lora_unpack")
+        return out
+
     # ------------------------------------------------------------------ backward
     def backward(self, dy: torch.Tensor, x: torch.Tensor, xa: Optional[torch.Tensor], need_dx: bool = True,
                  dx_residual: Optional[torch.Tensor] = None, aux: Optional[dict] = None):
@@ -247,11 +291,15 @@ class ProjGroup:
                 dxl = gemm(dxa_s, A_cat, b_mn=True)  # [T, in]
                 dx = torch.addcmul(dx, dxl, mask.to(dtype), value=aux["keep_scale"])
         # parameter gradients in the order of trainable()
+        lora_grads = self._unpack_grads(dA_cat, dB_blk, slices, dtype, dev) if self.has_lora else None
         for i, (b, l) in enumerate(zip(self.bases, self.loras)):
             o0, o1 = self.offsets[i], self.offsets[i + 1]
             if self.kind == "dense" and b.weight.requires_grad:
                 grads.append(gemm(dy[:, o0:o1], x, a_mn=True, b_mn=True, out_dtype=torch.float32))
             if l is not None:
+                if lora_grads is not None:
+                    grads += lora_grads[i]
+                    continue
                 r0, r1, s = slices[i]
                 A, B, _ = _lora_parts(l)
                 grads.append(dA_cat[r0:r1].to(A.dtype))

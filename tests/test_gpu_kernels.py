@@ -581,3 +581,46 @@ def test_scale_cast_rounds_once(n, dtype):
     src, factor = torch.randn(n, device=DEV), torch.tensor(0.37, device=DEV)
     assert torch.equal(_scaled_cast(src, factor, dtype), (src * factor).to(dtype))
     assert torch.equal(_scaled_cast(torch.randn(n + 1, device=DEV)[1:].copy_(src), factor, dtype), (src * factor).to(dtype))
+
+
+@pytest.mark.parametrize("outs,ranks,inp,dtype", [([48], [3], 40, torch.bfloat16), ([64, None, 24], [16, 0, 5], 72, torch.float16),
+                                                  ([4096, 1024, 1024], [16, 16, 16], 512, torch.bfloat16), ([8] * 9, [2] * 9, 16, torch.bfloat16)])
+def test_lora_factors_pack_and_unpack_like_the_torch_form(outs, ranks, inp, dtype):
+    """Block-diagonal B with the scaling folded in, and the gradients of that layout cut apart: the same bits as the torch
+    operators (kept for what the kernels do not take: more than eight adapters, other dtypes)."""
+    from torch import nn
+
+    from fms_acceleration_b200.nn import LoraConfig, get_peft_model
+    from fms_acceleration_b200.ops.proj import ProjGroup
+
+    torch.manual_seed(len(outs) + inp)
+
+    class Holder(nn.Module):
+        def __init__(self):
+            super().__init__()
+            for i, o in enumerate(outs):
+                setattr(self, f"p{i}", nn.Linear(inp, o or 32, bias=False))
+
+    h = Holder().to(DEV, dtype)
+    for i, (o, r) in enumerate(zip(outs, ranks)):
+        if o is not None:
+            get_peft_model(h, LoraConfig(r=r, lora_alpha=3 * r + 1, target_modules=[f"p{i}"]))
+    group = ProjGroup([getattr(h, f"p{i}") for i in range(len(outs))], "t")
+    with torch.no_grad():
+        for p in group.trainable():
+            p.copy_(torch.randn_like(p))
+    A, B, slices = group.lora_cat(dtype, torch.device(DEV))
+    native = group._native_desc
+    assert (native(slices, dtype, torch.device(DEV)) is None) == (len(outs) > 8)
+    da, db = torch.randn(A.shape, device=DEV), torch.randn(B.shape, device=DEV)
+    got = group._unpack_grads(da, db, slices, dtype, torch.device(DEV))
+    group._native_desc = lambda *a: None
+    A2, B2, _ = group.lora_cat(dtype, torch.device(DEV))
+    assert torch.equal(A, A2) and torch.equal(B, B2)
+    if got is not None:
+        for g, sl, o0, o1 in zip(got, slices, group.offsets[:-1], group.offsets[1:]):
+            if sl is None:
+                assert g is None
+                continue
+            assert torch.equal(g[0], da[sl[0]:sl[1]].to(dtype))
+            assert torch.equal(g[1], (db[o0:o1, sl[0]:sl[1]] * sl[2]).to(dtype))
