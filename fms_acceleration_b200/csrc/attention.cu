@@ -49,9 +49,15 @@ __device__ __forceinline__ uint32_t swz_off(int r, int c16) {
 // operand from tensor memory.  The running maximum is only advanced (and O rescaled) when the
 // block maximum exceeds it by more than 2^8, so most blocks skip the O round trip.
 // The softmax warps bound it (two per scheduler: issue and the special-function unit), so their chains are split and
-// multiply-add / add work on pairs.  T = 16384 packed, 32/8 heads, d = 128: 729 -> 565 us; one document of 4001
+// multiply-add / add work on pairs.  T = 16384 packed, 32/8 heads, d = 128: 729 -> 571 us; one document of 4001
 // tokens: 250 -> 147 us (890 TFLOP/s; most of that from the order of the grid).
 // ----------------------------------------------------------------------------------------
+// Warps 0 (TMA) and 1 (MMA) and two idle ones give registers to the eight softmax warps: a row's 128 scores and what is made of
+// them do not fit into the 168 registers that an even split allows, and with shared memory this full a spill goes to L2
+// (T = 16384 packed, d = 128: 571 -> 548 us; T = 1500, d = 64: 22.9 -> 21.9 us; 4001 tokens of one document unchanged).
+constexpr int FWD_THREADS = 384;
+constexpr int FWD_REGS_MAIN = 72, FWD_REGS_SOFTMAX = 216;  // 128 * 72 + 256 * 216 = 384 * 168
+
 template <int D>
 struct AttnFwd2Cfg {
   static constexpr int kTileBytes = 128 * D * 2;
@@ -60,7 +66,7 @@ struct AttnFwd2Cfg {
 };
 
 template <int D, int FMT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
   using Cfg = AttnFwd2Cfg<D>;
@@ -83,8 +89,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // Heads run fastest: the CTAs of all heads that share a query tile start together and the tiles with the most key
   // blocks of a long document (the last ones) start first.  With the tiles fastest, the long tiles of the last heads
   // started at the end of the grid and the machine waited for them.
-  const int qt = gridDim.y - 1 - blockIdx.y;
-  const int head = blockIdx.x;
+  const int qt = gridDim.x / p.nh - 1 - blockIdx.x / p.nh;
+  const int head = blockIdx.x % p.nh;
   const int hk = head / (p.nh / p.nkv);
   const int q0 = qt * 256;
   // per-tile key-block ranges (tile 1 may lie completely beyond T)
@@ -127,8 +133,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   auto tS = [&](int x) { return tmem + 128u * x; };
   auto tO = [&](int x) { return tmem + 256u + 128u * x; };
 
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FWD_REGS_MAIN));
+    if (warp == 0 && lane == 0) {
       mbar_expect_tx(bar_q, (exists[1] ? 2 : 1) * Cfg::kTileBytes);
       for (int x = 0; x < 2; ++x) {
         if (!exists[x]) continue;
@@ -147,9 +154,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tma_load_2d(sV(s) + h * Cfg::kHalfBytes, &tmV, bar_kv_full(s), hk * D + 64 * h, k0);
         }
       }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    } else if (warp == 1 && lane == 0) {
       const uint32_t idesc_s = make_idesc_f16(128, 128, FMT, 0, 0);
       const uint32_t idesc_o = make_idesc_f16(128, D, FMT, 0, 1);
       auto issue_s = [&](int x, int j) {
@@ -199,8 +204,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FWD_REGS_SOFTMAX));
     // ------------------------------------------------------------------ softmax warpgroups
-    const int x = (warp - 2) >> 2;  // tile handled by this warpgroup
+    const int x = (warp - 4) >> 2;  // tile handled by this warpgroup
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int t = q0 + 128 * x + row;
@@ -400,6 +406,16 @@ namespace fmsb_host {
 int sm_count();
 }
 
+// The register split draws on what the block was launched with: a build that gave the kernel fewer registers per thread would
+// wait for them without end, so it is refused.
+template <typename K>
+static int fwd_regs(K kern) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return (int)e;
+  return a.numRegs * FWD_THREADS >= 128 * FWD_REGS_MAIN + 256 * FWD_REGS_SOFTMAX ? 0 : -3;
+}
+
 extern "C" int fmsb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv,
                              void* o, long long ldo, float* lse, const int* doc_start, const int* doc_end, int T,
                              int nh, int nkv, int d, float scale, int fmt, int* status, cudaStream_t stream) {
@@ -416,7 +432,9 @@ extern "C" int fmsb_attn_fwd(const void* q, long long ldq, const void* k, long l
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end;
   p.o = o; p.ldo = ldo; p.lse = lse; p.fmt = fmt; p.status = status;
-  dim3 grid(nh, (T + 255) / 256);
+  const long long ctas = (long long)nh * ((T + 255) / 256);
+  if (ctas > 0x7fffffffLL) return -2;
+  const dim3 grid((unsigned)ctas);
 #define FMSB_FWD2(DD, FF)                                                                                         \
   do {                                                                                                            \
     static bool cfg = false;                                                                                      \
@@ -424,9 +442,10 @@ extern "C" int fmsb_attn_fwd(const void* q, long long ldq, const void* k, long l
       cudaError_t e = cudaFuncSetAttribute(attn_fwd2_kernel<DD, FF>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                            AttnFwd2Cfg<DD>::kSmemBytes);                                          \
       if (e != cudaSuccess) return (int)e;                                                                        \
+      if (int r = fwd_regs(attn_fwd2_kernel<DD, FF>)) return r;                                                   \
       cfg = true;                                                                                                 \
     }                                                                                                             \
-    attn_fwd2_kernel<DD, FF><<<grid, 320, AttnFwd2Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, p);                  \
+    attn_fwd2_kernel<DD, FF><<<grid, FWD_THREADS, AttnFwd2Cfg<DD>::kSmemBytes, stream>>>(tq, tk, tv, p);                  \
   } while (0)
   if (d == 128 && fmt == 1) FMSB_FWD2(128, 1);
   else if (d == 128) FMSB_FWD2(128, 0);

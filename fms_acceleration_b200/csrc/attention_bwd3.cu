@@ -142,8 +142,8 @@ attn_bwd_dkv3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   float* scal_f = reinterpret_cast<float*>(smem_raw + (scal - smem_u32(smem_raw)));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.y;  // early tiles have the most queries: they start first, heads fastest
-  const int hk = blockIdx.x;
+  const int kt = blockIdx.x / p.nkv;  // early tiles have the most queries: they start first, heads fastest
+  const int hk = blockIdx.x % p.nkv;
   const int G = p.nh / p.nkv;
   const int k0 = kt * B3_T;
   const int k_last = min(k0 + B3_T - 1, p.T - 1);
@@ -405,8 +405,8 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t holder = bars + 8u * 16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.y - 1 - blockIdx.y;  // long tiles (late in their document) first, heads fastest
-  const int head = blockIdx.x;
+  const int qt = gridDim.x / p.nh - 1 - blockIdx.x / p.nh;  // long tiles (late in their document) first, heads fastest
+  const int head = blockIdx.x % p.nh;
   const int hk = head / (p.nh / p.nkv);
   const int q0 = qt * B3_T;
   const int q_last = min(q0 + B3_T - 1, p.T - 1);
@@ -483,7 +483,7 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int ks = 1; ks < 8; ++ks) tc_mma_f16_ts(tdQ, ds + b3_pcol(ks), smem_desc_at(b, ks * 2048), idesc_g, 1u);
       };
-      const bool tr = blockIdx.y == gridDim.y / 2 && blockIdx.x == 0;
+      const bool tr = blockIdx.x == gridDim.x / p.nh / 2 * p.nh;
       FMSB_TRACE3(tr, 4000);
       bool ok = mbar_wait(bar_q, 0, p.status, kTimeoutMma);
       FMSB_TRACE3(tr, 4001);
@@ -532,7 +532,7 @@ attn_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float dlt = row_ok ? p.delta[(long long)head * p.T + t] : 0.f;
     const uint64_t sl2x2 = pack_f32x2(sl2, sl2), nlse2 = pack_f32x2(-lse2, -lse2), ndlt2 = pack_f32x2(-dlt, -dlt);
     const int c0 = cq * 32;
-    const bool trc = blockIdx.y == gridDim.y / 2 && blockIdx.x == 0 && threadIdx.x == 64;
+    const bool trc = blockIdx.x == gridDim.x / p.nh / 2 * p.nh && threadIdx.x == 64;
     bool ok = true;
     FMSB_TRACE3(trc, 12);
     for (int j = 0; j < nblk && ok; ++j) {
@@ -650,7 +650,9 @@ extern "C" int fmsb_attn_bwd_dq3(const void* q, long long ldq, const void* k, lo
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end; p.lse = lse; p.delta = delta;
   p.dq = dq; p.lddq = lddq; p.fmt = fmt; p.status = status;
-  dim3 grid(nh, (T + B3_T - 1) / B3_T);
+  const long long ctas = (long long)nh * ((T + B3_T - 1) / B3_T);
+  if (ctas > 0x7fffffffLL) return -2;
+  const dim3 grid((unsigned)ctas);
 #define FMSB_B3(DD, FF)                                                                                          \
   do {                                                                                                           \
     static bool cfg = false;                                                                                     \
@@ -683,7 +685,9 @@ extern "C" int fmsb_attn_bwd_dkv3(const void* q, long long ldq, const void* k, l
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end; p.lse = lse; p.delta = delta;
   p.dk = dk; p.lddk = lddk; p.dv = dv; p.lddv = lddv; p.fmt = fmt; p.status = status;
-  dim3 grid(nkv, (T + B3_T - 1) / B3_T);
+  const long long ctas = (long long)nkv * ((T + B3_T - 1) / B3_T);
+  if (ctas > 0x7fffffffLL) return -2;
+  const dim3 grid((unsigned)ctas);
 #define FMSB_B3(DD, FF)                                                                                          \
   do {                                                                                                           \
     static bool cfg = false;                                                                                     \
