@@ -98,6 +98,12 @@ def launch_count() -> int:
     return 0 if _LIB is None else _LIB.calls
 
 
+def add_launches(n: int) -> None:
+    """Counts the launches of a native call that makes ``n`` more than one (whole sequences in one call)."""
+    if _LIB is not None:
+        _LIB.calls += n
+
+
 def declare(name: str, argtypes) -> None:
     """Register the signature of an entry point defined outside this table."""
     _SIGNATURES[name] = argtypes

@@ -112,6 +112,7 @@ def _bwd(q2, k2, v2, o, lse, dout, doc_start, doc_end, nh, nkv, d, scale, dq=Non
                                doc_start.data_ptr(), doc_end.data_ptr(), T, nh, nkv, d, float(scale),
                                N.dtype_code(q2.dtype), st.data_ptr(), N.stream_ptr())
     N.check(rc, "fmsb_attn_bwd")
+    N.add_launches(2)
     return dq, dk, dv
 
 

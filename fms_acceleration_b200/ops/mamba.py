@@ -524,6 +524,7 @@ def _fused_forward(x2, dt, A32, B2, C2, D32, h0, y, nh, G):
                                     ws.data_ptr(), nc, nh, G, NV.dtype_code(x2.dtype), NV.status_word(dev).data_ptr(),
                                     NV.stream_ptr())
     NV.check(rc, "fmsb_ssdf_forward")
+    NV.add_launches(2 + (y is not None))
     return hprev, hT
 
 
@@ -583,6 +584,7 @@ class _SSDScanFused(torch.autograd.Function):
                                              sums.data_ptr(), NV.ptr(dh0), ws.data_ptr(), nc, nh, G, NV.dtype_code(dtp),
                                              NV.status_word(dev).data_ptr(), NV.stream_ptr())
             NV.check(rc, "fmsb_ssdf_backward")
+            NV.add_launches(12)
             dA, dD = sums.sum(1)
             return (dx, ddt, dA.to(A.dtype), dB, dC, dD.to(D.dtype), dh0, None, None, None)
         # context parallelism: the same launches around the exchange

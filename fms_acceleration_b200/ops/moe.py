@@ -488,6 +488,7 @@ def _local_fwd(mctx, x, gates, idx, w1, w3, w2, act, cap):
                                     _counter(_overflow, dev).data_ptr(), N.dtype_code(dt), mctx.gemm_ctas,
                                     N.status_word(dev).data_ptr(), N.stream_ptr())
     N.check(rc, "fmsb_moe_local_fwd")
+    N.add_launches(6)
     return out, (seg_off, seg_cnt, dest_row, gu, Xs, Ys)
 
 
@@ -511,6 +512,7 @@ def _local_bwd(mctx, dout, gates, idx, w1, w3, w2, act, seg_off, seg_cnt, dest_r
                                     N.ptr(dws[1]), N.ptr(dws[2]), N.dtype_code(dt), mctx.gemm_ctas,
                                     N.status_word(dev).data_ptr(), N.stream_ptr())
     N.check(rc, "fmsb_moe_local_bwd")
+    N.add_launches(9 if need_dw else 5)
     return dx, dgate, dws
 
 
