@@ -861,23 +861,6 @@ extern "C" int fmsb_moe_dispatch(const void* x, long long ldx, const int* topk_i
 }
 
 // Dispatch that also delivers one fp32 value per (token, k) pair into the owner's per-row array `meta_recv`.
-extern "C" int fmsb_moe_dispatch_meta(const void* x, long long ldx, const int* topk_idx, const int* dest_row,
-                                      const float* meta_vals, long long n_pairs, int k, int H, int E_local,
-                                      void* const* recv, long long ld_recv, void* const* meta_recv, int world, int dtype,
-                                      cudaStream_t stream) {
-  if (n_pairs <= 0) return 0;
-  if (H % 8 != 0 || ldx % 8 != 0 || ld_recv % 8 != 0 || meta_vals == nullptr || k < 1 || k > 32 || n_pairs % k != 0)
-    return -2;
-  MoePeers r = moe_ptrs(recv, world), m = moe_ptrs(meta_recv, world);
-  const long long n_tokens = n_pairs / k;
-  const long long blocks = (n_tokens * 32 + 255) / 256;
-  if (dtype == 1)
-    moe_dispatch_kernel<__nv_bfloat16, false><<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, topk_idx, dest_row, nullptr, n_tokens, k, H, E_local, r, ld_recv, meta_vals, m, 0, nullptr);
-  else
-    moe_dispatch_kernel<__half, false><<<(unsigned)blocks, 256, 0, stream>>>((const __half*)x, ldx, topk_idx, dest_row, nullptr, n_tokens, k, H, E_local, r, ld_recv, meta_vals, m, 0, nullptr);
-  return (int)cudaGetLastError();
-}
-
 // see moe_dispatch_dot_kernel; one GPU (rows of a local buffer)
 extern "C" int fmsb_moe_dispatch_dot(const void* dout, long long ldd, const int* dest_row, const float* gate,
                                      long long n_tokens, int k, int H, const void* y, long long ldy, void* dy,

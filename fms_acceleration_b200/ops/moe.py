@@ -47,7 +47,6 @@ N.declare("fmsb_moe_dispatch", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_zero_pad", [P, L, I, P, P, I, I, P])
 N.declare("fmsb_moe_combine", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_gate_grad", [P, L, P, P, P, L, L, I, I, I, P, I, I, P])
-N.declare("fmsb_moe_dispatch_meta", [P, L, P, P, P, L, I, I, I, P, L, P, I, I, P])
 N.declare("fmsb_moe_local_fwd", [P, L, P, P, L, I, I, I, I, P, P, P, I, P, P, P, P, I, P, P, P, P, P, P, P, I, I, P, P])
 N.declare("fmsb_moe_local_bwd", [P, L, P, P, P, P, P, P, P, P, L, I, I, I, I, P, P, P, I, I, P, P, P, P, P, P, P, P, P, I, I, P, P])
 N.declare("fmsb_moe_dispatch_dot", [P, L, P, P, L, I, I, P, L, P, L, P, I, P])
