@@ -860,7 +860,6 @@ extern "C" int fmsb_moe_dispatch(const void* x, long long ldx, const int* topk_i
   return (int)cudaGetLastError();
 }
 
-// Dispatch that also delivers one fp32 value per (token, k) pair into the owner's per-row array `meta_recv`.
 // see moe_dispatch_dot_kernel; one GPU (rows of a local buffer)
 extern "C" int fmsb_moe_dispatch_dot(const void* dout, long long ldd, const int* dest_row, const float* gate,
                                      long long n_tokens, int k, int H, const void* y, long long ldy, void* dy,
