@@ -465,11 +465,18 @@ extern "C" int fmsb_conv1d_bwd(const void* dy, long long lddy, const void* dy2, 
   return (int)cudaGetLastError();
 }
 
+// The state kernels move four elements an access: fp32 pointers on 16 bytes, 16-bit ones on 8 (null passes).
+static bool state_aligned(const void* a, const void* b, const void* c, const void* h16, const void* s16) {
+  const uintptr_t f = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+  const uintptr_t h = reinterpret_cast<uintptr_t>(h16) | reinterpret_cast<uintptr_t>(s16);
+  return (f & 15u) == 0 && (h & 7u) == 0;
+}
+
 extern "C" int fmsb_ssd_state_fwd(const float* S, const float* Ltot, const float* h0, void* hprev, float* hT, int nc,
                                   int nh, int PN, int dtype, cudaStream_t stream) {
   const long long total = (long long)nh * PN;
   if (total <= 0) return 0;
-  if (PN % 4 != 0) return -2;
+  if (PN % 4 != 0 || !state_aligned(S, h0, hT, hprev, nullptr)) return -2;
   const unsigned blocks = (unsigned)((total / 4 + 127) / 128);
   if (dtype == 1) ssd_state_fwd_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(S, Ltot, h0, (__nv_bfloat16*)hprev, hT, nc, nh, PN);
   else if (dtype == 0) ssd_state_fwd_kernel<__half><<<blocks, 128, 0, stream>>>(S, Ltot, h0, (__half*)hprev, hT, nc, nh, PN);
@@ -482,7 +489,7 @@ extern "C" int fmsb_ssd_state_bwd(const float* dhprev_direct, const float* dhT, 
                                   cudaStream_t stream) {
   const long long total = (long long)nh * PN;
   if (total <= 0) return 0;
-  if (PN % 4 != 0) return -2;
+  if (PN % 4 != 0 || !state_aligned(dhprev_direct, dhT, dh0, hprev, dS)) return -2;
   const unsigned blocks = (unsigned)((total / 4 + 127) / 128);
   if (dtype == 1) ssd_state_bwd_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(dhprev_direct, dhT, Ltot, (const __nv_bfloat16*)hprev, (__nv_bfloat16*)dS, dh0, dLtot, nc, nh, PN);
   else if (dtype == 0) ssd_state_bwd_kernel<__half><<<blocks, 128, 0, stream>>>(dhprev_direct, dhT, Ltot, (const __half*)hprev, (__half*)dS, dh0, dLtot, nc, nh, PN);

@@ -156,6 +156,16 @@ def _rows16(t2):
     return t2 if t2.data_ptr() % 16 == 0 and t2.is_contiguous() else t2.contiguous().clone()
 
 
+def _state32(t):
+    """A state [nh, P, N] (or its gradient) for the recurrence kernels, which read it 16 bytes at a time: fp32, dense and
+    16-byte aligned.  ``float().contiguous()`` alone returns an fp32 view as it is, at whatever offset of its buffer it
+    starts (a state behind a scalar in a flat buffer, the gradient of a concatenation)."""
+    if t is None:
+        return None
+    t = t.float().contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _chunk_major(v, nc, Q, nh):
     """[T, nh] fp32 -> [nc, nh, Q] contiguous (unit stride along the chunk for the Q x Q kernels)."""
     return v.view(nc, Q, nh).transpose(1, 2).contiguous()
@@ -223,7 +233,7 @@ def _chunk_states(x2, dt, A, B2, C2, h0, T, nh, P, G, N, Q, dtp, dev, cp=None, w
         NV.check(rc, "fmsb_ssd_state_fwd")
     hprev = torch.empty(nc * nh * P, N, dtype=dtp, device=dev)
     hT = torch.empty(nh, P, N, dtype=torch.float32, device=dev)
-    h0c = None if h0 is None else h0.float().contiguous()
+    h0c = _state32(h0)
     rc = NV.lib().fmsb_ssd_state_fwd(S.data_ptr(), Ltot.data_ptr(), NV.ptr(h0c), hprev.data_ptr(), hT.data_ptr(), nc,
                                      nh, P * N, NV.dtype_code(dtp), NV.stream_ptr())
     NV.check(rc, "fmsb_ssd_state_fwd")
@@ -328,7 +338,7 @@ class _SSDScan(torch.autograd.Function):
         dS16 = torch.empty(nc * nh * P, N, dtype=dtp, device=dev)
         dh0 = torch.empty(nh, P, N, dtype=torch.float32, device=dev) if (has_h0 or cp is not None) else None
         dLtot = torch.zeros(nc, nh, dtype=torch.float32, device=dev)
-        dhTc = None if dhT is None else dhT.float().contiguous()
+        dhTc = _state32(dhT)
         rc = NV.lib().fmsb_ssd_state_bwd(dhp.data_ptr(), NV.ptr(dhTc), Ltot.data_ptr(), hprev.data_ptr(),
                                          dS16.data_ptr(), NV.ptr(dh0), dLtot.data_ptr(), nc, nh, P * N, code,
                                          NV.stream_ptr())
@@ -495,7 +505,7 @@ class _Fused:
             self._recur(S, None, hprev0, torch.empty(self.nh, 64, 128, dtype=torch.float32, device=self.dev))
         hprev = torch.empty(shape, dtype=self.dtype, device=self.dev)
         hT = torch.empty(self.nh, 64, 128, dtype=torch.float32, device=self.dev)
-        h0 = None if h0 is None else h0.float().contiguous()
+        h0 = _state32(h0)
         self._recur(S, h0, hprev, hT)
         return hprev, hT, h0, hprev0
 
@@ -517,7 +527,7 @@ def _fused_forward(x2, dt, A32, B2, C2, D32, h0, y, nh, G):
     nc, dev = x2.shape[0] // 256, x2.device
     hprev = torch.empty(nc * nh * 64, 128, dtype=x2.dtype, device=dev)
     hT = torch.empty(nh, 64, 128, dtype=torch.float32, device=dev)
-    h0 = None if h0 is None else h0.float().contiguous()
+    h0 = _state32(h0)
     ws = torch.empty(_fused_workspace(0, nc, nh, G), dtype=torch.uint8, device=dev)
     rc = NV.lib().fmsb_ssdf_forward(x2.data_ptr(), dt.data_ptr(), A32.data_ptr(), B2.data_ptr(), B2.stride(0), C2.data_ptr(),
                                     C2.stride(0), NV.ptr(D32), NV.ptr(h0), NV.ptr(y), hT.data_ptr(), hprev.data_ptr(),
@@ -569,7 +579,7 @@ class _SSDScanFused(torch.autograd.Function):
         B2, C2 = _vec_rows(B.reshape(T, G * N)), _vec_rows(C.reshape(T, G * N))
         dy2 = _rows16(dy.reshape(T, nh * P))
         A32, D32 = A.float().contiguous(), D.float().contiguous()
-        dhTc = None if dhT is None else dhT.float().contiguous()
+        dhTc = _state32(dhT)
         dx = torch.empty(T, nh, P, dtype=dtp, device=dev)
         ddt = torch.empty(T, nh, dtype=torch.float32, device=dev)
         sums = torch.empty(2, nc, nh, dtype=torch.float32, device=dev)

@@ -105,3 +105,20 @@ def test_gemm_host_statement_of_the_kernel_contract():
     assert gemm(a, b, a2=a2, b2=b2, c=c, alpha=0.5, beta=2.0, out=out) is out
     assert torch.allclose(out, want, atol=1e-6)
     assert gemm(a.bfloat16(), b.bfloat16(), out_dtype=torch.float32).dtype == torch.float32
+
+
+def test_states_reach_the_recurrence_kernels_dense_and_aligned():
+    """What the recurrence kernels read 16 bytes at a time is copied when it starts elsewhere; an aligned state is not."""
+    import torch
+
+    from fms_acceleration_b200.ops.mamba import _state32
+
+    flat = torch.arange(2 * 8 * 16 + 4, dtype=torch.float32)
+    assert flat.data_ptr() % 16 == 0 and _state32(None) is None
+    for off in range(4):
+        v = flat[off: off + 256].view(2, 8, 16)
+        got = _state32(v)
+        assert got.data_ptr() % 16 == 0 and got.is_contiguous() and torch.equal(got, v)
+        assert (got.data_ptr() == v.data_ptr()) == (off == 0)
+    half = torch.randn(2, 8, 16).bfloat16().transpose(1, 2)
+    assert _state32(half).dtype == torch.float32 and torch.equal(_state32(half), half.float())
