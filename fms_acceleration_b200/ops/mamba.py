@@ -433,6 +433,14 @@ def _fused_ok(x, B, C, Q):
             and x.dtype in (torch.bfloat16, torch.float16) and B.dtype == x.dtype and C.dtype == x.dtype)
 
 
+def _fused_vectors_ok(x, dt, A, D):
+    """``dt [T, nh]``, ``A [nh]`` and ``D [nh]`` on the device of ``x``: the fused kernels read them by address.  The general path
+    takes ``dt`` and ``A`` through tensor operators, which broadcast or refuse what has another shape or device; such a call
+    goes there."""
+    T, nh = x.shape[:2]
+    return dt.shape == (T, nh) and A.shape == D.shape == (nh,) and dt.device == A.device == D.device == x.device
+
+
 @functools.lru_cache(maxsize=256)
 def _fused_heads(kind, nc, nh, G):
     hp = NV.lib().fmsb_ssdf_heads(kind, nc, nh, G)
@@ -728,5 +736,5 @@ def ssd_scan(x, dt, A, B, C, D, h0=None, chunk_size=256, recompute=False, cp=Non
     if not x.is_cuda:
         y, h = ssd_ref(x, dt, A, B, C, D, h0)
         return y.to(x.dtype), h.float()
-    fn = _SSDScanFused if _fused_ok(x, B, C, chunk_size) else _SSDScan
+    fn = _SSDScanFused if _fused_ok(x, B, C, chunk_size) and _fused_vectors_ok(x, dt, A, D) else _SSDScan
     return fn.apply(x, dt, A, B, C, D, h0, chunk_size, bool(recompute), cp)

@@ -171,6 +171,24 @@ def test_fused_scan_with_an_exchange_around_it(recompute):
         assert _rel(a, b) < 1e-5, (i, _rel(a, b))
 
 
+def test_scan_broadcasts_or_refuses_per_head_vectors_of_other_shapes():
+    """One decay rate for all heads (shape [1]) gives what the expanded vector gives; a step size of another shape and a
+    decay rate on the host are refused before any launch."""
+    torch.manual_seed(7)
+    T, nh, P, N = 512, 4, 64, 128
+    x = (torch.randn(T, nh, P, device=DEV) * 0.5).bfloat16()
+    B, C = ((torch.randn(T, 1, N, device=DEV) * 0.3).bfloat16() for _ in range(2))
+    dt, A, D = torch.rand(T, nh, device=DEV) * 0.09 + 0.01, torch.tensor([-1.5], device=DEV), torch.randn(nh, device=DEV)
+    with torch.no_grad():
+        y, h = MB.ssd_scan(x, dt, A, B, C, D)
+        yr, hr = MB.ssd_scan(x, dt, A.expand(nh).contiguous(), B, C, D)
+        for bad in ((dt[:, :1], A.expand(nh)), (dt[:256], A.expand(nh)), (dt, A.expand(nh).cpu())):
+            with pytest.raises((RuntimeError, ValueError)):
+                MB.ssd_scan(x, bad[0], bad[1], B, C, D)
+    NV.check_status()
+    assert _rel(y, yr) < 4 * 2.0 ** -8 and _rel(h, hr) < 4 * 2.0 ** -8
+
+
 @pytest.mark.parametrize("fused", [True, False])
 def test_states_at_any_offset_of_their_buffer(fused):
     """An entering state and a gradient of the final state that are dense fp32 views one element into their buffers give the

@@ -122,3 +122,18 @@ def test_states_reach_the_recurrence_kernels_dense_and_aligned():
         assert (got.data_ptr() == v.data_ptr()) == (off == 0)
     half = torch.randn(2, 8, 16).bfloat16().transpose(1, 2)
     assert _state32(half).dtype == torch.float32 and torch.equal(_state32(half), half.float())
+
+
+def test_fused_scan_takes_only_vectors_it_may_read_by_address():
+    """Per-head vectors of another length, shape or device go to the general path, whose tensor operators broadcast or
+    refuse them."""
+    import torch
+
+    from fms_acceleration_b200.ops.mamba import _fused_vectors_ok
+
+    x, dt, A, D = torch.zeros(512, 4, 64), torch.zeros(512, 4), torch.zeros(4), torch.zeros(4)
+    assert _fused_vectors_ok(x, dt, A, D) and _fused_vectors_ok(x, torch.zeros(4, 512).t(), A.double(), D)
+    for bad in (dict(dt=torch.zeros(512, 1)), dict(dt=torch.zeros(256, 4)), dict(dt=torch.zeros(1, 512, 4)),
+                dict(A=torch.zeros(1)), dict(A=torch.zeros(())), dict(A=torch.zeros(5)), dict(D=torch.zeros(1)),
+                dict(dt=dt.to("meta")), dict(A=A.to("meta")), dict(D=D.to("meta"))):
+        assert not _fused_vectors_ok(**{**dict(x=x, dt=dt, A=A, D=D), **bad}), bad
