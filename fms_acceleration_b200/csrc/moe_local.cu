@@ -39,10 +39,11 @@ struct Group {  // what the grouped products of one call share
   int* status;
   cudaStream_t stream;
 
-  // D [cap, n] = A [cap, K] . B_g (+ A2 . B2_g); B stored [E * K, n] (b_mn) or [E * n, K]; B_alt: the right half of D
+  // D [cap, n] = A [cap, K] . B_g (+ A2 . B2_g); B stored [E * K, n] (b_mn) or [E * n, K]; B_alt: the right half of D, rows
+  // as far apart as B's
   int rows(const void* A, long long lda, const void* B, long long ldb, int K, int b_mn, const void* B_alt, int n_split,
-           const void* A2, long long lda2, const void* B2, int K2, void* D, long long ldd, int n) const {
-    return fmsb_grouped_gemm2(A, lda, B, ldb, K, b_mn, B_alt, n_split, A2, lda2, B2, A2 ? ldb : 0, K2, D, ldd, 0, nullptr, 0, 0,
+           const void* A2, long long lda2, const void* B2, long long ldb2, int K2, void* D, long long ldd, int n) const {
+    return fmsb_grouped_gemm2(A, lda, B, ldb, K, b_mn, B_alt, n_split, A2, lda2, B2, ldb2, K2, D, ldd, 0, nullptr, 0, 0,
                               1.f, 0.f, 0, n, fmt, tile_n(n, n_split), 1, E, seg_off, 0, cap, (long long)E * (b_mn ? K : n),
                               max_ctas, status, stream);
   }
@@ -56,12 +57,12 @@ struct Group {  // what the grouped products of one call share
 
 #define FMSB_TRY(call) do { if (int rc_ = (call)) return rc_; } while (0)
 
-// x [T, H]; idx, gates [T, k]; w1, w3 [E, H, I], w2 [E, I, H].  ws: 3 E + max(1, ceil(T k / 1024)) E ints.  seg_off [E + 1],
-// seg_cnt [E], dest_row [T, k]; Xs, Ys [cap, H], gu [cap, 2 I], hs [cap, I]; out [T, H].
+// x [T, H]; idx, gates [T, k]; w1, w3 [E, H, I] with rows ld13 apart, w2 [E, I, H] with rows ld2 apart.
+// ws: 3 E + max(1, ceil(T k / 1024)) E ints.  seg_off [E + 1], seg_cnt [E], dest_row [T, k]; Xs, Ys [cap, H], gu [cap, 2 I], hs [cap, I]; out [T, H].
 extern "C" int fmsb_moe_local_fwd(const void* x, long long ldx, const int* idx, const float* gates, long long T, int k, int H,
-                                  int I, int E, const void* w1, const void* w3, const void* w2, int act, int* ws, int* seg_off,
-                                  int* seg_cnt, int* dest_row, int cap, void* Xs, void* gu, void* hs, void* Ys, void* out,
-                                  int* needed, int* overflow, int fmt, int max_ctas, int* status, cudaStream_t stream) {
+                                  int I, int E, const void* w1, const void* w3, long long ld13, const void* w2, long long ld2,
+                                  int act, int* ws, int* seg_off, int* seg_cnt, int* dest_row, int cap, void* Xs, void* gu,
+                                  void* hs, void* Ys, void* out, int* needed, int* overflow, int fmt, int max_ctas, int* status, cudaStream_t stream) {
   FMSB_TRY((int)cudaMemsetAsync(ws, 0, sizeof(int) * E, stream));
   FMSB_TRY(fmsb_moe_plan(idx, T * k, E, 0, 1, cap, ws, nullptr, nullptr, 0, seg_off, seg_cnt, ws + E, dest_row, needed,
                          ws + 3 * E, overflow, status, stream));
@@ -70,9 +71,9 @@ extern "C" int fmsb_moe_local_fwd(const void* x, long long ldx, const int* idx, 
   FMSB_TRY(fmsb_moe_dispatch(x, ldx, idx, dest_row, nullptr, T * k, k, H, E, xs, H, 1, fmt, stream));
   const Group g{seg_off, E, cap, fmt, max_ctas, status, stream};
   uint16_t* gu16 = (uint16_t*)gu;
-  FMSB_TRY(g.rows(Xs, H, w1, I, H, 1, w3, I, nullptr, 0, nullptr, 0, gu, 2LL * I, 2 * I));
+  FMSB_TRY(g.rows(Xs, H, w1, ld13, H, 1, w3, I, nullptr, 0, nullptr, 0, 0, gu, 2LL * I, 2 * I));
   FMSB_TRY(fmsb_glu_fwd(gu16, gu16 + I, hs, cap, I, 2LL * I, 2LL * I, I, act, fmt, seg_off + E, stream));
-  FMSB_TRY(g.rows(hs, I, w2, H, I, 1, nullptr, 0, nullptr, 0, nullptr, 0, Ys, H, H));
+  FMSB_TRY(g.rows(hs, I, w2, ld2, I, 1, nullptr, 0, nullptr, 0, nullptr, 0, 0, Ys, H, H));
   void* ys[1] = {Ys};
   return fmsb_moe_combine(ys, H, idx, dest_row, gates, T, k, H, E, out, H, 1, fmt, stream);
 }
@@ -81,9 +82,9 @@ extern "C" int fmsb_moe_local_fwd(const void* x, long long ldx, const int* idx, 
 // [E, H, I], dw2 [E, I, H] (all or none null); dgate [T, k]; dx [T, H].
 extern "C" int fmsb_moe_local_bwd(const void* dout, long long ldd, const int* idx, const float* gates, const int* seg_off,
                                   const int* seg_cnt, const int* dest_row, const void* Xs, void* gu, const void* Ys, long long T,
-                                  int k, int H, int I, int E, const void* w1, const void* w3, const void* w2, int act, int cap,
-                                  void* dYs, void* hs, void* dhs, void* dXs, float* dgate, void* dx, void* dw1, void* dw3,
-                                  void* dw2, int fmt, int max_ctas, int* status, cudaStream_t stream) {
+                                  int k, int H, int I, int E, const void* w1, const void* w3, long long ld13, const void* w2,
+                                  long long ld2, int act, int cap, void* dYs, void* hs, void* dhs, void* dXs, float* dgate,
+                                  void* dx, void* dw1, void* dw3, void* dw2, int fmt, int max_ctas, int* status, cudaStream_t stream) {
   FMSB_TRY(fmsb_moe_zero_pad(dYs, H, H, seg_off, seg_cnt, E, fmt, stream));
   FMSB_TRY(fmsb_moe_dispatch_dot(dout, ldd, dest_row, gates, T, k, H, Ys, H, dYs, H, dgate, fmt, stream));
   const Group g{seg_off, E, cap, fmt, max_ctas, status, stream};
@@ -92,14 +93,14 @@ extern "C" int fmsb_moe_local_bwd(const void* dout, long long ldd, const int* id
     FMSB_TRY(fmsb_glu_fwd(gu16, gu16 + I, hs, cap, I, 2LL * I, 2LL * I, I, act, fmt, seg_off + E, stream));
     FMSB_TRY(g.weights(hs, I, dYs, H, dw2, I, H));
   }
-  FMSB_TRY(g.rows(dYs, H, w2, H, H, 0, nullptr, 0, nullptr, 0, nullptr, 0, dhs, I, I));
+  FMSB_TRY(g.rows(dYs, H, w2, ld2, H, 0, nullptr, 0, nullptr, 0, nullptr, 0, 0, dhs, I, I));
   FMSB_TRY(fmsb_glu_bwd(dhs, gu16, gu16 + I, gu16, gu16 + I, nullptr, cap, I, I, 2LL * I, 2LL * I, 2LL * I, 2LL * I, 0, act, fmt,
                         seg_off + E, stream));
   if (dw2 != nullptr) {
     FMSB_TRY(g.weights(Xs, H, gu16, 2LL * I, dw1, H, I));
     FMSB_TRY(g.weights(Xs, H, gu16 + I, 2LL * I, dw3, H, I));
   }
-  FMSB_TRY(g.rows(gu16, 2LL * I, w1, I, I, 0, nullptr, 0, gu16 + I, 2LL * I, w3, I, dXs, H, H));
+  FMSB_TRY(g.rows(gu16, 2LL * I, w1, ld13, I, 0, nullptr, 0, gu16 + I, 2LL * I, w3, ld13, I, dXs, H, H));
   void* xs[1] = {dXs};
   return fmsb_moe_combine(xs, H, idx, dest_row, nullptr, T, k, H, E, dx, H, 1, fmt, stream);
 }

@@ -47,8 +47,8 @@ N.declare("fmsb_moe_dispatch", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_zero_pad", [P, L, I, P, P, I, I, P])
 N.declare("fmsb_moe_combine", [P, L, P, P, P, L, I, I, I, P, L, I, I, P])
 N.declare("fmsb_moe_gate_grad", [P, L, P, P, P, L, L, I, I, I, P, I, I, P])
-N.declare("fmsb_moe_local_fwd", [P, L, P, P, L, I, I, I, I, P, P, P, I, P, P, P, P, I, P, P, P, P, P, P, P, I, I, P, P])
-N.declare("fmsb_moe_local_bwd", [P, L, P, P, P, P, P, P, P, P, L, I, I, I, I, P, P, P, I, I, P, P, P, P, P, P, P, P, P, I, I, P, P])
+N.declare("fmsb_moe_local_fwd", [P, L, P, P, L, I, I, I, I, P, P, L, P, L, I, P, P, P, P, I, P, P, P, P, P, P, P, I, I, P, P])
+N.declare("fmsb_moe_local_bwd", [P, L, P, P, P, P, P, P, P, P, L, I, I, I, I, P, P, L, P, L, I, I, P, P, P, P, P, P, P, P, P, I, I, P, P])
 N.declare("fmsb_moe_dispatch_dot", [P, L, P, P, L, I, I, P, L, P, L, P, I, P])
 N.declare("fmsb_moe_rowdot_scale", [P, L, P, L, P, P, P, I, I, I, I, P])
 N.declare("fmsb_moe_gather_scalar", [P, P, P, L, I, P, I, P])
@@ -468,6 +468,16 @@ def _weight_grads(mctx, acc, w1, w3, w2, needs):
     return dw1, dw3, dw2
 
 
+def _weight_rows(w1, w3, w2, E, H, I_):
+    """The expert weights as rows ``[E * in, out]`` of unit stride, w1's and w3's equally far apart (the grouped kernel reads
+    both with one leading dimension).  Rows may lie in a wider tensor (the halves of a merged gate|up weight); only what
+    has neither form is copied."""
+    r1, r3, r2 = w1.view(E * H, I_), w3.view(E * H, I_), w2.view(E * I_, H)
+    if r1.stride() != r3.stride():
+        r1, r3 = r1.contiguous(), r3.contiguous()
+    return tuple(r if r.stride(1) == 1 else r.contiguous() for r in (r1, r3, r2))
+
+
 def _local_fwd(mctx, x, gates, idx, w1, w3, w2, act, cap):
     """Forward of :class:`_Experts` without low-rank factors, all launches in one native call (``csrc/moe_local.cu``)."""
     T, H = x.shape
@@ -479,11 +489,12 @@ def _local_fwd(mctx, x, gates, idx, w1, w3, w2, act, cap):
     Xs, Ys = torch.empty(cap, H, dtype=dt, device=dev), torch.empty(cap, H, dtype=dt, device=dev)
     gu, hs = torch.empty(cap, 2 * I_, dtype=dt, device=dev), torch.empty(cap, I_, dtype=dt, device=dev)
     out = torch.empty(T, H, dtype=dt, device=dev)
+    r1, r3, r2 = _weight_rows(w1, w3, w2, E, H, I_)
     rc = N.lib().fmsb_moe_local_fwd(x.data_ptr(), x.stride(0), idx.data_ptr(), gates.data_ptr(), T, k, H, I_, E,
-                                    w1.view(E * H, I_).data_ptr(), w3.view(E * H, I_).data_ptr(),
-                                    w2.view(E * I_, H).data_ptr(), ACT.ACT_CODES[act], ws.data_ptr(), seg_off.data_ptr(),
-                                    seg_cnt.data_ptr(), dest_row.data_ptr(), cap, Xs.data_ptr(), gu.data_ptr(),
-                                    hs.data_ptr(), Ys.data_ptr(), out.data_ptr(), MoEContext.needed_counter(dev).data_ptr(),
+                                    r1.data_ptr(), r3.data_ptr(), r1.stride(0), r2.data_ptr(), r2.stride(0),
+                                    ACT.ACT_CODES[act], ws.data_ptr(), seg_off.data_ptr(), seg_cnt.data_ptr(),
+                                    dest_row.data_ptr(), cap, Xs.data_ptr(), gu.data_ptr(), hs.data_ptr(), Ys.data_ptr(),
+                                    out.data_ptr(), MoEContext.needed_counter(dev).data_ptr(),
                                     _counter(_overflow, dev).data_ptr(), N.dtype_code(dt), mctx.gemm_ctas,
                                     N.status_word(dev).data_ptr(), N.stream_ptr())
     N.check(rc, "fmsb_moe_local_fwd")
@@ -503,10 +514,11 @@ def _local_bwd(mctx, dout, gates, idx, w1, w3, w2, act, seg_off, seg_cnt, dest_r
     dx = torch.empty(T, H, dtype=dt, device=dev)
     dws = tuple(torch.empty(w.shape, dtype=w.dtype, device=dev) for w in (w1, w3, w2)) if need_dw else (None,) * 3
     gates_c = gates.contiguous()
+    r1, r3, r2 = _weight_rows(w1, w3, w2, E, H, I_)
     rc = N.lib().fmsb_moe_local_bwd(dout.data_ptr(), dout.stride(0), idx.data_ptr(), gates_c.data_ptr(), seg_off.data_ptr(),
                                     seg_cnt.data_ptr(), dest_row.data_ptr(), Xs.data_ptr(), gu.data_ptr(), Ys.data_ptr(), T, k,
-                                    H, I_, E, w1.view(E * H, I_).data_ptr(), w3.view(E * H, I_).data_ptr(),
-                                    w2.view(E * I_, H).data_ptr(), ACT.ACT_CODES[act], cap, dYs.data_ptr(), N.ptr(hs),
+                                    H, I_, E, r1.data_ptr(), r3.data_ptr(), r1.stride(0), r2.data_ptr(), r2.stride(0),
+                                    ACT.ACT_CODES[act], cap, dYs.data_ptr(), N.ptr(hs),
                                     dhs.data_ptr(), dXs.data_ptr(), dgate.data_ptr(), dx.data_ptr(), N.ptr(dws[0]),
                                     N.ptr(dws[1]), N.ptr(dws[2]), N.dtype_code(dt), mctx.gemm_ctas,
                                     N.status_word(dev).data_ptr(), N.stream_ptr())

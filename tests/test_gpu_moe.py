@@ -254,3 +254,35 @@ def test_grouped_weight_gradients_store_whole_and_ragged_tiles(m, n, dtype):
         s, e = int(seg_off[g]), int(seg_off[g + 1])
         ref = a[s:e].double().t() @ b[s:e].double()
         assert (out[g].double() - ref).abs().max() <= ulp * ref.abs().max().clamp(min=1e-9)
+
+
+@pytest.mark.parametrize("form", ["merged gate|up", "rows of different lengths", "every second column"])
+def test_expert_weights_whose_rows_lie_in_a_wider_tensor(form):
+    """Weights that are views with rows further apart than they are long give the bits of their dense copies, forward and
+    every gradient."""
+    torch.manual_seed(5)
+    T, H, I, E, k = 300, 256, 128, 8, 2
+    x, dy = (torch.randn(T, H, device=DEV).bfloat16() for _ in range(2))
+    gates, idx = torch.rand(T, k, device=DEV), torch.randint(0, E, (T, k), device=DEV, dtype=torch.int32)
+    wide = (torch.randn(3, E, max(H, I), 4 * H, device=DEV) * 0.05).bfloat16()
+    if form == "merged gate|up":
+        w1, w3 = wide[0, :, :H, :2 * I].contiguous().split(I, dim=2)
+        w2 = wide[2, :, :I, : H + 64].contiguous()[..., :H]
+    elif form == "rows of different lengths":
+        w1, w3 = wide[0, :, :H, : I + 8].contiguous()[..., :I], wide[1, :, :H, : I + 16].contiguous()[..., 8: I + 8]
+        w2 = wide[2, :, :I, :H].contiguous()
+    else:
+        w1, w3, w2 = wide[0, :, :H, : 2 * I].contiguous()[..., ::2], wide[1, :, :H, : 2 * I].contiguous()[..., ::2], \
+            wide[2, :, :I, : 2 * H].contiguous()[..., ::2]
+    mctx = MOE.MoEContext(H, I, E, k)
+
+    def run(*ws):
+        t = [v.detach().requires_grad_() for v in (x, gates) + ws]
+        y = MOE.experts_forward(t[0], t[1], idx, *t[2:], mctx)
+        return [y] + list(torch.autograd.grad(y, t, dy))
+
+    assert not w1.is_contiguous() and not w3.is_contiguous()
+    got, want = run(w1, w3, w2), run(w1.contiguous(), w3.contiguous(), w2.contiguous())
+    NV.check_status()
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), i
