@@ -174,9 +174,17 @@ class _FusedLinearCE(torch.autograd.Function):
 N.declare("fmsb_scale_cast", [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p])
 
 
+def _readable(t) -> bool:
+    """Whether a kernel may read ``t`` by address: a plain tensor, not one that stands for a batch of them (``is_grads_batched``,
+    ``torch.func.vmap``) or is being traced, and nothing that the graph of a higher derivative has to record."""
+    return (type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and not torch._C._functorch.is_legacy_batchedtensor(t) and not (t.requires_grad and torch.is_grad_enabled()))
+
+
 def _scaled_cast(src, factor, dtype):
-    """``(src * factor).to(dtype)`` for a dense fp32 ``src`` and a device scalar, in one pass."""
-    if dtype not in (torch.bfloat16, torch.float16) or factor.dtype != torch.float32 or not src.is_contiguous():
+    """``(src * factor).to(dtype)`` for a dense fp32 ``src`` and a device scalar, in one pass where a kernel may read both."""
+    if (dtype not in (torch.bfloat16, torch.float16) or factor.dtype != torch.float32 or not src.is_contiguous()
+            or not src.is_cuda or not _readable(factor)):
         return (src * factor).to(dtype)
     out = torch.empty(src.shape, dtype=dtype, device=src.device)
     rc = N.lib().fmsb_scale_cast(src.data_ptr(), factor.data_ptr(), out.data_ptr(), src.numel(), N.dtype_code(dtype),

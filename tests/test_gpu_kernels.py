@@ -624,3 +624,20 @@ def test_lora_factors_pack_and_unpack_like_the_torch_form(outs, ranks, inp, dtyp
                 continue
             assert torch.equal(g[0], da[sl[0]:sl[1]].to(dtype))
             assert torch.equal(g[1], (db[o0:o1, sl[0]:sl[1]] * sl[2]).to(dtype))
+
+
+def test_fused_linear_ce_gradients_in_a_batch_and_on_the_graph():
+    """Both gradients for a batch of incoming gradients, and recorded for a second derivative with respect to that one."""
+    torch.manual_seed(0)
+    x, w = (torch.randn(n, 256, device=DEV).bfloat16().requires_grad_() for n in (64, 1000))
+    loss = CE.fused_linear_cross_entropy(x, w, torch.randint(0, 1000, (64,), device=DEV))
+    one = torch.autograd.grad(loss, [x, w], retain_graph=True)
+    two = torch.autograd.grad(loss, [x, w], torch.tensor([1.0, 2.0], device=DEV), is_grads_batched=True, retain_graph=True)
+    for a, b in zip(one, two):
+        assert torch.equal(b[0], a) and torch.equal(b[1], 2 * a)
+    s = torch.ones((), device=DEV, requires_grad=True)
+    again = torch.autograd.grad(loss, [x, w], s, create_graph=True)
+    NV.check_status()
+    for a, b in zip(one, again):
+        (ds,) = torch.autograd.grad((b.float() * a.float()).sum(), s, retain_graph=True)
+        assert torch.equal(b, a) and abs(ds.item() / (a.float() ** 2).sum().item() - 1) < 2e-2  # 16-bit products

@@ -137,3 +137,38 @@ def test_fused_scan_takes_only_vectors_it_may_read_by_address():
                 dict(A=torch.zeros(1)), dict(A=torch.zeros(())), dict(A=torch.zeros(5)), dict(D=torch.zeros(1)),
                 dict(dt=dt.to("meta")), dict(A=A.to("meta")), dict(D=D.to("meta"))):
         assert not _fused_vectors_ok(**{**dict(x=x, dt=dt, A=A, D=D), **bad}), bad
+
+
+def test_scaled_cast_leaves_batched_and_recorded_factors_to_tensor_operators():
+    """The gradient of the fused head scales by the incoming gradient; a batch of those, one under ``torch.func``, one that a
+    second derivative needs and a fake one cannot be read by address."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from fms_acceleration_b200.ops.cross_entropy import _readable, _scaled_cast
+
+    src, seen = torch.randn(4, 8), []
+
+    class Scale(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, w):
+            return w.sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            seen.append(_readable(g))
+            return _scaled_cast(src, g, torch.float32)
+
+    w = torch.randn(4, 8, requires_grad=True)
+    loss = Scale.apply(w)
+    (one,) = torch.autograd.grad(loss, w, torch.tensor(2.0), retain_graph=True)
+    (two,) = torch.autograd.grad(loss, w, torch.tensor([1.0, 3.0]), is_grads_batched=True, retain_graph=True)
+    s = torch.tensor(2.0, requires_grad=True)
+    (three,) = torch.autograd.grad(loss, w, s, create_graph=True)
+    assert seen == [True, False, False]
+    assert torch.equal(one, 2 * src) and torch.equal(two, torch.stack([src, 3 * src]))
+    assert torch.allclose(torch.autograd.grad(three.sum(), s)[0], src.sum())
+    torch.func.vmap(lambda g: (seen.append(_readable(g)), g)[1])(torch.ones(2))
+    with FakeTensorMode():
+        seen.append(_readable(torch.ones(())))
+    assert seen[3:] == [False, False] and _readable(torch.ones(()))
