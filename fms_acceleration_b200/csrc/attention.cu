@@ -18,6 +18,7 @@ namespace fmsb {
 constexpr int ATT_BQ = 128;
 constexpr int ATT_BK = 128;
 constexpr float kMasked = -1e30f;  // score of a key outside the row's range
+constexpr float kMinScale = 1e-25f;
 
 struct AttnParams {
   int T, nh, nkv, d;
@@ -429,6 +430,10 @@ extern "C" int fmsb_attn_fwd(const void* q, long long ldq, const void* k, long l
   if ((rc = make_tmap_2d_16b(&tk, k, T, (uint64_t)nkv * d, ldk, 128, 64))) return rc;
   if ((rc = make_tmap_2d_16b(&tv, v, T, (uint64_t)nkv * d, ldv, 128, 64))) return rc;
   AttnParams p;
+  // A masked score becomes exp2(kMasked * scale * log2(e) - ...) = 0, which takes a scale that leaves kMasked far from 0.  A
+  // smaller one (0: every key of a row weighs the same) is raised to 1e-25: products of scores up to 1e17 with it are below
+  // half an ulp of 1 in the exponential, so the result is that of the scale asked for.
+  if (scale >= 0.f && scale < kMinScale) scale = kMinScale;
   p.T = T; p.nh = nh; p.nkv = nkv; p.d = d; p.scale = scale;
   p.doc_start = doc_start; p.doc_end = doc_end;
   p.o = o; p.ldo = ldo; p.lse = lse; p.fmt = fmt; p.status = status;

@@ -153,3 +153,23 @@ def test_doc_bounds_from_position_ids_equal_the_host_form(lens, lead, dtype):
     ds, de = AT.doc_bounds_from_cu_seqlens(cu, pos.numel())
     assert torch.equal(got[0].cpu(), pos.to(torch.int32))
     assert torch.equal(got[1].cpu(), ds) and torch.equal(got[2].cpu(), de)
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-30, 3e-25, 1e-3])
+@pytest.mark.parametrize("d", [128, 64])
+def test_attention_with_a_vanishing_scale_keeps_the_mask(d, scale):
+    """Down to a scale of 0 (every key of a row weighs the same) no masked key has a weight: scores, outputs and the
+    gradient of the values against fp32.  Tolerances of the other forward tests: one rounding of P and of the output."""
+    T, nh, nkv = 330, 2, 1
+    qkv, ds, de = _make(T, nh, nkv, d, [70, 1, 259], torch.bfloat16)
+    q, k, v = (t.detach().requires_grad_() for t in (qkv[:, : nh * d].view(T, nh, d), qkv[:, nh * d: (nh + 1) * d].view(T, 1, d),
+                                                     qkv[:, (nh + 1) * d:].view(T, 1, d)))
+    o = AT._VarlenAttention.apply(q, k, v, ds, de, scale)
+    g = torch.randn_like(o)
+    got = torch.autograd.grad(o, [q, k, v], g)
+    NV.check_status()
+    t = [x.detach().float().requires_grad_() for x in (q, k, v)]
+    ref = AT.attention_ref(*t, ds, scale)
+    want = torch.autograd.grad(ref, t, g.float())
+    assert _rel(o, ref) < 1.5e-2 and _rel(got[2], want[2]) < 1.5e-2
+    assert all(torch.isfinite(x).all() for x in got)
