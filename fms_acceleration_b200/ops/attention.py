@@ -36,23 +36,24 @@ def cu_seqlens_from_position_ids(position_ids: torch.Tensor) -> torch.Tensor:
     return torch.cat([starts, end]).to(torch.int32)
 
 
-N.declare("fmsb_doc_bounds", [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
-                              ctypes.c_void_p])
+N.declare("fmsb_doc_bounds", [ctypes.c_void_p, ctypes.c_int] + [ctypes.c_void_p] * 4 + [ctypes.c_int, ctypes.c_void_p])
 
 
 def doc_bounds_from_position_ids(position_ids: torch.Tensor):
     """(positions, doc_start, doc_end), int32 ``[T]`` each, of a flattened batch: a new document starts wherever the
-    position is 0.  One launch on a GPU, no host synchronisation."""
+    position is 0.  One native call on a GPU, no host synchronisation."""
     flat = position_ids.reshape(-1)
     T = flat.numel()
-    if not flat.is_cuda or flat.dtype not in (torch.int64, torch.int32) or T >= 1 << 31 or T == 0:
+    if not flat.is_cuda or flat.dtype not in (torch.int64, torch.int32) or T >= (1 << 31) - 1024 or T == 0:
         ds, de = doc_bounds_from_cu_seqlens(cu_seqlens_from_position_ids(flat), T)
         return flat.to(torch.int32).contiguous(), ds, de
     flat = flat.contiguous()
-    pos, ds, de = torch.empty(3, T, dtype=torch.int32, device=flat.device).unbind(0)
+    n = -(-T // 1024)
+    tiles, pos, ds, de = torch.empty(2 * n + 3 * T, dtype=torch.int32, device=flat.device).split([2 * n, T, T, T])
     rc = N.lib().fmsb_doc_bounds(flat.data_ptr(), int(flat.dtype == torch.int64), pos.data_ptr(), ds.data_ptr(),
-                                 de.data_ptr(), T, N.stream_ptr())
+                                 de.data_ptr(), tiles.data_ptr(), T, N.stream_ptr())
     N.check(rc, "fmsb_doc_bounds")
+    N.add_launches(n > 1)
     return pos, ds, de
 
 

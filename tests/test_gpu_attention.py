@@ -173,3 +173,14 @@ def test_attention_with_a_vanishing_scale_keeps_the_mask(d, scale):
     want = torch.autograd.grad(ref, t, g.float())
     assert _rel(o, ref) < 1.5e-2 and _rel(got[2], want[2]) < 1.5e-2
     assert all(torch.isfinite(x).all() for x in got)
+
+
+@pytest.mark.parametrize("lens,lead", [([9217, 4], 5), ([30000, 2], 3000), ([20000, 1, 20000], 1023), ([1, 9300], 1),
+                                       ([70000], 1024), ([], 11000), ([1100000, 5, 1050000], 0), ([1100000, 3], 1060000)])
+def test_doc_bounds_of_long_documents_and_leads(lens, lead):
+    """Documents and leads of many tiles, and (beyond 1024 tiles) of more than one step of the search over them."""
+    pos = torch.cat([torch.arange(7, 7 + lead)] + [torch.arange(n) for n in lens])
+    got = AT.doc_bounds_from_position_ids(pos.to(DEV))
+    ds, de = AT.doc_bounds_from_cu_seqlens(AT.cu_seqlens_from_position_ids(pos), pos.numel())
+    assert torch.equal(got[0].cpu(), pos.to(torch.int32))
+    assert torch.equal(got[1].cpu(), ds) and torch.equal(got[2].cpu(), de)
