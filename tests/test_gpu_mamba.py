@@ -189,6 +189,33 @@ def test_scan_broadcasts_or_refuses_per_head_vectors_of_other_shapes():
     assert _rel(y, yr) < 4 * 2.0 ** -8 and _rel(h, hr) < 4 * 2.0 ** -8
 
 
+@pytest.mark.parametrize("fn", ["_SSDScanFused", "_SSDScan"])
+def test_row_and_column_sums_of_the_decay_gradient_cancel(fn):
+    """One chunk without states, inputs at 64 positions, an output gradient at a later one: the gradient that reaches the
+    decay of position 0 is the sum of dG o G over the row minus its sum over the columns, which is 0 if both come from a G
+    with the same bits.  fp32 sums of 64 terms over dot products of 64: at most 128 * 2^-24 of the sum of their magnitudes;
+    one element of G that rounds differently shows as 2^-8 of its term, about 6e-5."""
+    T, nh, P, N = 256, 512, 64, 128
+    for seed in range(20):
+        torch.manual_seed(seed)
+        x, dy = torch.zeros(2, T, nh, P, device=DEV, dtype=torch.bfloat16).unbind(0)
+        s0 = 100 + 2 * seed
+        x[s0: s0 + 64] = torch.randn(64, nh, P, device=DEV).bfloat16()
+        dy[250] = torch.randn(nh, P, device=DEV).bfloat16()
+        dt = torch.rand(T, nh, device=DEV) * 0.09 + 0.01
+        A = -(torch.rand(nh, device=DEV) * 3 + 0.5)
+        B, C = ((torch.randn(T, 1, N, device=DEV) * 0.3).bfloat16() for _ in range(2))
+        t = [v.detach().requires_grad_() for v in (x, dt, A, B, C, torch.zeros(nh, device=DEV))]
+        y, _ = getattr(MB, fn).apply(*t, None, 256, False)
+        ddt = torch.autograd.grad(y, t, dy)[1]  # at position 0, where x is 0: the decay's share alone, times A
+        L = (dt * A).double().cumsum(0)
+        terms = (C[250, 0].double() @ B[:251, 0].double().t())[:, None] * torch.exp(L[250] - L[:251]) * dt[:251].double()
+        terms = terms * torch.einsum("hp,thp->th", dy[250].double(), x[:251].double())
+        left = (ddt[0] / A).double().abs() / terms.abs().sum(0)
+        assert left.max() < 128 * 2.0 ** -24, (seed, left.max().item())
+    NV.check_status()
+
+
 @pytest.mark.parametrize("fused", [True, False])
 def test_states_at_any_offset_of_their_buffer(fused):
     """An entering state and a gradient of the final state that are dense fp32 views one element into their buffers give the
