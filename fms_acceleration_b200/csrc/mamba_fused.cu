@@ -88,16 +88,24 @@ struct HeadScalars {
   float rf[CQ];        // as row t: exp(L_t - ref_t)
   float ref[CQ / 8];   // L of every eighth position
   int ok[8];
+  unsigned zero[8];    // MODE 2: one bit per position with dt = 0
 };
 
-template <bool ROWS>
+// MODE 2 takes 1 for a step size of 0.  ddt is the derivative of products with dt by dt, taken as the product over dt: where
+// dt is 0 the products without it are that derivative, and everything else leaves such a position out (`zero`).
+template <int MODE>
 __device__ __forceinline__ void publish(HeadScalars& hs, int i, float L, float d) {
   const int lane = i & 31;
+  if (MODE == 2) {
+    const unsigned zero = __ballot_sync(0xffffffffu, d == 0.f);
+    if (lane == 0) hs.zero[i >> 5] = zero;
+    if (d == 0.f) d = 1.f;
+  }
   const float ref = __shfl_sync(0xffffffffu, L, lane & ~7), last = __shfl_sync(0xffffffffu, L, lane | 7);
   hs.L[i] = L;
   hs.d[i] = d;
   hs.cf[i] = __expf(ref - L) * d;
-  if (ROWS) hs.rf[i] = __expf(L - ref);
+  if (MODE <= 2) hs.rf[i] = __expf(L - ref);
   if ((lane & 7) == 0) hs.ref[i >> 3] = L;
   const int ok = __all_sync(0xffffffffu, fabsf(ref - last) < kSplitLimit);
   if (lane == 0) hs.ok[i >> 5] = ok;
@@ -369,6 +377,7 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
         // weight of the second product: exp(L_t) for rows t, w_s for rows s
         const float ew = MODE == 2 ? __expf(q.L[CQ - 1] - Lrow) * q.d[pos] : __expf(Lrow);
         const float dh = MODE == 1 ? 0.f : p.D[h];
+        const bool still = MODE == 2 && ((q.zero[pos >> 5] >> lane) & 1u) != 0;  // dt = 0: the row gets D dy alone
         uint32_t ra[16], ri[16];
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
@@ -401,6 +410,14 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
                 d1 += i0 * x0 + i1 * x1;
                 d2 += a0 * x0 + a1 * x1;
               }
+            }
+          }
+          if (still) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float v0, v1;
+              unpack2<FMT>(vw[j], v0, v1);
+              ow[j] = pack2f<FMT>(dh * v0, dh * v1);
             }
           }
           if (MODE != 1) sts128(sE(e) + off, ow[0], ow[1], ow[2], ow[3]);
@@ -444,7 +461,7 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
         }
       }
     };
-    publish<true>(hs[0], ctid, nL, nd);
+    publish<MODE>(hs[0], ctid, nL, nd);
     if (n_heads > 1) {
       nL = Lg[CQ];
       nd = dg[CQ];
@@ -455,7 +472,7 @@ ssd_scan_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constant__
     for (int it = 0; it < n_heads; ++it) {
       const bool more = it + 1 < n_heads;
       if (more) {
-        publish<true>(hs[(it + 1) % 3], ctid, nL, nd);
+        publish<MODE>(hs[(it + 1) % 3], ctid, nL, nd);
         if (it + 2 < n_heads) {
           nL = Lg[(it + 2) * CQ];
           nd = dg[(it + 2) * CQ];
@@ -755,7 +772,7 @@ ssd_dcb_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__
     for (int it = 0; it < n_heads; ++it) {
       const int b = it & 1;
       HeadScalars& q = hs[it % 3];
-      publish<false>(q, ctid, nL, nd);
+      publish<3>(q, ctid, nL, nd);
       if (it + 1 < n_heads) {
         nL = Lg[(it + 1) * CQ];
         nd = dg[(it + 1) * CQ];
@@ -904,7 +921,8 @@ __global__ void __launch_bounds__(256) ssd_decay_kernel(const float* __restrict_
 
 // Gradients through the decay.  yd = dy . (y - D x), dww = w x.(B dS^T), col = x.(G^T dy), dyx = dy . x per (chunk, head,
 // position).  dL = yd - dww - col (+ dLtot and the sum of dww at the last position); through L = cumsum(dt A) that is a
-// reverse cumulative sum da; ddt = (dww + col) / dt + da A; partial dA = sum da dt and dD = sum dyx per (chunk, head).
+// reverse cumulative sum da; ddt = (dww + col) / dt + da A; partial dA = sum da dt and dD = sum dyx per (chunk, head).  Where dt
+// is 0, dww and col come without it (see publish): they are the derivative themselves and have no part in dL.
 __global__ void __launch_bounds__(256) ssd_decay_bwd_kernel(const float* __restrict__ yd, const float* __restrict__ red,
                                                             const float* __restrict__ dtt, const float* __restrict__ A,
                                                             const float* __restrict__ dLtot, float* __restrict__ ddt,
@@ -926,9 +944,12 @@ __global__ void __launch_bounds__(256) ssd_decay_bwd_kernel(const float* __restr
     ld(red + plane + o, ww);
     ld(red + 2 * plane + o, co);
     ld(dtt + o, d);
-    float sw = 0.f, sk = 0.f;
+    float sw = 0.f, sk = 0.f, direct[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      direct[j] = ww[j] + co[j];
+      if (d[j] == 0.f) ww[j] = co[j] = 0.f;
+      else direct[j] /= d[j];
       sw += ww[j];
       sk += k[j];
     }
@@ -958,7 +979,7 @@ __global__ void __launch_bounds__(256) ssd_decay_bwd_kernel(const float* __restr
     for (int j = 0; j < 8; ++j) {
       const float da = dl[j] + after;
       sa += da * d[j];
-      sd[w][lane * 8 + j] = (ww[j] + co[j]) / d[j] + da * a;
+      sd[w][lane * 8 + j] = direct[j] + da * a;
     }
     sa = warp_sum(sa);
     if (lane == 0) {

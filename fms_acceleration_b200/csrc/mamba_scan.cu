@@ -245,7 +245,7 @@ __global__ void ssd_fwd_combine_kernel(const float* __restrict__ y_intra, const 
 }
 
 // One (t, h) row of P = 8 * vpr values per TPR lanes (TPR = power of two >= vpr, <= 32).
-//   dx      = D dy + dxw wgt + dx_intra
+//   dx      = D dy + dxw wgt + dx_intra   (without dx_intra where dt = 0: see the caller's G)
 //   red[0]  = dy . x              (dD, summed over t by the caller)
 //   red[1]  = exp(L) dy . y_inter (dL through the inter-chunk term)
 //   red[2]  = dxw . x             (d of the chunk-state weight)
@@ -255,8 +255,8 @@ template <typename T, int TPR>
 __global__ void __launch_bounds__(256) ssd_bwd_combine_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ y_inter, const float* __restrict__ dxw,
     const float* __restrict__ dx_intra, const float* __restrict__ y_intra, const float* __restrict__ L,
-    const float* __restrict__ wgt, const float* __restrict__ D, T* __restrict__ dx, float* __restrict__ red,
-    long long rows, int vpr, int nh) {
+    const float* __restrict__ wgt, const float* __restrict__ dt, const float* __restrict__ D, T* __restrict__ dx,
+    float* __restrict__ red, long long rows, int vpr, int nh) {
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long row = gt / TPR;
   const int v = (int)(gt % TPR);
@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(256) ssd_bwd_combine_kernel(
   if (live) {
     const long long off = (row * vpr + v) * 8;
     const float d = D[(int)(row % nh)], w = wgt[row];
+    const bool moves = dt[row] != 0.f;
     float dyv[8], xv[8], yi[8], xw[8], di[8], ya[8], o[8];
     unpack8<T>(*reinterpret_cast<const uint4*>(dy + off), dyv);
     unpack8<T>(*reinterpret_cast<const uint4*>(x + off), xv);
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(256) ssd_bwd_combine_kernel(
     ld8f(y_intra + off, ya);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      o[j] = d * dyv[j] + xw[j] * w + di[j];
+      o[j] = d * dyv[j] + xw[j] * w + (moves ? di[j] : 0.f);
       s0 += dyv[j] * xv[j];
       s1 += dyv[j] * yi[j];
       s2 += xw[j] * xv[j];
@@ -407,7 +408,7 @@ extern "C" int fmsb_ssd_fwd_combine(const float* y_intra, const float* y_inter, 
 
 template <typename T>
 static int launch_bwd_combine(const void* dy, const void* x, const float* y_inter, const float* dxw,
-                              const float* dx_intra, const float* y_intra, const float* L, const float* wgt,
+                              const float* dx_intra, const float* y_intra, const float* L, const float* wgt, const float* dt,
                               const float* D, void* dx, float* red, long long rows, int P, int nh, cudaStream_t stream) {
   const int vpr = P / 8;
   int tpr = 1;
@@ -418,7 +419,7 @@ static int launch_bwd_combine(const void* dy, const void* x, const float* y_inte
 #define FMSB_BC(TPR_)                                                                                              \
   case TPR_:                                                                                                       \
     ssd_bwd_combine_kernel<T, TPR_><<<blocks, 256, 0, stream>>>((const T*)dy, (const T*)x, y_inter, dxw, dx_intra, \
-                                                                y_intra, L, wgt, D, (T*)dx, red, rows, vpr, nh);   \
+                                                                y_intra, L, wgt, dt, D, (T*)dx, red, rows, vpr, nh); \
     break;
   switch (tpr) {
     FMSB_BC(1) FMSB_BC(2) FMSB_BC(4) FMSB_BC(8) FMSB_BC(16) FMSB_BC(32)
@@ -430,14 +431,14 @@ static int launch_bwd_combine(const void* dy, const void* x, const float* y_inte
 
 extern "C" int fmsb_ssd_bwd_combine(const void* dy, const void* x, const float* y_inter, const float* dxw,
                                     const float* dx_intra, const float* y_intra, const float* L, const float* wgt,
-                                    const float* D, void* dx, float* red, long long rows, int P, int nh, int dtype,
-                                    cudaStream_t stream) {
+                                    const float* dt, const float* D, void* dx, float* red, long long rows, int P, int nh,
+                                    int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (P % 8 != 0) return -2;
   if (dtype == 1)
-    return launch_bwd_combine<__nv_bfloat16>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, D, dx, red, rows, P, nh, stream);
+    return launch_bwd_combine<__nv_bfloat16>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, dt, D, dx, red, rows, P, nh, stream);
   if (dtype == 0)
-    return launch_bwd_combine<__half>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, D, dx, red, rows, P, nh, stream);
+    return launch_bwd_combine<__half>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, dt, D, dx, red, rows, P, nh, stream);
   return -2;
 }
 

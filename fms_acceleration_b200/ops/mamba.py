@@ -29,7 +29,7 @@ NV.declare("fmsb_ssd_rowscale", [P_, P_, P_, L_, I_, I_, P_])
 NV.declare("fmsb_ssd_fwd_combine", [P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_addscaled", [P_, P_, P_, P_, L_, I_, I_, P_])
 NV.declare("fmsb_ssd_rowdot", [P_, P_, P_, P_, L_, I_, I_, P_])
-NV.declare("fmsb_ssd_bwd_combine", [P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
+NV.declare("fmsb_ssd_bwd_combine", [P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_fwd", [P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_bwd", [P_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssdf_heads", [I_, I_, I_, I_])
@@ -370,15 +370,20 @@ class _SSDScan(torch.autograd.Function):
         del xw, dS16
         # ---- intra-chunk term  y += G X,  G = CB o exp(L_t - L_s) dt_s (s <= t); slabs of chunks bound the
         # [chunks, heads, Q, Q] temporaries
+        # ddt is a product with dt over dt; where dt is 0, this G and dx_intra go without it (the product without it is the
+        # derivative) and everything else leaves the position out: x in G X, dx_intra in dx, col in dL
+        still = (dt == 0).view(T, nh)
+        dtg = _chunk_major(dt.view(T, nh).masked_fill(still, 1.0), nc, Q, nh)
+        xg = x2.view(T, nh, P).masked_fill(still[:, :, None], 0.0).view(T, nh * P)
         dx_intra = torch.empty(T, nh * P, dtype=torch.float32, device=dev)
         y_intra = torch.empty(T, nh * P, dtype=torch.float32, device=dev)
         for c0, c1 in _slabs(nc, nh, Q):
             n = c1 - c0
             rows = slice(c0 * Q, c1 * Q)
-            g = _make_g(cb[c0 * G * Q: c1 * G * Q], Lt[c0:c1], dtt[c0:c1], n, nh, G, Q)
+            g = _make_g(cb[c0 * G * Q: c1 * G * Q], Lt[c0:c1], dtg[c0:c1], n, nh, G, Q)
             batched_gemm(g, dy2[rows], M=Q, N=P, K=Q, n_batch=n * nh, n_inner=nh, a_off=(nh * Q, Q, 0, 1),
                          b_off=(Q, 0, P, 1), d_off=(Q, 0, P), a_mn=True, b_mn=True, out=dx_intra[rows])
-            batched_gemm(g, x2[rows], M=Q, N=P, K=Q, n_batch=n * nh, n_inner=nh, a_off=(nh * Q, Q, 0, 1),
+            batched_gemm(g, xg[rows], M=Q, N=P, K=Q, n_batch=n * nh, n_inner=nh, a_off=(nh * Q, Q, 0, 1),
                          b_off=(Q, 0, P, 1), d_off=(Q, 0, P), b_mn=True, out=y_intra[rows])
             del g
             dG = batched_gemm(dy2[rows], x2[rows], M=Q, N=Q, K=P, n_batch=n * nh, n_inner=nh, a_off=(Q, 0, P, 1),
@@ -402,15 +407,16 @@ class _SSDScan(torch.autograd.Function):
         Df = D.float().contiguous()
         rc = NV.lib().fmsb_ssd_bwd_combine(dy2.data_ptr(), x2.data_ptr(), y_inter.data_ptr(), dxw.data_ptr(),
                                            dx_intra.data_ptr(), y_intra.data_ptr(), L.data_ptr(), wgt.data_ptr(),
-                                           Df.data_ptr(), dx.data_ptr(), red.data_ptr(), T * nh, P, nh, code,
+                                           dt.data_ptr(), Df.data_ptr(), dx.data_ptr(), red.data_ptr(), T * nh, P, nh, code,
                                            NV.stream_ptr())
         NV.check(rc, "fmsb_ssd_bwd_combine")
         del y_inter, dxw, dx_intra, y_intra
         dD = red[0].sum(0)
         dww = red[2] * wgt                                                    # through w = exp(Ltot - L) dt
         row, col = red[3], red[4]                                             # sums of dG o G over s / over t
-        dL = red[1] - dww + row - col
-        ddt = (dww + col) / dt
+        w1 = torch.exp(Ltot.view(nc, 1, nh) - L.view(nc, Q, nh)).view(T, nh)  # w without dt
+        ddt = torch.where(still, red[2] * w1 + col, (dww + col) / dt)
+        dL = red[1] - dww + row - col.masked_fill(still, 0.0)
         dLtot = dLtot + dww.view(nc, Q, nh).sum(1)
         # ---- through L = cumsum(dt A) within the chunk, Ltot = L[last]: a reverse cumulative sum per chunk
         dLt = _chunk_major(dL, nc, Q, nh)

@@ -189,6 +189,37 @@ def test_scan_broadcasts_or_refuses_per_head_vectors_of_other_shapes():
     assert _rel(y, yr) < 4 * 2.0 ** -8 and _rel(h, hr) < 4 * 2.0 ** -8
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("fn", ["_SSDScanFused", "_SSDScan"])
+def test_step_sizes_of_zero_have_finite_gradients(fn, dtype):
+    """Step sizes that are exactly 0 (padded positions, a softplus that underflows): all heads at some positions, one head
+    over a range, one head everywhere.  Every gradient against the fp64 recurrence, within the bound of
+    test_fused_scan_matches_recurrence_and_general_path."""
+    torch.manual_seed(8)
+    nc, nh, P, N, Q = 2, 4, 64, 128, 256
+    T = nc * Q
+    dt = torch.rand(T, nh, device=DEV) * 0.09 + 0.01
+    dt[[0, 10, 127, 128, 255, 256, T - 1]] = 0
+    dt[300:340, 2] = 0
+    dt[:, 3] = 0
+    ins = [(torch.randn(T, nh, P, device=DEV) * 0.5).to(dtype), dt, -(torch.rand(nh, device=DEV) * 3 + 0.5),
+           (torch.randn(T, 1, N, device=DEV) * 0.3).to(dtype), (torch.randn(T, 1, N, device=DEV) * 0.3).to(dtype),
+           torch.randn(nh, device=DEV), torch.randn(nh, P, N, device=DEV) * 0.2]
+    gy, gh = torch.randn(T, nh, P, device=DEV).to(dtype), torch.randn(nh, P, N, device=DEV) * 0.1
+
+    t = [v.detach().requires_grad_() for v in ins]
+    got = torch.autograd.grad(getattr(MB, fn).apply(*t, Q, False), t, [gy, gh])
+    NV.check_status()
+    t = [v.detach().double().cpu().requires_grad_() for v in ins]
+    want = torch.autograd.grad(MB.ssd_ref(*t), t, [gy.double().cpu(), gh.double().cpu()])
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.isfinite(a.float()).all(), i
+        assert _rel(a.cpu(), b) < 4 * ulp, (i, _rel(a.cpu(), b))
+    zero = (dt == 0).cpu()  # the positions themselves, which the norm over all of them could hide
+    assert _rel(got[1].cpu()[zero], want[1][zero]) < 4 * ulp and _rel(got[0].cpu()[zero], want[0][zero]) < 4 * ulp
+
+
 @pytest.mark.parametrize("fn", ["_SSDScanFused", "_SSDScan"])
 def test_row_and_column_sums_of_the_decay_gradient_cancel(fn):
     """One chunk without states, inputs at 64 positions, an output gradient at a later one: the gradient that reaches the
