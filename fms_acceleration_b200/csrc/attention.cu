@@ -10,7 +10,7 @@
 // o [T, nh*d], lse [nh, T] fp32 (natural log).  d in {64, 128}.
 //
 // This file holds the forward kernel (two query tiles per CTA, see below) and the delta = rowsum(dO*O)
-// kernel; the backward kernels live in attention_bwd3.cu (in use) and attention_bwd.cu (cross-check).
+// kernel; the backward kernels live in attention_bwd3.cu.
 #include "common.cuh"
 
 namespace fmsb {

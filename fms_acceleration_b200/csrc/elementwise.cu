@@ -594,7 +594,6 @@ glu_bwd_kernel(const T* __restrict__ dh, const T* e, const T* g, T* de, T* dg, T
   }
 }
 
-// y = a + b (residual add), 16-bit
 // out (16-bit) = src (fp32) * *factor: the gradient of a weight that was accumulated in fp32, scaled and rounded in one pass
 // (a broadcast product and a cast, each a pass of its own, took 262 us for 75.5 M elements; 450 MB are 68 us).
 template <typename T>
@@ -610,6 +609,7 @@ __global__ void __launch_bounds__(256) scale_cast_kernel(const float* __restrict
   for (long long i = n8 * 8 + i0; i < n; i += stride) out[i] = (T)(src[i] * f);
 }
 
+// y = a + b (residual add), 16-bit
 template <typename T>
 __global__ void add_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long n8) {
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n8;

@@ -28,8 +28,11 @@
 // of the FSDP-sharded packed parameter that precedes them.
 //
 // Roles (320 threads): warp 0 TMA producer (x, and xa/Bl for the LoRA blocks), warp 1 MMA issuer,
-// warps 2-9 dequantise W tiles and afterwards run the epilogue.  6- or 8-stage ring.  77 x 14336 x 4096: 95.8 -> 66.6 us
-// without the per-block 64-bit divisions and with the tile width chosen by turns of the machine.  Every wait is bounded.
+// warps 2-9 dequantise W tiles and afterwards run the epilogue.  6- or 8-stage ring.  Every wait is bounded.
+//
+// This first kernel serves peers' shards, a LoRA pair, fp32 block scales and GPTQ weights (77 x 14336 x 4096, one shard: 95.8 ->
+// 66.6 us without the per-block 64-bit divisions and with the tile width chosen by turns of the machine).  A plain local
+// weight goes to gemm_q4_tma_kernel (double-quantised) or, up to four rows, to q4_rows_kernel.
 #include "common.cuh"
 
 namespace fmsb {

@@ -443,7 +443,9 @@ __global__ void __launch_bounds__(256) moe_dispatch_dot_kernel(const T* __restri
   }
   const T* src = dout + t * ldd;
   const int nvec = H >> 3;
-  constexpr int NV = 6;  // 1536 columns a pass
+  // 1536 columns a pass: the dout row, a row of y and the next one take 72 registers.  A width that is no multiple leaves lanes
+  // idle in its last pass only.
+  constexpr int NV = 6;
   for (int v0 = 0; v0 < nvec; v0 += 32 * NV) {
     uint4 d[NV];
 #pragma unroll
