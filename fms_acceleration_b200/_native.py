@@ -224,4 +224,3 @@ class StatusMonitor:
             raise NativeError(f"device status {v}: {_STATUS_NAMES.get(v, 'unknown')} (reported by an earlier step)")
 
 declare("fmsb_attn_fwd", [P, L, P, L, P, L, P, L, P, P, P, I, I, I, I, F, I, P, P])
-declare("fmsb_attn_delta", [P, P, L, L, P, I, I, I, I, P])

@@ -10,7 +10,8 @@
 // reaches into a tile and the one that ends it from those notes, 1024 tiles a step, and the rest within the tile.  Tokens
 // before the first 0 also need the start after it: the CTA looks for that one too, once.  Searching the positions
 // themselves, tile by tile, and letting every token before the first 0 walk through the next document by itself took
-// 5629 us for 1000 such tokens before a document of 64536 and 2458 us for one document of 2^20 tokens; this form 38 and 117 us (a call, host included).
+// 5629 us for 1000 such tokens before a document of 64536 and 2458 us for one document of 2^20 tokens; this form 38 and
+// 117 us (a call, host included).
 #include "common.cuh"
 
 namespace fmsb {

@@ -324,8 +324,9 @@ gemm_q4_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 // four warps take K blocks in turn, a thread expands a longer piece of a row (64 values at 128 wide) and nothing is
 // outstanding when it fences: the packed bytes come in by TMA (a W stage is [BN rows x 128 bytes] = four K blocks,
 // 128-byte swizzle) and the 8-bit scale codes of the tile (BN * K / 64 bytes) are copied to shared memory once.
-// 77 x 14336 x 4096: 66.6 -> 37.7 us, 77 x 4096 x 4096 (32 wide): 30.8 -> 22.7 us; what is left at 128 wide is shared memory (look-ups,
-// operand writes and the tensor core's reads: about 850 of 1000 cycles per K block).
+// 77 x 14336 x 4096: 66.6 -> 36.9 us back to back (43.0 with L2 flushed), 77 x 4096 x 4096 (32 wide): 30.8 -> 22.7 us (26.6);
+// what is left at 128 wide is shared memory (look-ups, operand writes and the tensor core's reads: about 850 of 1000 cycles
+// per K block).
 // ----------------------------------------------------------------------------------------
 constexpr int Q4T_GROUPS = 4;           // dequant groups of four warps
 constexpr int Q4T_DQ_THREADS = Q4T_GROUPS * 128;
@@ -554,8 +555,8 @@ gemm_q4_tma_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 // bytes (32 values of one scale block), looks the codes up in a 16-word shared table (conflict-free), multiplies
 // them with x in fp32 and applies the block's scale once per 32 products.  x lies in shared memory as fp32, ordered so
 // that the 16-byte reads of a warp are contiguous.  What bounds it is issue: about four instructions per weight
-// (two to extract, one look-up, one fused multiply-add).  1 x 4096 x 4096, NF4: 7.9 us against 44.5 us for the
-// tensor-core form it replaces there.
+// (two to extract, one look-up, one fused multiply-add).  1 x 4096 x 4096, NF4: 7.9 us back to back (about 12.5
+// with L2 flushed) against 44.5 us for the tensor-core form it replaces there.
 // ----------------------------------------------------------------------------------------
 constexpr int Q4V_WARPS = 8;
 

@@ -124,8 +124,9 @@ __device__ __forceinline__ bool all_ok(const HeadScalars& hs) {
 // buffer: while the tensor core works on unit w, the compute warps build G of unit w + 1, then drain unit w.
 // Tensor memory: G of the two tiles 64 + 128 columns (16-bit pairs), accumulators 2 x (64 + 64) from column 256.
 // 384 threads: warps 0 and 1 as above, 2 and 3 idle, 4-11 compute with 232 registers (C B^T is 96 of them).
-// 16384 tokens, 80 heads (one tile per CTA, 168 registers -> this): y 331 -> 144 us, dots 332 -> 141, dx 413 -> 183 us;
-// reading and writing everything once would take 63 us at the copy rate.
+// 16384 tokens, 80 heads (one tile per CTA, 168 registers -> this): y 331 -> 146 us, dots 332 -> 142, dx 413 -> 194 us (183
+// before it took the factors of the other modes and looked at rows with dt = 0); reading and writing everything once would
+// take 63 us at the copy rate.
 // ----------------------------------------------------------------------------------------
 constexpr int kScanThreads = 384;
 constexpr int kScanRegsMain = 40, kScanRegsCompute = 232;  // 128 * 40 + 256 * 232 = 384 * 168
@@ -1172,7 +1173,7 @@ extern "C" int fmsb_ssdf_decay_bwd(const float* yd, const float* red, const floa
 // ----------------------------------------------------------------------------------------
 // The launches of a whole forward and of a whole backward in one call each: from Python every launch costs the host some
 // 10 us (allocation, argument conversion, tensor maps apart), and at a few thousand tokens the kernels are shorter than that.
-// 1024 tokens, 48 heads, forward: 65 -> 45 us a pass; 4352 tokens, forward and backward: 406 -> 297 us.
+// 1024 tokens, 48 heads, forward: 65 -> 44 us a pass; 4352 tokens, forward and backward: 406 -> 299 us.
 // ----------------------------------------------------------------------------------------
 extern "C" int fmsb_ssd_state_fwd(const float*, const float*, const float*, void*, float*, int, int, int, int, cudaStream_t);
 extern "C" int fmsb_ssd_state_bwd(const float*, const float*, const float*, const void*, void*, float*, float*, int, int, int, int,
