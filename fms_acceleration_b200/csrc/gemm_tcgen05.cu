@@ -980,14 +980,16 @@ static int gemm_impl(const void* A1, long long lda1, const void* B1, long long l
   int rc;
   // CTA pairs: plain mode, 256-column tiles, and either enough 256 x 256 tiles to fill the machine about twice, or a
   // grid that takes no more turns with pairs than with single CTAs (a ragged M can cost the pairs a turn: 1111 x 4096 x
-  // 4096 40 us single, 68 us pairs) and is long enough for the pair's longer start: two turns (2048 x 4096 x 14336:
-  // 207 -> 189 us; 5376 x 1536 x 49160: 724 -> 622 us) or a contraction of 8192 (256 x 4096 x 14336: 111 -> 100 us, while
-  // 4096 x 1024 x 4096 goes from 36 to 38 us).
+  // 4096 40 us single, 68 us pairs) and a contraction that is worth the pair's longer start: 3072 over two turns or 8192 in
+  // one.  Pair / single time with operands from memory: two turns 0.84 to 1.01 from 3072 on (512 x 14336 x 3072: 0.89, 1500 x
+  // 4096 x 4096: 0.90, 5376 x 1536 x 49160: 0.70), 0.94 to 1.07 at 2048, 0.91 to 1.12 at 512 and 1024; one turn 0.83 to 0.94 at
+  // 8192 (256 x 2560: 0.87, 1000 x 4096: 0.94), while 4096 x 1024 x 4096 goes from 36 to 38 us.  Operands that are all in
+  // L2 from the call before gain less: 0.90 to 1.08 for the same shapes.
   bool use_pair = false;
   if (mode == 0 && bn == 256 && g_pair_mode != 0 && M >= 256 && N >= 256) {
     const long long t2 = (long long)((M + 255) / 256) * ((N + 255) / 256), t1 = (long long)((M + 127) / 128) * ((N + 255) / 256);
     const long long turns1 = (t1 + sm_count() - 1) / sm_count(), turns2 = (t2 + sm_count() / 2 - 1) / (sm_count() / 2);
-    use_pair = g_pair_mode == 2 || t2 >= 2LL * (sm_count() / 2) || (turns2 <= turns1 && (turns2 >= 2 || K1 + K2 >= 8192));
+    use_pair = g_pair_mode == 2 || t2 >= 2LL * (sm_count() / 2) || (turns2 <= turns1 && K1 + K2 >= (turns2 >= 2 ? 3072 : 8192));
   }
   const int b_box_rows = use_pair ? fmsb::BNH : bn;
   // a_rows / b_rows: number of rows of the stored A / B matrices when it differs from the per-tile view
