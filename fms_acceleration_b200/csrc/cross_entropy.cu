@@ -186,34 +186,33 @@ ce_kernel(T* logits, long long row_stride, const long long* __restrict__ labels,
     if (scale_ptr != nullptr) sc *= *scale_ptr;
     if (row_scale != nullptr) sc *= row_scale[row];
     const float eps_v = label_smoothing / (float)V;
-    // four vectors a trip, their loads (L2: this CTA has just read the row) in flight together; one test per vector for
-    // the label instead of a 64-bit comparison per element
+    // four vectors a trip, their loads (L2: this CTA has just read the row) in flight together, then one a trip: four guarded
+    // vectors a trip throughout were 2 to 3 % slower for every vocabulary (8192 rows of 49155: 386 -> 378 us; of 256: 76 -> 74).
+    // One test per vector for the label instead of a 64-bit comparison per element.
     const long long lv = label / n;
-    for (int v0 = threadIdx.x; v0 < nvec; v0 += CE_THREADS * U) {
+    auto put = [&](const uint4& raw, int v) {
+      const T* e = reinterpret_cast<const T*>(&raw);
+      float f[n];
+#pragma unroll
+      for (int i = 0; i < n; ++i) f[i] = __expf(ld_as_float<T>(e + i) - lse) - eps_v;
+      if (v == lv) {
+#pragma unroll
+        for (int i = 0; i < n; ++i)
+          if (i == (int)(label - lv * n)) f[i] -= (1.f - label_smoothing);
+      }
+#pragma unroll
+      for (int i = 0; i < n; ++i) f[i] *= sc;
+      store_vec<T>(x + v * n, f);
+    };
+    int v0 = threadIdx.x;
+    for (; v0 + (U - 1) * CE_THREADS < nvec; v0 += CE_THREADS * U) {
       uint4 raw[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int v = v0 + u * CE_THREADS;
-        if (v < nvec) raw[u] = *reinterpret_cast<const uint4*>(x + v * n);
-      }
+      for (int u = 0; u < U; ++u) raw[u] = *reinterpret_cast<const uint4*>(x + (v0 + u * CE_THREADS) * n);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int v = v0 + u * CE_THREADS;
-        if (v >= nvec) continue;
-        const T* e = reinterpret_cast<const T*>(&raw[u]);
-        float f[n];
-#pragma unroll
-        for (int i = 0; i < n; ++i) f[i] = __expf(ld_as_float<T>(e + i) - lse) - eps_v;
-        if (v == lv) {
-#pragma unroll
-          for (int i = 0; i < n; ++i)
-            if (i == (int)(label - lv * n)) f[i] -= (1.f - label_smoothing);
-        }
-#pragma unroll
-        for (int i = 0; i < n; ++i) f[i] *= sc;
-        store_vec<T>(x + v * n, f);
-      }
+      for (int u = 0; u < U; ++u) put(raw[u], v0 + u * CE_THREADS);
     }
+    for (; v0 < nvec; v0 += CE_THREADS) put(*reinterpret_cast<const uint4*>(x + v0 * n), v0);
     for (int i = nvec * n + threadIdx.x; i < V; i += CE_THREADS) {
       float g = __expf(ld_as_float<T>(x + i) - lse) - eps_v;
       if ((long long)i == label) g -= (1.f - label_smoothing);
