@@ -187,8 +187,8 @@ ce_kernel(T* logits, long long row_stride, const long long* __restrict__ labels,
     if (row_scale != nullptr) sc *= row_scale[row];
     const float eps_v = label_smoothing / (float)V;
     // four vectors a trip, their loads (L2: this CTA has just read the row) in flight together, then one a trip: four guarded
-    // vectors a trip throughout were 2 to 3 % slower for every vocabulary (8192 rows of 49155: 386 -> 378 us; of 256: 76 -> 74).
-    // One test per vector for the label instead of a 64-bit comparison per element.
+    // vectors a trip throughout were 2 to 3 % slower for every vocabulary (8192 rows of 49155: 386 -> 378 us; of 256: 76 -> 74),
+    // one vector a trip throughout takes 417 and 66 us.  One test per vector for the label instead of a 64-bit comparison per element.
     const long long lv = label / n;
     auto put = [&](const uint4& raw, int v) {
       const T* e = reinterpret_cast<const T*>(&raw);

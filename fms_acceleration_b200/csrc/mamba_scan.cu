@@ -245,18 +245,21 @@ __global__ void ssd_fwd_combine_kernel(const float* __restrict__ y_intra, const 
 }
 
 // One (t, h) row of P = 8 * vpr values per TPR lanes (TPR = power of two >= vpr, <= 32).
-//   dx      = D dy + dxw wgt + dx_intra   (without dx_intra where dt = 0: see the caller's G)
+//   dx      = D dy + dxw wgt + dx_intra
 //   red[0]  = dy . x              (dD, summed over t by the caller)
 //   red[1]  = exp(L) dy . y_inter (dL through the inter-chunk term)
-//   red[2]  = dxw . x             (d of the chunk-state weight)
+//   red[2]  = wgt dxw . x         (dL through the chunk-state weight wgt = exp(Ltot - L) dt)
 //   red[3]  = dy . y_intra        (row sums of dG o G)
 //   red[4]  = x . dx_intra        (column sums of dG o G)
+//   red[5]  = (red[2] + red[4]) / dt   (ddt through wgt and G, both products with dt)
+// Where dt = 0, dx_intra comes without dt (see the caller's G): red[5] is then exp(Ltot - L) dxw . x + x . dx_intra, and dx
+// and red[4] leave dx_intra out.
 template <typename T, int TPR>
 __global__ void __launch_bounds__(256) ssd_bwd_combine_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ y_inter, const float* __restrict__ dxw,
     const float* __restrict__ dx_intra, const float* __restrict__ y_intra, const float* __restrict__ L,
-    const float* __restrict__ wgt, const float* __restrict__ dt, const float* __restrict__ D, T* __restrict__ dx,
-    float* __restrict__ red, long long rows, int vpr, int nh) {
+    const float* __restrict__ Ltot, const float* __restrict__ wgt, const float* __restrict__ dt, const float* __restrict__ D,
+    T* __restrict__ dx, float* __restrict__ red, long long rows, int vpr, int nh, int Q) {
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long row = gt / TPR;
   const int v = (int)(gt % TPR);
@@ -295,9 +298,11 @@ __global__ void __launch_bounds__(256) ssd_bwd_combine_kernel(
   if (row < rows && v == 0) {
     red[row] = s0;
     red[rows + row] = __expf(L[row]) * s1;
-    red[2 * rows + row] = s2;
+    const float d = dt[row], ww = s2 * wgt[row];
+    red[2 * rows + row] = ww;
     red[3 * rows + row] = s3;
-    red[4 * rows + row] = s4;
+    red[4 * rows + row] = d != 0.f ? s4 : 0.f;
+    red[5 * rows + row] = d != 0.f ? (ww + s4) / d : s2 * __expf(Ltot[row / (nh * (long long)Q) * nh + row % nh] - L[row]) + s4;
   }
 }
 
@@ -408,8 +413,9 @@ extern "C" int fmsb_ssd_fwd_combine(const float* y_intra, const float* y_inter, 
 
 template <typename T>
 static int launch_bwd_combine(const void* dy, const void* x, const float* y_inter, const float* dxw,
-                              const float* dx_intra, const float* y_intra, const float* L, const float* wgt, const float* dt,
-                              const float* D, void* dx, float* red, long long rows, int P, int nh, cudaStream_t stream) {
+                              const float* dx_intra, const float* y_intra, const float* L, const float* Ltot,
+                              const float* wgt, const float* dt, const float* D, void* dx, float* red, long long rows, int P,
+                              int nh, int Q, cudaStream_t stream) {
   const int vpr = P / 8;
   int tpr = 1;
   while (tpr < vpr) tpr <<= 1;
@@ -419,7 +425,7 @@ static int launch_bwd_combine(const void* dy, const void* x, const float* y_inte
 #define FMSB_BC(TPR_)                                                                                              \
   case TPR_:                                                                                                       \
     ssd_bwd_combine_kernel<T, TPR_><<<blocks, 256, 0, stream>>>((const T*)dy, (const T*)x, y_inter, dxw, dx_intra, \
-                                                                y_intra, L, wgt, dt, D, (T*)dx, red, rows, vpr, nh); \
+                                                                y_intra, L, Ltot, wgt, dt, D, (T*)dx, red, rows, vpr, nh, Q); \
     break;
   switch (tpr) {
     FMSB_BC(1) FMSB_BC(2) FMSB_BC(4) FMSB_BC(8) FMSB_BC(16) FMSB_BC(32)
@@ -430,15 +436,15 @@ static int launch_bwd_combine(const void* dy, const void* x, const float* y_inte
 }
 
 extern "C" int fmsb_ssd_bwd_combine(const void* dy, const void* x, const float* y_inter, const float* dxw,
-                                    const float* dx_intra, const float* y_intra, const float* L, const float* wgt,
-                                    const float* dt, const float* D, void* dx, float* red, long long rows, int P, int nh,
-                                    int dtype, cudaStream_t stream) {
+                                    const float* dx_intra, const float* y_intra, const float* L, const float* Ltot,
+                                    const float* wgt, const float* dt, const float* D, void* dx, float* red, long long rows,
+                                    int P, int nh, int Q, int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (P % 8 != 0) return -2;
+  if (P % 8 != 0 || Q <= 0) return -2;
   if (dtype == 1)
-    return launch_bwd_combine<__nv_bfloat16>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, dt, D, dx, red, rows, P, nh, stream);
+    return launch_bwd_combine<__nv_bfloat16>(dy, x, y_inter, dxw, dx_intra, y_intra, L, Ltot, wgt, dt, D, dx, red, rows, P, nh, Q, stream);
   if (dtype == 0)
-    return launch_bwd_combine<__half>(dy, x, y_inter, dxw, dx_intra, y_intra, L, wgt, dt, D, dx, red, rows, P, nh, stream);
+    return launch_bwd_combine<__half>(dy, x, y_inter, dxw, dx_intra, y_intra, L, Ltot, wgt, dt, D, dx, red, rows, P, nh, Q, stream);
   return -2;
 }
 

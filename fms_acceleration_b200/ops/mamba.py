@@ -29,7 +29,7 @@ NV.declare("fmsb_ssd_rowscale", [P_, P_, P_, L_, I_, I_, P_])
 NV.declare("fmsb_ssd_fwd_combine", [P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_addscaled", [P_, P_, P_, P_, L_, I_, I_, P_])
 NV.declare("fmsb_ssd_rowdot", [P_, P_, P_, P_, L_, I_, I_, P_])
-NV.declare("fmsb_ssd_bwd_combine", [P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, P_, L_, I_, I_, I_, P_])
+NV.declare("fmsb_ssd_bwd_combine", [P_] * 13 + [L_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_fwd", [P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssd_state_bwd", [P_, P_, P_, P_, P_, P_, P_, I_, I_, I_, I_, P_])
 NV.declare("fmsb_ssdf_heads", [I_, I_, I_, I_])
@@ -403,27 +403,24 @@ class _SSDScan(torch.autograd.Function):
             del dcb16
         # ---- dx and the per-(t, h) dot products, one pass over the [T, heads, P] tensors
         dx = torch.empty(T, nh, P, dtype=dtp, device=dev)
-        red = torch.empty(5, T, nh, dtype=torch.float32, device=dev)
+        red = torch.empty(6, T, nh, dtype=torch.float32, device=dev)
         Df = D.float().contiguous()
         rc = NV.lib().fmsb_ssd_bwd_combine(dy2.data_ptr(), x2.data_ptr(), y_inter.data_ptr(), dxw.data_ptr(),
-                                           dx_intra.data_ptr(), y_intra.data_ptr(), L.data_ptr(), wgt.data_ptr(),
-                                           dt.data_ptr(), Df.data_ptr(), dx.data_ptr(), red.data_ptr(), T * nh, P, nh, code,
-                                           NV.stream_ptr())
+                                           dx_intra.data_ptr(), y_intra.data_ptr(), L.data_ptr(), Ltot.data_ptr(),
+                                           wgt.data_ptr(), dt.data_ptr(), Df.data_ptr(), dx.data_ptr(), red.data_ptr(),
+                                           T * nh, P, nh, Q, code, NV.stream_ptr())
         NV.check(rc, "fmsb_ssd_bwd_combine")
         del y_inter, dxw, dx_intra, y_intra
         dD = red[0].sum(0)
-        dww = red[2] * wgt                                                    # through w = exp(Ltot - L) dt
-        row, col = red[3], red[4]                                             # sums of dG o G over s / over t
-        w1 = torch.exp(Ltot.view(nc, 1, nh) - L.view(nc, Q, nh)).view(T, nh)  # w without dt
-        ddt = torch.where(still, red[2] * w1 + col, (dww + col) / dt)
-        dL = red[1] - dww + row - col.masked_fill(still, 0.0)
+        dww, row, col, ddt = red[2], red[3], red[4], red[5]  # through w = exp(Ltot - L) dt; sums of dG o G over s / over t
+        dL = red[1] - dww + row - col
         dLtot = dLtot + dww.view(nc, Q, nh).sum(1)
         # ---- through L = cumsum(dt A) within the chunk, Ltot = L[last]: a reverse cumulative sum per chunk
         dLt = _chunk_major(dL, nc, Q, nh)
         dLt[:, :, -1] += dLtot
         dat = dLt.sum(-1, keepdim=True) - dLt.cumsum(-1) + dLt
         da = dat.transpose(1, 2).reshape(T, nh)
-        ddt = ddt + da * A.float()[None, :]
+        ddt = (ddt + da * A.float()[None, :]).view(dt.shape)
         dA = (da * dt).sum(0)
         return (dx, ddt.to(dt.dtype), dA.to(A.dtype), dB.view(T, G, N).to(B.dtype), dC.view(T, G, N).to(C.dtype),
                 dD.to(D.dtype), dh0, None, None, None)
